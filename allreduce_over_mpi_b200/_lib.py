@@ -46,6 +46,7 @@ class Choice(C.Structure):
 
 
 _lib = None
+_native = None
 
 
 def _declare(lib):
@@ -147,6 +148,29 @@ def lib() -> C.CDLL:
         from . import _lib_cuda
         _lib_cuda.declare(_lib)
     return _lib
+
+
+#: entry points that the native call path (csrc/python/ft_torch.cpp) calls
+_NATIVE = ("ft_reduce_nway", "ft_reduce_nway_scaled")
+
+
+def native():
+    """The native call path of the CUDA entry points (lib/_ft_torch.so), bound to the loaded library."""
+    global _native
+    if _native is None:
+        import importlib.util
+        import torch  # noqa: F401 - its libraries have to be in the process first
+        L = lib()
+        path = LIB_PATH.with_name("_ft_torch.so")
+        if not path.exists():
+            from .build import build_ext
+            path = build_ext()
+        spec = importlib.util.spec_from_file_location("_ft_torch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in _NATIVE})
+        _native = mod
+    return _native
 
 
 def text_call(fn, *args, cap: int = 1 << 16) -> str:

@@ -22,6 +22,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "csrc" / "build"
 LIB = PKG / "lib" / "libflextree.so"
+EXT = PKG / "lib" / "_ft_torch.so"
 
 NVCC = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -81,6 +82,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     build_tools()
+    build_ext(force)
     if verbose:
         print("\n".join(logs))
     return LIB
@@ -131,11 +133,31 @@ def build_tools() -> list[Path]:
     return out
 
 
+def build_ext(force: bool = False) -> Path:
+    """The native call path of the Python entry points (csrc/python/ft_torch.cpp), a CPython module on torch's C++
+    headers.  It holds no kernels and does not link libflextree: the loader hands it the entry points."""
+    import sysconfig
+    import torch
+    src = CSRC / "python" / "ft_torch.cpp"
+    if not force and EXT.exists() and EXT.stat().st_mtime >= max(src.stat().st_mtime, (CSRC / "api" / "ft_types.h").stat().st_mtime):
+        return EXT
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(NVCC).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+           "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"], str(src), "-o", str(EXT),
+           "-L", str(root / "lib"), f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{src.name} failed to build:\n{r.stdout}\n{r.stderr}")
+    return EXT
+
+
 def ensure_built() -> Path:
     """Build if the library is missing or older than its sources (needs nvcc)."""
     if LIB.exists():
         newest = max([s.stat().st_mtime for s in sources()] + [headers_mtime()])
-        if LIB.stat().st_mtime >= newest:
+        if LIB.stat().st_mtime >= newest and EXT.exists():
             return LIB
         if not os.path.exists(NVCC):
             return LIB

@@ -13,6 +13,7 @@ from typing import Sequence
 
 import torch
 
+from .. import _lib
 from .._lib import DTYPES, FT_MAX_FANIN, OPS, check, lib
 
 _TORCH2FT = {
@@ -52,6 +53,10 @@ def _check_inputs(tensors, out):
         raise ValueError("out must be contiguous, same size and device")
 
 
+def _failed(code: int, what: str):
+    check(code, lib().ft_last_cuda_error().decode() if code == 6 else what)
+
+
 def reduce_nway(tensors: Sequence[torch.Tensor], op: str = "sum", out: torch.Tensor | None = None,
                 variant: int = 0, threads: int = 0) -> torch.Tensor:
     """Reduce ``tensors`` element-wise into ``out`` (allocated when omitted).
@@ -59,6 +64,9 @@ def reduce_nway(tensors: Sequence[torch.Tensor], op: str = "sum", out: torch.Ten
     ``variant`` selects the device data path: 0/1 vector loads, 2 TMA bulk pipeline,
     11..16 tuning configurations of the vector path (fp32 / bf16 only).
     """
+    fast = (_lib._native or _lib.native()).reduce_nway(tensors, op, out, variant)
+    if fast is not NotImplemented:
+        return fast if type(fast) is not int else _failed(fast, f"{op} on {tensors[0].dtype}")
     _check_inputs(tensors, out)
     t0 = tensors[0]
     if out is None:
@@ -72,7 +80,8 @@ def reduce_nway(tensors: Sequence[torch.Tensor], op: str = "sum", out: torch.Ten
             stream = torch.cuda.current_stream().cuda_stream
             code = lib().ft_reduce_nway(OPS[op], dt, srcs, out.data_ptr(), len(tensors), t0.numel(), variant,
                                         C.c_void_p(stream))
-        check(code, lib().ft_last_cuda_error().decode() if code == 6 else f"{op} on {t0.dtype}")
+        if code:
+            _failed(code, f"{op} on {t0.dtype}")
     else:
         check(lib().ft_cpu_reduce(OPS[op], dt, srcs, out.data_ptr(), len(tensors), t0.numel(), threads),
               f"{op} on {t0.dtype}")
@@ -88,6 +97,9 @@ def reduce_nway_scaled(tensors: Sequence[torch.Tensor], scale: float = 1.0,
                        out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """``out = scale * sum(tensors)`` with fp32 accumulation and an optional fp32<->bf16 cast
     fused into the store (gradient averaging: scale = 1/world, bf16 out)."""
+    fast = (_lib._native or _lib.native()).reduce_nway_scaled(tensors, scale, out_dtype, out)
+    if fast is not NotImplemented:
+        return fast if type(fast) is not int else _failed(fast, f"{tensors[0].dtype}->{out_dtype or tensors[0].dtype}")
     _check_inputs(tensors, out)
     t0 = tensors[0]
     if not t0.is_cuda:
@@ -99,7 +111,8 @@ def reduce_nway_scaled(tensors: Sequence[torch.Tensor], scale: float = 1.0,
         stream = torch.cuda.current_stream().cuda_stream
         code = lib().ft_reduce_nway_scaled(ft_dtype(t0.dtype), ft_dtype(out.dtype), _ptr_array(tensors),
                                            out.data_ptr(), len(tensors), t0.numel(), float(scale), C.c_void_p(stream))
-    check(code, lib().ft_last_cuda_error().decode() if code == 6 else f"{t0.dtype}->{out.dtype}")
+    if code:
+        _failed(code, f"{t0.dtype}->{out.dtype}")
     return out
 
 
