@@ -8,11 +8,13 @@
 // groups so that GROUP x UNROLL independent 16-byte loads are in flight per thread.
 //
 // Data paths:
-//   * 32-byte path (reduce_nway_wide.cu): the default whenever every pointer sits on a 32-byte boundary;
-//   * vector path: persistent grid-stride loop of 16-byte non-allocating loads;
+//   * 32-byte path (reduce_nway_wide.cu): the default whenever all pointers have the same offset from a 32-byte boundary;
+//   * shifted path (reduce_nway_shift.cu): the default for any other pointers;
+//   * vector path (by number): persistent grid-stride loop of 16-byte non-allocating loads;
 //   * TMA path: per-CTA ring of shared-memory stages filled by 1-D bulk async copies
 //     (cp.async.bulk, completion on an mbarrier) and drained by all threads.
-// Unaligned pointers and the sub-16-byte tail take a scalar path with the same arithmetic.
+// The first two do a vector in one launch, edges included; the others leave unaligned pointers and the
+// sub-16-byte tail to a scalar kernel with the same arithmetic.
 //
 // 16-bit floats accumulate in fp32; 64-bit indexing throughout.
 #include <atomic>
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(256) reduce_nway_scalar_kernel(const __grid_co
   using S = ScalarOp<POL>;
   using T = typename S::elem;
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long i = first_unit + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.nunit; i += stride) {
+  for (unsigned long long i = first_unit + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.nbody; i += stride) {
     typename S::acc acc = S::load(((const T*)a.src[0])[i]);
     for (int k = 1; k < a.n; ++k) acc = S::comb(acc, S::load(((const T*)a.src[k])[i]));
     ((T*)a.dst)[i] = S::store(acc);
@@ -274,8 +276,8 @@ static cudaError_t launch_vec(const NwayArgs& a, int threads, int ctas_per_sm, c
 
 template <int POL>
 static cudaError_t launch_scalar(const NwayArgs& a, unsigned long long first_unit, cudaStream_t st) {
-  if (first_unit >= a.nunit) return cudaSuccess;
-  unsigned long long want = (a.nunit - first_unit + 255) / 256;
+  if (first_unit >= a.nbody) return cudaSuccess;
+  unsigned long long want = (a.nbody - first_unit + 255) / 256;
   unsigned long long cap = (unsigned long long)dev_info().sms * 8;
   reduce_nway_scalar_kernel<POL><<<(int)(want < cap ? want : cap), 256, 0, st>>>(a, first_unit);
   g_launches++;
@@ -317,37 +319,80 @@ static cudaError_t launch_tma(const NwayArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Cut the vector for the 32-byte kernel: possible when every pointer has the same offset from a 32-byte boundary
+// (a slice of a flat buffer reduced into the same slice of another, or whole tensors).
+static bool layout_wide(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
+  const uintptr_t phase = (uintptr_t)in.dst & 31;
+  for (int k = 0; k < in.n; ++k)
+    if (((uintptr_t)in.src[k] & 31) != phase) return false;
+  const size_t head = (32 - phase) & 31;
+  if (bytes < head + 32) return false;
+  *out = in;
+  out->nvec = (bytes - head) / 32;
+  out->nbody = out->nvec * 32 / unit;
+  out->head = (uint16_t)(head / unit);
+  out->edge = (uint16_t)((bytes - out->nvec * 32) / unit);
+  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
+  out->dst = (unsigned char*)in.dst + head;
+  return true;
+}
+// Cut it on the result's 16-byte boundaries for the shifted kernel.  A source that lies s bytes behind such a
+// boundary is read from s bytes before the body to 16 - s bytes behind it; the body is kept small enough for these
+// to be the vector's own bytes.  A vector too short for that is all edges.
+static void layout_shift(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
+  *out = in;
+  size_t head = (16 - ((uintptr_t)in.dst & 15)) & 15, widest = 0;
+  bool any = false;
+  for (int k = 0; k < in.n; ++k) {
+    out->shift[k] = (uint8_t)(((uintptr_t)in.src[k] + head) & 15);
+    any = any || out->shift[k];
+    if (out->shift[k] > widest) widest = out->shift[k];
+  }
+  if (widest > head) head += 16;
+  unsigned long long nvec = bytes > head ? (bytes - head) / 16 : 0;
+  for (int k = 0; k < in.n; ++k)
+    if (out->shift[k]) {
+      const unsigned long long whole = (bytes > head ? bytes - head + out->shift[k] : 0) / 16;
+      const unsigned long long fits = whole ? whole - 1 : 0;
+      if (fits < nvec) nvec = fits;
+    }
+  if (!nvec) head = 0;
+  out->nvec = nvec;
+  out->nbody = nvec * 16 / unit;
+  out->head = (uint16_t)(head / unit);
+  out->edge = (uint16_t)((bytes - nvec * 16) / unit);
+  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
+  out->dst = (unsigned char*)in.dst + head;
+}
+
 template <int POL>
 static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
+  const size_t unit = sizeof(typename ScalarOp<POL>::elem);
+  cudaError_t e = cudaSuccess;
+  if (variant == 0 || variant >= 1000) {
+    NwayArgs b;
+    e = cudaErrorInvalidValue;
+    if (layout_wide(a, bytes, unit, &b)) e = launch_wide(POL, b, variant, dev_info().sms, st);
+    if (e == cudaErrorInvalidValue) {   // other phases, or no such configuration
+      cudaGetLastError();
+      layout_shift(a, bytes, unit, &b);
+      e = launch_shift(POL, b, st);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "reduce_nway launch");
+    g_launches++;
+    return FT_OK;
+  }
+  // the configurations that are asked for by number: 16-byte accesses where every pointer allows them, a second
+  // launch for the rest
   bool aligned = ((uintptr_t)a.dst & 15) == 0;
   for (int k = 0; k < a.n; ++k) aligned = aligned && (((uintptr_t)a.src[k] & 15) == 0);
-  const size_t unit = sizeof(typename ScalarOp<POL>::elem);
-  a.nunit = bytes / unit;
+  a.nbody = bytes / unit;
   a.nvec = aligned ? bytes / 16 : 0;
-  cudaError_t e = cudaSuccess;
-  // 32-byte accesses (reduce_nway_wide.cu) when every pointer sits on a 32-byte boundary
-  if (a.nvec >= 2 && (variant >= 1000 || variant == 0)) {
-    bool a32 = ((uintptr_t)a.dst & 31) == 0;
-    for (int k = 0; k < a.n; ++k) a32 = a32 && (((uintptr_t)a.src[k] & 31) == 0);
-    if (a32) {
-      const unsigned long long n32 = bytes / 32;
-      e = launch_wide(POL, a, n32, variant >= 1000 ? variant : 0, dev_info().sms, st);
-      if (e == cudaSuccess) {
-        g_launches++;
-        e = launch_scalar<POL>(a, n32 * 32 / unit, st);
-        if (e != cudaSuccess) return cuda_fail(e, "reduce_nway scalar launch");
-        return FT_OK;
-      }
-      if (e != cudaErrorInvalidValue) return cuda_fail(e, "reduce_nway wide launch");
-      cudaGetLastError();
-      e = cudaSuccess;   // no such instantiation: the 16-byte kernels take it
-    }
-  }
   if (a.nvec) {
     bool done = false;
     if (variant == 2) { e = launch_tma<POL>(a, st); done = true; }
     if constexpr (POL == POL_F32 || POL == POL_BF16) {
-      // tuning variants (unroll, fan-in group, threads, CTAs per SM); 0/1 pick the default
+      // tuning variants (unroll, fan-in group, threads, CTAs per SM)
       switch (variant) {
         case 11: e = launch_vec<POL, 2, 2>(a, 512, 4, st); done = true; break;
         case 12: e = launch_vec<POL, 2, 4>(a, 512, 4, st); done = true; break;
@@ -366,7 +411,7 @@ static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
         default: break;
       }
     }
-    // defaults picked from a B200 sweep (fp32 and bf16, 64 Mi elements): low fan-in runs a
+    // picked from a B200 sweep (fp32 and bf16, 64 Mi elements): low fan-in runs a
     // persistent grid of 2 CTAs x 512 threads per SM with 4 vectors x 2 sources in flight; from
     // fan-in 6 up one CTA per tile with 1 vector x 4 sources in flight does better;
     // fp32 with three or more sources: 8 bytes per thread, one CTA per tile, all loads up front

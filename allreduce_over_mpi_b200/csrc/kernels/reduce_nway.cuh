@@ -1,22 +1,45 @@
-// Argument block of the single-GPU n-way reduction kernels (reduce_nway.cu, reduce_nway_wide.cu).
+// Argument block of the single-GPU n-way reduction kernels (reduce_nway.cu, reduce_nway_wide.cu, reduce_nway_shift.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include "../api/ft_types.h"
 
 namespace ftk {
 
+// One launch covers a whole vector: the body in 32- or 16-byte vectors, and the elements in front of and behind it
+// (the edges) one by one in a CTA of their own (block 0), so that neither a ragged length nor a slice that starts
+// off a vector boundary costs a second launch or takes the rest of the vector off the vector loads.
 struct NwayArgs {
-  const void* src[FT_MAX_FANIN];
+  const void* src[FT_MAX_FANIN];  // start of the body in every source
   void* dst;
-  unsigned long long nvec;   // 16-byte vectors
-  unsigned long long nunit;  // scalar units (see ScalarOp) for the scalar kernel
+  unsigned long long nvec;    // body length, in the kernel's vectors
+  unsigned long long nbody;   // ... and in scalar units (see ScalarOp)
   int n;
+  uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
+  uint8_t shift[FT_MAX_FANIN];  // shifted kernel: bytes by which source k's body lies behind a 16-byte boundary
 };
 
-// 32-byte-per-access kernels (reduce_nway_wide.cu).  `code` selects a configuration (0: the default;
-// see launch_cfg there); returns cudaErrorInvalidValue when (policy, fan-in, code) has no
-// instantiation, in which case the caller falls back to the 16-byte kernels.
-cudaError_t launch_wide(int pol, const NwayArgs& a, unsigned long long n32, int code, int sms, cudaStream_t st);
+// Kernels for pointers that agree modulo 32 (reduce_nway_wide.cu).  `code` selects a configuration (0: by size;
+// see launch_cfg there); returns cudaErrorInvalidValue when (policy, fan-in, code) has no instantiation.
+cudaError_t launch_wide(int pol, const NwayArgs& a, int code, int sms, cudaStream_t st);
+// Kernel for pointers that do not agree modulo 32 (reduce_nway_shift.cu).
+cudaError_t launch_shift(int pol, const NwayArgs& a, cudaStream_t st);
+
+#ifdef __CUDACC__
+// The edges of the vector, by the CTA the launch adds for them (at most 3 x 32 bytes: one or two units a thread).
+template <int POL, template <int> class Scalar>
+__device__ __forceinline__ void reduce_edges(const NwayArgs& a) {
+  using S = Scalar<POL>;
+  using T = typename S::elem;
+  for (int e = threadIdx.x; e < a.edge; e += blockDim.x) {
+    const long long i = e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head));
+    typename S::acc acc = S::load(((const T*)a.src[0])[i]);
+#pragma unroll 4
+    for (int k = 1; k < a.n; ++k) acc = S::comb(acc, S::load(((const T*)a.src[k])[i]));
+    ((T*)a.dst)[i] = S::store(acc);
+  }
+}
+#endif
 
 }  // namespace ftk

@@ -9,6 +9,7 @@
 //
 // Same job as the reference's reduce_sum_2 .. reduce_sum_8 kernels
 // (vector_add/reduce_sum_gpu.h:13-69), which move 4 bytes per thread.
+#include "pdl.cuh"
 #include "reduce_nway.cuh"
 #include "vec.cuh"
 
@@ -44,13 +45,21 @@ __device__ __forceinline__ void st32(void* p, const uint4& a, const uint4& b) {
 // One thread handles UNROLL 32-byte units per step, THREADS apart (every warp access is one
 // contiguous 1 KiB run).  The grid either covers the vector once (one step per thread) or is
 // capped and strides over it.  NSRC > 0: the fan-in is known at compile time; NSRC == 0: it is
-// a.n (any value up to FT_MAX_FANIN), taken four sources at a time.
-template <int POL, int NSRC, int UNROLL, int LD, int ST, int THREADS>
-__global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a, unsigned long long n32) {
+// a.n (any value up to FT_MAX_FANIN).  Sources are taken GROUP at a time: all loads of a group are
+// issued before its first add.
+template <int POL, int NSRC, int UNROLL, int LD, int ST, int THREADS, int GROUP>
+__global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
+  pdl_begin();
+  const int edge_ctas = a.edge != 0;
+  if (edge_ctas && blockIdx.x == 0) {
+    reduce_edges<POL, ScalarOp>(a);
+    return;
+  }
+  const unsigned long long n32 = a.nvec;
   const int nsrc = NSRC > 0 ? NSRC : a.n;
-  const unsigned long long stride = (unsigned long long)gridDim.x * THREADS * UNROLL;
-  for (unsigned long long base = (unsigned long long)blockIdx.x * THREADS * UNROLL; base < n32; base += stride) {
+  const unsigned long long stride = (unsigned long long)(gridDim.x - edge_ctas) * THREADS * UNROLL;
+  for (unsigned long long base = (unsigned long long)(blockIdx.x - edge_ctas) * THREADS * UNROLL; base < n32; base += stride) {
     unsigned long long idx[UNROLL];
     bool ok[UNROLL];
 #pragma unroll
@@ -58,8 +67,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
       idx[u] = base + (unsigned long long)u * THREADS + threadIdx.x;
       ok[u] = idx[u] < n32;
     }
-    // sources are taken four at a time: all loads of a group are issued before its first add
-    constexpr int G = (NSRC > 0 && NSRC < 4) ? NSRC : 4;
+    constexpr int G = (NSRC > 0 && NSRC < GROUP) ? NSRC : GROUP;
     typename P::Acc al[UNROLL], ah[UNROLL];
 #pragma unroll
     for (int g0 = 0; g0 < (NSRC > 0 ? NSRC : FT_MAX_FANIN); g0 += G) {
@@ -86,38 +94,44 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
   }
 }
 
-// code = U*1000 + LD*100 + ST*10 + T, with U units per thread per step, LD/ST as above,
+// The default: 256 threads, one 32-byte unit each, up to eight sources in flight, evict-first stores, the grid
+// covers the vector once.  What bounds it is HBM; from 2 to 16 sources of 4 to 80 MB fp32 / bf16 / fp16 it is within
+// 3 % of the best of 16 configurations swept (128-512 threads, groups of 4 or 8, cache hints, persistent grids).
+// Groups of eight instead of four sources matter where the chip is not full: fp16 x16 of 1 Mi 9.6 -> 6.2 us,
+// bf16 x8 of 4 Mi 16.4 -> 14.4 us; with the dependent launch (pdl.cuh) 5.7 and 12.9.
+// fp32 x8 of 20 M: 104.5 -> 102.0 us, 7.06 TB/s.
+//
+// Other configurations by code = U*1000 + LD*100 + ST*10 + T, with U units per thread per step, LD/ST as above,
 // T: 0 = 256 threads and one step per thread (the grid covers the vector), 1 = 512 threads likewise,
-//    3 = 512 threads x 4 CTAs per SM striding over the vector.
-// Measured on B200 over fan-in 2/3/4/8, fp32 and bf16, 64 Mi elements, launches back to back: 1011 is within
-// 1 % of the best configuration in every case (6.5-7.2 TB/s) and is the default; the others stay selectable.
-constexpr int kWideDefault = 1011;
-
+//    3 = 512 threads x 4 CTAs per SM striding over the vector; groups of four sources.
+template <int POL, int NSRC, int UNROLL, int LD, int ST, int THREADS, int GROUP>
+static cudaError_t launch_t(const NwayArgs& a, int ctas_per_sm, int sms, cudaStream_t st) {
+  const unsigned long long per_cta = (unsigned long long)THREADS * UNROLL;
+  unsigned long long grid = (a.nvec + per_cta - 1) / per_cta;
+  if (ctas_per_sm && grid > (unsigned long long)sms * ctas_per_sm) grid = (unsigned long long)sms * ctas_per_sm;
+  grid += a.edge != 0;
+  if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
+  return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, UNROLL, LD, ST, THREADS, GROUP>, (unsigned)grid, THREADS, 0, st, a);
+}
 template <int POL, int NSRC, int UNROLL, int LD, int ST>
-static cudaError_t launch_t(const NwayArgs& a, unsigned long long n32, int t, int sms, cudaStream_t st) {
-  const int threads = t == 0 ? 256 : 512;
-  const unsigned long long per_cta = (unsigned long long)threads * UNROLL;
-  unsigned long long grid = (n32 + per_cta - 1) / per_cta;
-  if (t == 3 && grid > (unsigned long long)sms * 4) grid = (unsigned long long)sms * 4;
-  if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-  if (grid < 1) grid = 1;
-  if (threads == 256) reduce_nway_wide_kernel<POL, NSRC, UNROLL, LD, ST, 256><<<(unsigned)grid, 256, 0, st>>>(a, n32);
-  else reduce_nway_wide_kernel<POL, NSRC, UNROLL, LD, ST, 512><<<(unsigned)grid, 512, 0, st>>>(a, n32);
-  return cudaGetLastError();
+static cudaError_t launch_v(const NwayArgs& a, int t, int sms, cudaStream_t st) {
+  return t == 0 ? launch_t<POL, NSRC, UNROLL, LD, ST, 256, 4>(a, 0, sms, st)
+                : launch_t<POL, NSRC, UNROLL, LD, ST, 512, 4>(a, t == 3 ? 4 : 0, sms, st);
 }
 
 template <int POL, int NSRC, bool TUNING>
-static cudaError_t launch_cfg(const NwayArgs& a, unsigned long long n32, int code, int sms, cudaStream_t st) {
+static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t st) {
   const int t = code % 10;
   if (t != 0 && t != 1 && t != 3) return cudaErrorInvalidValue;
-  if (code / 10 == kWideDefault / 10) return launch_t<POL, NSRC, 1, 0, 1>(a, n32, t, sms, st);
+  if (code == 0) return launch_t<POL, NSRC, 1, 0, 1, 256, 8>(a, 0, sms, st);
   if constexpr (TUNING) {
     switch (code / 10) {
-      case 100: return launch_t<POL, NSRC, 1, 0, 0>(a, n32, t, sms, st);
-      case 111: return launch_t<POL, NSRC, 1, 1, 1>(a, n32, t, sms, st);
-      case 200: return launch_t<POL, NSRC, 2, 0, 0>(a, n32, t, sms, st);
-      case 201: return launch_t<POL, NSRC, 2, 0, 1>(a, n32, t, sms, st);
-      case 211: return launch_t<POL, NSRC, 2, 1, 1>(a, n32, t, sms, st);
+      case 101: return launch_v<POL, NSRC, 1, 0, 1>(a, t, sms, st);
+      case 100: return launch_v<POL, NSRC, 1, 0, 0>(a, t, sms, st);
+      case 111: return launch_v<POL, NSRC, 1, 1, 1>(a, t, sms, st);
+      case 200: return launch_v<POL, NSRC, 2, 0, 0>(a, t, sms, st);
+      case 201: return launch_v<POL, NSRC, 2, 0, 1>(a, t, sms, st);
+      case 211: return launch_v<POL, NSRC, 2, 1, 1>(a, t, sms, st);
       default: break;
     }
   }
@@ -125,33 +139,32 @@ static cudaError_t launch_cfg(const NwayArgs& a, unsigned long long n32, int cod
 }
 
 template <int POL, bool TUNING>
-static cudaError_t launch_n(const NwayArgs& a, unsigned long long n32, int code, int sms, cudaStream_t st) {
+static cudaError_t launch_n(const NwayArgs& a, int code, int sms, cudaStream_t st) {
   switch (a.n) {
-    case 1: return launch_cfg<POL, 1, false>(a, n32, code, sms, st);
-    case 2: return launch_cfg<POL, 2, TUNING>(a, n32, code, sms, st);
-    case 3: return launch_cfg<POL, 3, TUNING>(a, n32, code, sms, st);
-    case 4: return launch_cfg<POL, 4, TUNING>(a, n32, code, sms, st);
-    case 5: return launch_cfg<POL, 5, false>(a, n32, code, sms, st);
-    case 6: return launch_cfg<POL, 6, false>(a, n32, code, sms, st);
-    case 7: return launch_cfg<POL, 7, false>(a, n32, code, sms, st);
-    case 8: return launch_cfg<POL, 8, TUNING>(a, n32, code, sms, st);
-    default: return launch_cfg<POL, 0, false>(a, n32, code, sms, st);
+    case 1: return launch_cfg<POL, 1, false>(a, code, sms, st);
+    case 2: return launch_cfg<POL, 2, TUNING>(a, code, sms, st);
+    case 3: return launch_cfg<POL, 3, TUNING>(a, code, sms, st);
+    case 4: return launch_cfg<POL, 4, TUNING>(a, code, sms, st);
+    case 5: return launch_cfg<POL, 5, false>(a, code, sms, st);
+    case 6: return launch_cfg<POL, 6, false>(a, code, sms, st);
+    case 7: return launch_cfg<POL, 7, false>(a, code, sms, st);
+    case 8: return launch_cfg<POL, 8, TUNING>(a, code, sms, st);
+    default: return launch_cfg<POL, 0, false>(a, code, sms, st);
   }
 }
 
-cudaError_t launch_wide(int pol, const NwayArgs& a, unsigned long long n32, int code, int sms, cudaStream_t st) {
-  if (code <= 0) code = kWideDefault;
+cudaError_t launch_wide(int pol, const NwayArgs& a, int code, int sms, cudaStream_t st) {
   switch (pol) {
-    case POL_ADD8: return launch_n<POL_ADD8, false>(a, n32, code, sms, st);
-    case POL_ADD16: return launch_n<POL_ADD16, false>(a, n32, code, sms, st);
-    case POL_ADD32: return launch_n<POL_ADD32, false>(a, n32, code, sms, st);
-    case POL_ADD64: return launch_n<POL_ADD64, false>(a, n32, code, sms, st);
-    case POL_OR: return launch_n<POL_OR, false>(a, n32, code, sms, st);
-    case POL_AND: return launch_n<POL_AND, false>(a, n32, code, sms, st);
-    case POL_F32: return launch_n<POL_F32, true>(a, n32, code, sms, st);
-    case POL_F64: return launch_n<POL_F64, false>(a, n32, code, sms, st);
-    case POL_BF16: return launch_n<POL_BF16, true>(a, n32, code, sms, st);
-    case POL_F16: return launch_n<POL_F16, false>(a, n32, code, sms, st);
+    case POL_ADD8: return launch_n<POL_ADD8, false>(a, code, sms, st);
+    case POL_ADD16: return launch_n<POL_ADD16, false>(a, code, sms, st);
+    case POL_ADD32: return launch_n<POL_ADD32, false>(a, code, sms, st);
+    case POL_ADD64: return launch_n<POL_ADD64, false>(a, code, sms, st);
+    case POL_OR: return launch_n<POL_OR, false>(a, code, sms, st);
+    case POL_AND: return launch_n<POL_AND, false>(a, code, sms, st);
+    case POL_F32: return launch_n<POL_F32, true>(a, code, sms, st);
+    case POL_F64: return launch_n<POL_F64, false>(a, code, sms, st);
+    case POL_BF16: return launch_n<POL_BF16, true>(a, code, sms, st);
+    case POL_F16: return launch_n<POL_F16, false>(a, code, sms, st);
     default: return cudaErrorInvalidValue;
   }
 }
