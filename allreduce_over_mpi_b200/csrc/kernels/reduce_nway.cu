@@ -426,48 +426,6 @@ static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
   return FT_OK;
 }
 
-// ---------------------------------------------------------------------------- scaled / cast variant
-// out = scale * sum_k src[k], fp32 accumulation; IN/OUT in {fp32, bf16}.
-template <bool IN_BF16, bool OUT_BF16>
-__global__ void __launch_bounds__(512) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, unsigned long long len, float scale, bool vec_ok) {
-  // work in groups of 8 elements: 8 bf16 = 16 B, 8 fp32 = 32 B
-  const unsigned long long ngroups = vec_ok ? len / 8 : 0;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += stride) {
-    float acc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (int k = 0; k < a.n; ++k) {
-      if (IN_BF16) {
-        uint4 v = ld_stream((const uint4*)a.src[k] + g);
-        acc[0] += bf_lo(v.x); acc[1] += bf_hi(v.x); acc[2] += bf_lo(v.y); acc[3] += bf_hi(v.y);
-        acc[4] += bf_lo(v.z); acc[5] += bf_hi(v.z); acc[6] += bf_lo(v.w); acc[7] += bf_hi(v.w);
-      } else {
-        uint4 v = ld_stream((const uint4*)a.src[k] + 2 * g), w = ld_stream((const uint4*)a.src[k] + 2 * g + 1);
-        acc[0] += __uint_as_float(v.x); acc[1] += __uint_as_float(v.y); acc[2] += __uint_as_float(v.z); acc[3] += __uint_as_float(v.w);
-        acc[4] += __uint_as_float(w.x); acc[5] += __uint_as_float(w.y); acc[6] += __uint_as_float(w.z); acc[7] += __uint_as_float(w.w);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] *= scale;
-    if (OUT_BF16) {
-      st_vec((uint4*)a.dst + g, make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7])));
-    } else {
-      st_vec((uint4*)a.dst + 2 * g, make_uint4(__float_as_uint(acc[0]), __float_as_uint(acc[1]), __float_as_uint(acc[2]), __float_as_uint(acc[3])));
-      st_vec((uint4*)a.dst + 2 * g + 1, make_uint4(__float_as_uint(acc[4]), __float_as_uint(acc[5]), __float_as_uint(acc[6]), __float_as_uint(acc[7])));
-    }
-  }
-  // ragged tail / unaligned: scalar
-  for (unsigned long long i = ngroups * 8 + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride) {
-    float acc = 0.f;
-    for (int k = 0; k < a.n; ++k)
-      acc += IN_BF16 ? __bfloat162float(((const __nv_bfloat16*)a.src[k])[i]) : ((const float*)a.src[k])[i];
-    acc *= scale;
-    if (OUT_BF16) ((__nv_bfloat16*)a.dst)[i] = __float2bfloat16_rn(acc);
-    else ((float*)a.dst)[i] = acc;
-  }
-}
-
 // ---------------------------------------------------------------------------- scale in place
 // buf[i] *= scale for every floating type, with the policies' arithmetic (16-bit floats through fp32,
 // one rounding): what a one-rank "average" all-reduce has to do.
@@ -552,24 +510,14 @@ int ft_reduce_nway_scaled(int in_dtype, int out_dtype, const void* const* src, v
   if (len == 0) return FT_OK;
   if (!src || !dst) return FT_ERR_INVALID_ARG;
   NwayArgs a{};
-  bool aligned = ((uintptr_t)dst & 15) == 0;
   for (int k = 0; k < n; ++k) {
     if (!src[k]) return FT_ERR_INVALID_ARG;
     a.src[k] = src[k];
-    aligned = aligned && (((uintptr_t)src[k] & 15) == 0);
   }
   a.dst = dst;
   a.n = n;
-  unsigned long long want = (len / 8 + 511) / 512 + 1, cap = (unsigned long long)dev_info().sms * 4;
-  const int grid = (int)(want < cap ? want : cap);
-  cudaStream_t st = (cudaStream_t)stream;
-  const bool ib = in_dtype == FT_BF16, ob = out_dtype == FT_BF16;
-  if (ib && ob) reduce_nway_scaled_kernel<true, true><<<grid, 512, 0, st>>>(a, len, scale, aligned);
-  else if (ib) reduce_nway_scaled_kernel<true, false><<<grid, 512, 0, st>>>(a, len, scale, aligned);
-  else if (ob) reduce_nway_scaled_kernel<false, true><<<grid, 512, 0, st>>>(a, len, scale, aligned);
-  else reduce_nway_scaled_kernel<false, false><<<grid, 512, 0, st>>>(a, len, scale, aligned);
+  const cudaError_t e = launch_scaled(in_dtype == FT_BF16, out_dtype == FT_BF16, a, len, scale, dev_info().sms, (cudaStream_t)stream);
   g_launches++;
-  cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FT_OK : cuda_fail(e, "reduce_nway_scaled launch");
 }
 

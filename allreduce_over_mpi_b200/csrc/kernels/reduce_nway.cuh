@@ -1,4 +1,5 @@
-// Argument block of the single-GPU n-way reduction kernels (reduce_nway.cu, reduce_nway_wide.cu, reduce_nway_shift.cu).
+// Argument block of the single-GPU n-way reduction kernels (reduce_nway.cu, reduce_nway_wide.cu,
+// reduce_nway_shift.cu, reduce_nway_scaled.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,6 +26,8 @@ struct NwayArgs {
 cudaError_t launch_wide(int pol, const NwayArgs& a, int code, int sms, cudaStream_t st);
 // Kernel for pointers that do not agree modulo 32 (reduce_nway_shift.cu).
 cudaError_t launch_shift(int pol, const NwayArgs& a, cudaStream_t st);
+// out = scale * sum over `len` elements of whole vectors in `a` (reduce_nway_scaled.cu).
+cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st);
 
 #ifdef __CUDACC__
 // The edges of the vector, by the CTA the launch adds for them (at most 3 x 32 bytes: one or two units a thread).
@@ -34,9 +37,16 @@ __device__ __forceinline__ void reduce_edges(const NwayArgs& a) {
   using T = typename S::elem;
   for (int e = threadIdx.x; e < a.edge; e += blockDim.x) {
     const long long i = e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head));
-    typename S::acc acc = S::load(((const T*)a.src[0])[i]);
-#pragma unroll 4
-    for (int k = 1; k < a.n; ++k) acc = S::comb(acc, S::load(((const T*)a.src[k])[i]));
+    typename S::acc acc{};
+    for (int k0 = 0; k0 < a.n; k0 += 8) {   // eight loads in flight, like the body: a small vector waits for this CTA
+      T v[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g)
+        if (k0 + g < a.n) v[g] = ((const T*)a.src[k0 + g])[i];
+#pragma unroll
+      for (int g = 0; g < 8; ++g)
+        if (k0 + g < a.n) acc = k0 + g == 0 ? S::load(v[g]) : S::comb(acc, S::load(v[g]));
+    }
     ((T*)a.dst)[i] = S::store(acc);
   }
 }

@@ -1,0 +1,145 @@
+// out = scale * sum_k src[k] on one GPU, fp32 accumulation, fp32 or bf16 in and out (gradient averaging with the cast
+// fused into the store).
+//
+// HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, up to
+// eight sources in flight, the grid covers the vector once, edges in a CTA of their own, dependent launch.  The unit
+// is 8 fp32 or 16 bf16 elements, whatever the output type, so that the source side (n streams to one) stays on 256-bit
+// loads.  fp32 -> bf16, 8 sources of 6.5 M: 38.9 us (5.7 TB/s, a strided loop with 16-byte loads of one source at a
+// time) -> 33.7 us (6.6 TB/s).
+#include "../api/flextree.h"
+#include "pdl.cuh"
+#include "reduce_nway.cuh"
+#include "vec.cuh"
+
+namespace ftk {
+
+template <bool WIDE>
+__device__ __forceinline__ void load32(const unsigned char* p, uint4& a, uint4& b) {
+  if (WIDE) {
+    asm volatile("ld.global.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(p) : "memory");
+  } else {
+    a = ld_stream(p);
+    b = ld_stream(p + 16);
+  }
+}
+template <bool WIDE>
+__device__ __forceinline__ void store32(unsigned char* p, const uint4& a, const uint4& b) {
+  if (WIDE) {
+    asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+  } else {
+    st_vec_cs(p, a);
+    st_vec_cs(p + 16, b);
+  }
+}
+
+// Element i (of a body that starts at element 0) of the result.
+template <bool IN_BF16, bool OUT_BF16>
+__device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, float scale) {
+  float acc = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < a.n; ++k)
+    acc += IN_BF16 ? __bfloat162float(((const __nv_bfloat16*)a.src[k])[i]) : ((const float*)a.src[k])[i];
+  acc *= scale;
+  if (OUT_BF16) ((__nv_bfloat16*)a.dst)[i] = __float2bfloat16_rn(acc);
+  else ((float*)a.dst)[i] = acc;
+}
+
+// WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
+// 32); not WIDE: 128-bit ones.
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int GROUP>
+__global__ void __launch_bounds__(256) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, float scale) {
+  constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
+  pdl_begin();
+  const int edge_ctas = a.edge != 0;
+  if (edge_ctas && blockIdx.x == 0) {
+    for (int e = threadIdx.x; e < (int)a.edge; e += blockDim.x)
+      scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), scale);
+    return;
+  }
+  const unsigned long long i = (unsigned long long)(blockIdx.x - edge_ctas) * 256 + threadIdx.x;
+  if (i >= a.nvec) return;
+  float acc[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) acc[j] = 0.f;
+  for (int k0 = 0; k0 < a.n; k0 += GROUP) {
+    uint4 lo[GROUP], hi[GROUP];
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g)
+      if (k0 + g < a.n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g)
+      if (k0 + g < a.n) {
+        const uint32_t w[8] = {lo[g].x, lo[g].y, lo[g].z, lo[g].w, hi[g].x, hi[g].y, hi[g].z, hi[g].w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (IN_BF16) { acc[(2 * j) % E] += bf_lo(w[j]); acc[(2 * j + 1) % E] += bf_hi(w[j]); }
+          else acc[j] += __uint_as_float(w[j]);
+        }
+      }
+  }
+  constexpr int W = OUT_BF16 ? E / 2 : E;   // output words
+  uint32_t o[W];
+#pragma unroll
+  for (int j = 0; j < W; ++j) o[j] = OUT_BF16 ? pack_bf16x2(acc[(2 * j) % E] * scale, acc[(2 * j + 1) % E] * scale) : __float_as_uint(acc[j] * scale);
+  unsigned char* d = (unsigned char*)a.dst + i * (W * 4);
+  if constexpr (W == 4) {
+    st_vec_cs(d, make_uint4(o[0], o[1], o[2], o[3]));
+  } else {
+#pragma unroll
+    for (int j = 0; j + 8 <= W; j += 8)
+      store32<WIDE>(d + j * 4, make_uint4(o[j], o[j + 1], o[j + 2], o[j + 3]), make_uint4(o[j + 4], o[j + 5], o[j + 6], o[j + 7]));
+  }
+}
+
+// Pointers no common vector fits: one element at a time.
+template <bool IN_BF16, bool OUT_BF16>
+__global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __grid_constant__ NwayArgs a, unsigned long long len, float scale) {
+  pdl_begin();
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (unsigned long long)gridDim.x * blockDim.x)
+    scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, scale);
+}
+
+// First element from which every source lies on a boundary of `sa` bytes and the output on one of `da`, or -1.
+static int common_head(const NwayArgs& a, size_t is, size_t os, size_t sa, size_t da) {
+  for (size_t h = 0; h < sa / is; ++h) {
+    bool ok = ((uintptr_t)a.dst + h * os) % da == 0;
+    for (int k = 0; ok && k < a.n; ++k) ok = ((uintptr_t)a.src[k] + h * is) % sa == 0;
+    if (ok) return (int)h;
+  }
+  return -1;
+}
+
+template <bool IN_BF16, bool OUT_BF16>
+static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int sms, cudaStream_t st) {
+  constexpr unsigned long long E = IN_BF16 ? 16 : 8;
+  constexpr size_t is = IN_BF16 ? 2 : 4, os = OUT_BF16 ? 2 : 4;
+  bool wide = true;
+  int head = common_head(a, is, os, 32, IN_BF16 || !OUT_BF16 ? 32 : 16);
+  if (head < 0) { wide = false; head = common_head(a, is, os, 16, 16); }
+  if (head < 0) {
+    const unsigned long long want = (len + 255) / 256, cap = (unsigned long long)sms * 8;
+    return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, a, len, scale);
+  }
+  a.nvec = len >= head + E ? (len - head) / E : 0;   // shorter: all edges
+  a.nbody = a.nvec * E;
+  a.head = (uint16_t)(a.nvec ? head : 0);
+  a.edge = (uint16_t)(len - a.nbody);
+  for (int k = 0; k < a.n; ++k) a.src[k] = (const unsigned char*)a.src[k] + a.head * is;
+  a.dst = (unsigned char*)a.dst + a.head * os;
+  const unsigned long long grid = (a.nvec + 255) / 256 + (a.edge != 0);
+  if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
+  // groups of four where there are no more sources: fewer registers, more CTAs on an SM
+  if (a.n <= 4) return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 4>, (unsigned)grid, 256, 0, st, a, scale)
+                            : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 4>, (unsigned)grid, 256, 0, st, a, scale);
+  return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 8>, (unsigned)grid, 256, 0, st, a, scale)
+              : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 8>, (unsigned)grid, 256, 0, st, a, scale);
+}
+
+cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st) {
+  if (in_bf16) return out_bf16 ? launch_t<true, true>(a, len, scale, sms, st) : launch_t<true, false>(a, len, scale, sms, st);
+  return out_bf16 ? launch_t<false, true>(a, len, scale, sms, st) : launch_t<false, false>(a, len, scale, sms, st);
+}
+
+}  // namespace ftk

@@ -3,7 +3,7 @@ edges) or not (shifted kernel), at the lengths where body and edges meet."""
 import pytest
 import torch
 
-from allreduce_over_mpi_b200.ops import launch_count, reduce_nway
+from allreduce_over_mpi_b200.ops import launch_count, reduce_nway, reduce_nway_scaled
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -41,3 +41,19 @@ def test_in_place_with_sources_at_other_phases():
     want = ts[0] + ts[1] + ts[2]
     assert torch.equal(reduce_nway(ts, out=ts[0]), want)
     assert torch.equal(base[0, 1:10_001], want)
+
+
+@pytest.mark.parametrize("srcs,dst", [((0,), 0), ((3,), 3), ((8,), 0), ((4,), 8), ((0, 1), 0)])
+@pytest.mark.parametrize("tin", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tout", [torch.float32, torch.bfloat16])
+def test_scaled_every_layout_and_length(tin, tout, srcs, dst):
+    """256-bit, 128-bit and one-element forms, with heads and tails; small whole numbers, so every sum is exact."""
+    for length in (1, 7, 8, 15, 16, 17, 31, 33, 47, 1000, 4099, 70_001):
+        for n in (1, 4, 5, 9):
+            g = torch.Generator().manual_seed(length + n)
+            ts = [torch.randint(-8, 8, (length + 8,), generator=g).to(tin).to(DEV)[srcs[k % len(srcs)]:][:length] for k in range(n)]
+            flat = torch.zeros(length + 16, dtype=tout, device=DEV)
+            reduce_nway_scaled(ts, scale=0.25, out=flat[dst:dst + length])
+            want = (sum(t.float() for t in ts) * 0.25).to(tout)
+            assert torch.equal(flat[dst:dst + length], want), (length, n)
+            assert not flat[:dst].any() and not flat[dst + length:].any()
