@@ -131,6 +131,15 @@ uint64_t ft_block_elems(uint64_t count, int world, int elem_size);
  * loads at the same time) and fraction of the kernel's CTAs given to that part */
 void ft_comm_set_hybrid(ft_comm* c, double byte_fraction, double lane_fraction);
 
+/* All ranks of a world whose communicators live on one device (ft_comm_connect_local), in ONE launch: rank r's
+ * contribution is in[r], its result out[r] (may be in[r]).  algo: FT_ALGO_STAGED (any shape; also its halves, phase 1
+ * reduce-scatter and 2 all-gather, on heap tensors), FT_ALGO_ONESHOT, FT_ALGO_LL (with or without a shape),
+ * FT_ALGO_PUSH.  Same results, bit for bit, as the ft_allreduce_emulate_* calls below, rank after rank.
+ * FT_ERR_NOT_AVAILABLE: not a call this form takes (more than 16 ranks, unaligned or overlapping tensors, a limit
+ * exceeded, ...); nothing was launched and the calls below say what is wrong, if anything is. */
+int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void* const* out, size_t count, int dtype, int op,
+                       const int* widths, int nw, int lonely, int ring, int algo, int phase, float scale, void* stream);
+
 /* Single-GPU emulation helper: run only stages [stage_begin, stage_end) of the plan with no
  * rendezvous (the caller serialises ranks and stages on one stream). */
 int ft_allreduce_emulate_stage(ft_comm* c, const void* sendbuf, void* recvbuf, size_t count, int dtype, int op,

@@ -16,12 +16,12 @@ __device__ __forceinline__ void pdl_begin() {
 }
 
 template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const Args&... args) {
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Args&... args) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

@@ -1,0 +1,39 @@
+// What the host hands to world_reduce_kernel (world_reduce.cu): one pass over the copies of all ranks of a world that
+// lives on one device.  Programs are built by planner/world_program.hpp.
+#pragma once
+#include <stdint.h>
+
+namespace ftk {
+
+constexpr int kWorldRanks = 16;      // ranks, and entries of a program, that fit the kernel's parameters
+constexpr int kMaxRounds = 4;        // copies that may be finished after one step
+constexpr uint8_t kNoStore = 0xff;
+
+// Take the next value: start an accumulator with it (a running one is put aside) or add it.  Then `rounds` times:
+// round the accumulator to the element type as a stage of the plan does when it stores a copy, store it as rank
+// store[i]'s copy if that is how the copy ends; between two rounds, and after the last one if `pop`, add the
+// accumulator to the one put aside last.
+struct WorldStep {
+  uint8_t rank, start, rounds, pop;
+  uint8_t store[kMaxRounds];
+};
+// One block's program: its steps, and the ranks that get the result.
+struct WorldEntry {
+  uint16_t block, first, nsteps, scaled;   // scaled: the result is multiplied by the call's scale (float types)
+  uint64_t mask;
+};
+
+// What is left of a step in the kernel's parameters besides the pointer: start | pop << 1 | rounds << 2.
+template <int RANKS>
+struct WorldArgs {
+  void* out[RANKS];
+  WorldEntry entry[RANKS];
+  const void* src[RANKS * RANKS];      // of step k: the copy it takes (any valid pointer behind the last step)
+  uint8_t code[RANKS * RANKS];
+  uint8_t store[RANKS * RANKS][kMaxRounds];
+  uint64_t total_bytes, block_bytes;
+  uint32_t es;
+  float scale;
+};
+
+}  // namespace ftk

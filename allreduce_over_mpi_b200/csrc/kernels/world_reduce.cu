@@ -1,0 +1,188 @@
+// An all-reduce (or one half of it) over the copies of ALL ranks of a world that lives on one device, in one launch.
+//
+// Run stage by stage, the 2*4 tree over eight ranks moves 31 times a rank's bytes and takes 40 launches; the data
+// itself is 16 times a rank's bytes (every input read once, every result written once), and that is what this kernel
+// moves.  HBM bounds it from a few MB up, the launch below.  A thread takes 16 or 32 bytes of one block from every
+// rank, eight loads in flight, evaluates the block's program (planner/world_program.hpp: the plan's own order of
+// additions and roundings) in registers and stores the copies that change.  The program sits in the kernel's
+// parameters, so nothing has to be fetched before the first load; all its branches are uniform across the grid's CTA.
+#include "../api/flextree.h"
+#include "pdl.cuh"
+#include "vec.cuh"
+#include "world_dev.h"
+
+extern "C" void ft_count_launch(uint64_t n);
+
+namespace ftk {
+
+constexpr int kWorldThreads = 128;
+
+// Predicated accesses (no branch, so that the loads of all steps are issued back to back): V 16-byte vectors at p.
+template <int V>
+__device__ __forceinline__ void world_load(const unsigned char* p, bool ok, uint4 (&v)[V]) {
+  if constexpr (V == 2)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %9, 0;\n\t"
+                 "@q ld.global.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t}"
+                 : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w)
+                 : "l"(p), "r"((uint32_t)ok) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+                 "@q ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+                 : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w) : "l"(p), "r"((uint32_t)ok) : "memory");
+}
+template <int V>
+__device__ __forceinline__ void world_store(unsigned char* p, bool ok, const uint4 (&v)[V]) {
+  if constexpr (V == 2)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %9, 0;\n\t@q st.global.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n\t}"
+                 ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
+                   "r"((uint32_t)ok) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q st.global.v4.u32 [%0], {%1,%2,%3,%4};\n\t}"
+                 ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"((uint32_t)ok) : "memory");
+}
+// The last vector of the message, where fewer than V * 16 bytes hold data (one thread per launch): 16 bytes of it.
+// (By value: an array handed over by address would leave the registers.)
+__device__ __noinline__ uint4 tail_load(const unsigned char* p, int valid, uint32_t es) {
+  return ld_partial(p, valid > 16 ? 16u : (valid > 0 ? (uint32_t)valid : 0u), es);
+}
+__device__ __noinline__ void tail_store(unsigned char* p, int valid, uint32_t es, uint4 v) {
+  if (valid > 0) st_partial(p, v, valid > 16 ? 16u : (uint32_t)valid, es);
+}
+
+// blockIdx.y: the program entry.  V: 16-byte vectors per thread and rank; DEPTH: accumulators the program puts aside
+// (0: one flat sum, no step but the first does more than add); G: steps whose loads are in flight together; RANKS: size
+// of the parameters.  At most 128 registers, so that four CTAs of 128 threads fit an SM: with 144 and CTAs of 256 only
+// one did, and the 2*4 tree over eight bf16 buckets of 25 MB took 87 us instead of 66 (6.4 TB/s).
+template <int POL, int V, int DEPTH, int G, int RANKS>
+__global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __grid_constant__ WorldArgs<RANKS> a) {
+  using P = typename PolById<POL>::type;
+  pdl_begin();
+  const int first = a.entry[blockIdx.y].first, nsteps = a.entry[blockIdx.y].nsteps;
+  const uint32_t mask = (uint32_t)a.entry[blockIdx.y].mask;
+  const uint64_t lo = (uint64_t)a.entry[blockIdx.y].block * a.block_bytes;
+  const uint64_t off = lo + ((uint64_t)blockIdx.x * kWorldThreads + threadIdx.x) * (V * 16);
+  const uint64_t end = lo + a.block_bytes < a.total_bytes ? lo + a.block_bytes : a.total_bytes;
+  if (off >= end) return;
+  const uint32_t valid = (uint32_t)(end - off < V * 16 ? end - off : V * 16);
+  const bool full = valid == V * 16;
+  typename P::Acc acc[V], aside[DEPTH > 0 ? DEPTH : 1][V];
+  for (int k0 = 0; k0 < nsteps; k0 += G) {
+    uint4 v[G][V];
+#pragma unroll
+    for (int g = 0; g < G; ++g) world_load<V>((const unsigned char*)a.src[first + k0 + g] + off, full && k0 + g < nsteps, v[g]);
+    if (!full) {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        for (int h = 0; h < V; ++h)
+          if (k0 + g < nsteps) v[g][h] = tail_load((const unsigned char*)a.src[first + k0 + g] + off + h * 16, (int)valid - h * 16, a.es);
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (k0 + g >= nsteps) break;
+      const uint32_t code = DEPTH > 0 ? a.code[first + k0 + g] : (k0 + g == 0);
+      if (code & 1) {
+#pragma unroll
+        for (int h = 0; h < V; ++h) {
+          if (DEPTH > 0) {   // (the first step puts aside a value nothing takes back)
+#pragma unroll
+            for (int d = DEPTH - 1; d > 0; --d) aside[d][h] = aside[d - 1][h];
+            aside[0][h] = acc[h];
+          }
+          P::init(acc[h], v[g][h]);
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < V; ++h) P::add(acc[h], v[g][h]);
+      }
+      if (DEPTH == 0) continue;
+      const int rounds = (int)(code >> 2);
+      for (int r = 0; r < rounds; ++r) {
+        uint4 w[V];
+#pragma unroll
+        for (int h = 0; h < V; ++h) w[h] = P::fin(acc[h]);
+        const uint32_t to = a.store[first + k0 + g][r];
+        if (to != kNoStore) {
+          if (full) world_store<V>((unsigned char*)a.out[to] + off, true, w);
+          else
+#pragma unroll
+            for (int h = 0; h < V; ++h) tail_store((unsigned char*)a.out[to] + off + h * 16, (int)valid - h * 16, a.es, w[h]);
+        }
+        const bool pop = r + 1 < rounds || (code & 2);
+#pragma unroll
+        for (int h = 0; h < V; ++h) {
+          if (pop) {
+            acc[h] = aside[0][h];
+#pragma unroll
+            for (int d = 0; d + 1 < DEPTH; ++d) aside[d][h] = aside[d + 1][h];
+            P::add(acc[h], w[h]);
+          } else {
+            P::init(acc[h], w[h]);
+          }
+        }
+      }
+    }
+  }
+  uint4 w[V];
+#pragma unroll
+  for (int h = 0; h < V; ++h) w[h] = a.entry[blockIdx.y].scaled ? P::fins(acc[h], a.scale) : P::fin(acc[h]);
+#pragma unroll
+  for (int r = 0; r < RANKS; ++r) world_store<V>((unsigned char*)a.out[r] + off, full && (mask >> r & 1), w);
+  if (!full)
+    for (int r = 0; r < RANKS; ++r)
+#pragma unroll
+      for (int h = 0; h < V; ++h)
+        if (mask >> r & 1) tail_store((unsigned char*)a.out[r] + off + h * 16, (int)valid - h * 16, a.es, w[h]);
+}
+
+template <int POL, int V, int DEPTH, int G, int RANKS>
+static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t st) {
+  const uint64_t region = a.block_bytes < a.total_bytes ? a.block_bytes : a.total_bytes;
+  const uint64_t per = (region + (uint64_t)kWorldThreads * V * 16 - 1) / ((uint64_t)kWorldThreads * V * 16);
+  if (per == 0 || per > 0x7fffffffull) return cudaErrorInvalidValue;
+  ft_count_launch(1);
+  return launch_pdl(world_reduce_kernel<POL, V, DEPTH, G, RANKS>, dim3((unsigned)per, (unsigned)entries), kWorldThreads, 0, st, a);
+}
+
+// No more loads in flight and values put aside than the program has: they cost registers, and those CTAs.
+template <int POL, int V, int RANKS>
+static cudaError_t launch_v(const WorldArgs<RANKS>& a, int entries, int depth, int steps, cudaStream_t st) {
+  constexpr bool floats = POL == POL_F32 || POL == POL_BF16 || POL == POL_F16 || POL == POL_F64;
+  if constexpr (RANKS > 8) {
+    return launch_t<POL, V, 3, 8, RANKS>(a, entries, st);
+  } else {
+    if constexpr (POL == POL_OR)
+      if (steps == 1) return launch_t<POL, V, 0, 1, RANKS>(a, entries, st);
+    if constexpr (floats) {
+      if (depth == 0) return steps <= 4 ? launch_t<POL, V, 0, 4, RANKS>(a, entries, st) : launch_t<POL, V, 0, 8, RANKS>(a, entries, st);
+      if (depth == 1) return steps <= 4 ? launch_t<POL, V, 1, 4, RANKS>(a, entries, st) : launch_t<POL, V, 1, 8, RANKS>(a, entries, st);
+    }
+    return launch_t<POL, V, 2, 8, RANKS>(a, entries, st);
+  }
+}
+template <int POL, int RANKS>
+static cudaError_t launch_r(const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st) {
+  if constexpr (RANKS <= 8)
+    if (wide) return launch_v<POL, 2>(a, entries, depth, steps, st);
+  return launch_v<POL, 1>(a, entries, depth, steps, st);
+}
+
+template <int RANKS>
+cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st) {
+  switch (pol) {
+    case POL_ADD8: return launch_r<POL_ADD8>(a, entries, depth, steps, wide, st);
+    case POL_ADD16: return launch_r<POL_ADD16>(a, entries, depth, steps, wide, st);
+    case POL_ADD32: return launch_r<POL_ADD32>(a, entries, depth, steps, wide, st);
+    case POL_ADD64: return launch_r<POL_ADD64>(a, entries, depth, steps, wide, st);
+    case POL_OR: return launch_r<POL_OR>(a, entries, depth, steps, wide, st);
+    case POL_AND: return launch_r<POL_AND>(a, entries, depth, steps, wide, st);
+    case POL_F32: return launch_r<POL_F32>(a, entries, depth, steps, wide, st);
+    case POL_F64: return launch_r<POL_F64>(a, entries, depth, steps, wide, st);
+    case POL_BF16: return launch_r<POL_BF16>(a, entries, depth, steps, wide, st);
+    case POL_F16: return launch_r<POL_F16>(a, entries, depth, steps, wide, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template cudaError_t launch_world<8>(int, const WorldArgs<8>&, int, int, int, bool, cudaStream_t);
+template cudaError_t launch_world<16>(int, const WorldArgs<16>&, int, int, int, bool, cudaStream_t);
+
+}  // namespace ftk

@@ -1,0 +1,216 @@
+// A plan as one pass over the data of every rank, for worlds whose ranks share a device.
+//
+// A plan is element-wise: what a rank's copy of block b becomes depends on the other ranks' copies of block b at the
+// same offset only.  So the whole plan (or one half of it) for one offset is an expression over the ranks' inputs,
+// and one thread that holds the `world` values of an offset can evaluate it and store every copy the plan changes:
+// each input is read once and each result written once, where running the stages one after another moves the
+// intermediate copies through memory as well.
+//
+// build_world_program() executes the plan symbolically and linearises each block's expression, keeping the order of
+// the additions and the places where a copy is stored - and rounded to the element type - between two stages, so
+// that the results are the same bits.  Plans it cannot linearise (a block that ends in two different expressions, a
+// nesting deeper than the kernel's stack) come back with ok = false and are run stage by stage.
+#pragma once
+#include <cstdint>
+#include <map>
+#include <vector>
+
+#include "../kernels/world_dev.h"
+#include "plan.hpp"
+
+namespace ft {
+
+struct WorldProgram {
+  bool ok = false;
+  int depth = 0;                             // 0: plain sums; else the accumulators put aside at the same time, at least 1
+  int widest = 0;                            // steps of the longest entry
+  std::vector<ftk::WorldEntry> entries;      // one per block and pass over it
+  std::vector<ftk::WorldStep> steps;         // entries[i] uses steps [first, first + nsteps)
+};
+
+enum class WorldPhase { all, reduce_scatter, all_gather };
+
+class WorldProgramBuilder {
+ public:
+  explicit WorldProgramBuilder(int world) : world_(world) {
+    for (int r = 0; r < world; ++r) nodes_.push_back(Node{{}, r, false});
+  }
+
+  WorldProgram run(const Plan& p, WorldPhase phase) {
+    WorldProgram out;
+    const int half = p.num_stages / 2, begin = phase == WorldPhase::all_gather ? half : 0;
+    const int end = phase == WorldPhase::reduce_scatter ? half : p.num_stages;
+    for (int b = 0; b < world_; ++b) {
+      std::vector<int> val(world_);
+      for (int r = 0; r < world_; ++r) val[r] = r;   // node r: rank r's copy before the call
+      for (int s = begin; s < end; ++s) {
+        const std::vector<int> before = val;   // a plan reads nothing in a stage that the stage writes
+        for (int r = 0; r < world_; ++r)
+          for (const Pull& pl : p.stages[r][s].pulls) {
+            if (pl.block != b) continue;
+            if (!pl.reduce) { val[r] = before[pl.srcs[0]]; continue; }
+            std::vector<int> kids{val[r]};
+            for (int q : pl.srcs) kids.push_back(before[q]);
+            val[r] = make(kids, s == half - 1);
+          }
+      }
+      if (!(phase == WorldPhase::all_gather ? gather(b, val, &out) : reduce(b, val, phase, &out))) return WorldProgram{};
+    }
+    out.ok = true;
+    return out;
+  }
+
+  // All copies summed in the order first, first + 1, ... (modulo the world) in one go; every rank gets the result.
+  void flat(int block, int first, WorldProgram* out) const {
+    ftk::WorldEntry e{};
+    e.block = (uint16_t)block;
+    e.first = (uint16_t)out->steps.size();
+    e.nsteps = (uint16_t)world_;
+    e.scaled = 1;
+    e.mask = everyone();
+    for (int k = 0; k < world_; ++k) out->steps.push_back(step((first + k) % world_, k == 0));
+    add(e, out);
+    out->ok = true;
+  }
+
+ private:
+  struct Node {
+    std::vector<int> kids;   // empty: the copy of rank `rank`
+    int rank;
+    bool scaled;             // made in the stage that finishes the reduction
+  };
+  static void add(const ftk::WorldEntry& e, WorldProgram* out) {
+    if (e.nsteps > out->widest) out->widest = e.nsteps;
+    out->entries.push_back(e);
+  }
+  uint64_t everyone() const { return world_ >= 64 ? ~0ull : (1ull << world_) - 1; }
+  static ftk::WorldStep step(int rank, bool start) {
+    ftk::WorldStep s{};
+    s.rank = (uint8_t)rank;
+    s.start = start ? 1 : 0;
+    for (uint8_t& d : s.store) d = ftk::kNoStore;
+    return s;
+  }
+  // Equal expressions are one node: ranks that compute the same sum the same way agree.
+  int make(const std::vector<int>& kids, bool scaled) {
+    const auto key = std::make_pair(kids, scaled);
+    auto it = known_.find(key);
+    if (it != known_.end()) return it->second;
+    nodes_.push_back(Node{kids, -1, scaled});
+    return known_[key] = (int)nodes_.size() - 1;
+  }
+  int count(int node, std::vector<int>* leaves) const {
+    if (nodes_[node].kids.empty()) { ++(*leaves)[node]; return 1; }
+    int n = 0;
+    for (int k : nodes_[node].kids) n += count(k, leaves);
+    return n;
+  }
+  bool contains(int root, int node) const {
+    if (root == node) return true;
+    for (int k : nodes_[root].kids)
+      if (contains(k, node)) return true;
+    return false;
+  }
+
+  // Copies only: one entry per source rank that some other rank takes the block from.
+  bool gather(int b, const std::vector<int>& val, WorldProgram* out) const {
+    std::vector<uint64_t> mask(world_, 0);
+    for (int r = 0; r < world_; ++r) {
+      if (val[r] == r) continue;
+      if (val[r] >= world_ || val[val[r]] != val[r]) return false;   // not a copy of a rank that keeps its own
+      mask[val[r]] |= 1ull << r;
+    }
+    for (int q = 0; q < world_; ++q) {
+      if (!mask[q]) continue;
+      ftk::WorldEntry e{};
+      e.block = (uint16_t)b;
+      e.first = (uint16_t)out->steps.size();
+      e.nsteps = 1;
+      e.mask = mask[q];
+      out->steps.push_back(step(q, true));
+      add(e, out);
+    }
+    return true;
+  }
+
+  // One sum; copies that end as part of it are stored where they arise.
+  bool reduce(int b, const std::vector<int>& val, WorldPhase phase, WorldProgram* out) {
+    int root = 0;
+    std::size_t most = 0;
+    for (int r = 0; r < world_; ++r) {
+      std::vector<int> leaves(world_, 0);
+      const std::size_t n = (std::size_t)count(val[r], &leaves);
+      if (n > most) { most = n; root = val[r]; }
+    }
+    std::vector<int> leaves(world_, 0);
+    count(root, &leaves);
+    for (int n : leaves)
+      if (n != 1) return false;
+    if (!nodes_[root].scaled) return false;
+    ftk::WorldEntry e{};
+    e.block = (uint16_t)b;
+    e.first = (uint16_t)out->steps.size();
+    e.scaled = 1;
+    std::map<int, int> partial;   // node -> the rank whose copy ends as it
+    for (int r = 0; r < world_; ++r) {
+      if (val[r] == root) { e.mask |= 1ull << r; continue; }
+      if (val[r] < world_) {
+        if (val[r] != r) return false;   // takes another rank's input: not a reduction's doing
+        continue;
+      }
+      if (phase == WorldPhase::all || !contains(root, val[r]) || nodes_[val[r]].scaled || !partial.emplace(val[r], r).second) return false;
+    }
+    if (phase == WorldPhase::all && e.mask != everyone()) return false;
+    open_ = false;
+    stack_ = 0;
+    if (!eval(root, root, partial, out)) return false;
+    e.nsteps = (uint16_t)(out->steps.size() - e.first);
+    add(e, out);
+    return true;
+  }
+
+  // Append the steps of `node`.  An accumulator that is running already when it starts is put aside.
+  bool eval(int node, int root, const std::map<int, int>& partial, WorldProgram* out) {
+    std::vector<int> kids = nodes_[node].kids;
+    // x + y is y + x: the nested operand first needs no place to put the other one aside (the ring is a chain of these)
+    if (kids.size() == 2 && nodes_[kids[0]].kids.empty() && !nodes_[kids[1]].kids.empty()) std::swap(kids[0], kids[1]);
+    bool first = true;
+    for (int k : kids) {
+      const bool leaf = nodes_[k].kids.empty();
+      if (leaf) {
+        if (first) begin(out, k);
+        else out->steps.push_back(step(k, false));
+      } else {
+        if (!eval(k, root, partial, out)) return false;
+        if (!first) {   // fold the finished operand into the accumulator that was put aside for it
+          out->steps.back().pop = 1;
+          --stack_;
+        }
+      }
+      first = false;
+    }
+    if (node == root) return true;
+    ftk::WorldStep& last = out->steps.back();
+    if (last.rounds >= ftk::kMaxRounds) return false;
+    if (out->depth < 1) out->depth = 1;
+    auto it = partial.find(node);
+    last.store[last.rounds++] = it == partial.end() ? ftk::kNoStore : (uint8_t)it->second;
+    last.pop = 0;
+    return true;
+  }
+  void begin(WorldProgram* out, int leaf) {
+    if (open_) {
+      ++stack_;
+      if (stack_ > out->depth) out->depth = stack_;
+    }
+    open_ = true;
+    out->steps.push_back(step(leaf, true));
+  }
+
+  int world_, stack_ = 0;
+  bool open_ = false;
+  std::vector<Node> nodes_;
+  std::map<std::pair<std::vector<int>, bool>, int> known_;
+};
+
+}  // namespace ft

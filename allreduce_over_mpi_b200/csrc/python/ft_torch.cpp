@@ -33,6 +33,8 @@ namespace {
 int (*p_reduce_nway)(int, int, const void* const*, void*, int, size_t, int, void*) = nullptr;
 int (*p_reduce_nway_scaled)(int, int, const void* const*, void*, int, size_t, float, void*) = nullptr;
 
+int (*p_local_world_run)(void* const*, int, const void* const*, void* const*, size_t, int, int, const int*, int, int, int, int, int, float, void*) = nullptr;
+
 PyObject* other() { Py_RETURN_NOTIMPLEMENTED; }
 
 int dtype_of(at::ScalarType t) {
@@ -155,6 +157,62 @@ PyObject* reduce_nway_scaled(PyObject*, PyObject* const* args, Py_ssize_t nargs)
   return answer(code, args[3], made);
 }
 
+// local_world_run(handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale): `handles` is a list
+// and `widths` a tuple of ints.  None when done; outs is tensors for a call in place.
+PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 10 || !p_local_world_run || !PyList_CheckExact(args[0]) || !PyTuple_CheckExact(args[4])) return other();
+  const Py_ssize_t n = PyList_GET_SIZE(args[0]), nw = PyTuple_GET_SIZE(args[4]);
+  void* handles[FT_MAX_FANIN];
+  int widths[FT_MAX_FANIN];
+  const void *in[FT_MAX_FANIN], *res[FT_MAX_FANIN];
+  const at::Tensor *t0 = nullptr, *o0 = nullptr;
+  if (n > FT_MAX_FANIN || nw > FT_MAX_FANIN) return other();
+  if (gather_inputs(args[1], in, &t0) != n || gather_inputs(args[2], res, &o0) != n) return other();
+  if (o0->scalar_type() != t0->scalar_type() || o0->numel() != t0->numel() || o0->device() != t0->device()) return other();
+  for (Py_ssize_t k = 0; k < n; ++k) handles[k] = PyLong_AsVoidPtr(PyList_GET_ITEM(args[0], k));
+  for (Py_ssize_t k = 0; k < nw; ++k) widths[k] = (int)PyLong_AsLong(PyTuple_GET_ITEM(args[4], k));
+  const int op = op_of(args[3]), dt = dtype_of(t0->scalar_type());
+  const int lonely = (int)PyLong_AsLong(args[5]), ring = (int)PyLong_AsLong(args[6]), algo = (int)PyLong_AsLong(args[7]);
+  const int phase = (int)PyLong_AsLong(args[8]);
+  const double scale = PyFloat_AsDouble(args[9]);
+  if (op < 0 || dt < 0 || PyErr_Occurred()) { PyErr_Clear(); return other(); }
+  int code = 0;
+  Py_BEGIN_ALLOW_THREADS
+  try {
+    c10::cuda::CUDAGuard guard(t0->device());
+    code = p_local_world_run(handles, (int)n, in, const_cast<void* const*>(res), (size_t)t0->numel(), dt, op, widths, (int)nw, lonely, ring, algo,
+                             phase, (float)scale, c10::cuda::getCurrentCUDAStream(t0->device().index()).stream());
+  } catch (...) {
+    code = FT_ERR_NOT_AVAILABLE;
+  }
+  Py_END_ALLOW_THREADS
+  if (code == FT_ERR_NOT_AVAILABLE) return other();
+  if (code) return PyLong_FromLong(code);
+  Py_RETURN_NONE;
+}
+
+// narrow_all(tensors, ranges): for each tensor the list of its flat [lo, hi) views; ranges[k] is a tuple of (lo, hi).
+PyObject* narrow_all(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  const void* ptr[FT_MAX_FANIN];
+  const at::Tensor* t0 = nullptr;
+  if (nargs != 2 || !PyList_CheckExact(args[0]) || !PyTuple_CheckExact(args[1])) return other();
+  const int n = gather_inputs(args[0], ptr, &t0);
+  if (!n || PyTuple_GET_SIZE(args[1]) != n) return other();
+  PyObject* all = PyList_New(n);
+  for (int k = 0; all && k < n; ++k) {
+    const at::Tensor& t = THPVariable_Unpack(PyList_GET_ITEM(args[0], k));
+    PyObject* ranges = PyTuple_GET_ITEM(args[1], k);
+    PyObject* mine = PyList_New(PyTuple_GET_SIZE(ranges));
+    PyList_SET_ITEM(all, k, mine);
+    for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(ranges); ++j) {
+      const int64_t lo = PyLong_AsLongLong(PyTuple_GET_ITEM(PyTuple_GET_ITEM(ranges, j), 0));
+      const int64_t hi = PyLong_AsLongLong(PyTuple_GET_ITEM(PyTuple_GET_ITEM(ranges, j), 1));
+      PyList_SET_ITEM(mine, j, THPVariable_Wrap(t.as_strided({hi - lo}, {1}, t.storage_offset() + lo)));
+    }
+  }
+  return all;
+}
+
 // bind({name: address}): entry points of the libflextree build this process uses.
 PyObject* bind(PyObject*, PyObject* d) {
   if (!PyDict_Check(d)) { PyErr_SetString(PyExc_TypeError, "bind() takes a dict"); return nullptr; }
@@ -164,7 +222,9 @@ PyObject* bind(PyObject*, PyObject* d) {
     fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(PyLong_AsVoidPtr(v));
     return !PyErr_Occurred();
   };
-  if (!get("ft_reduce_nway", p_reduce_nway) || !get("ft_reduce_nway_scaled", p_reduce_nway_scaled)) return nullptr;
+  if (!get("ft_reduce_nway", p_reduce_nway) || !get("ft_reduce_nway_scaled", p_reduce_nway_scaled) ||
+      !get("ft_local_world_run", p_local_world_run))
+    return nullptr;
   Py_RETURN_NONE;
 }
 
@@ -172,6 +232,9 @@ PyMethodDef methods[] = {
     {"bind", bind, METH_O, "bind({name: address})"},
     {"reduce_nway", (PyCFunction)(void (*)(void))reduce_nway, METH_FASTCALL, "reduce_nway(tensors, op, out, variant)"},
     {"reduce_nway_scaled", (PyCFunction)(void (*)(void))reduce_nway_scaled, METH_FASTCALL, "reduce_nway_scaled(tensors, scale, out_dtype, out)"},
+    {"local_world_run", (PyCFunction)(void (*)(void))local_world_run, METH_FASTCALL,
+     "local_world_run(handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)"},
+    {"narrow_all", (PyCFunction)(void (*)(void))narrow_all, METH_FASTCALL, "narrow_all(tensors, ranges)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ft_torch", "native call path of the Python entry points", -1, methods};
 

@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
+#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -28,7 +29,9 @@
 #include "../kernels/comm_bounds.h"
 #include "../kernels/comm_dev.h"
 #include "../kernels/pol_ids.h"
+#include "../kernels/world_dev.h"
 #include "../planner/plan.hpp"
+#include "../planner/world_program.hpp"
 #include "dev_plan.hpp"
 #include "heap_alloc.hpp"
 #include <unistd.h>
@@ -42,6 +45,8 @@ cudaError_t launch_ll(int pol, const CommDev& c, const LLArgs& a, cudaStream_t s
 cudaError_t launch_hybrid(int pol, const CommDev& c, const NvlsArgs& a, int lanes, int nvls_lanes, uint64_t nvls_bytes, cudaStream_t st);
 cudaError_t launch_ll_tree(int pol, const CommDev& c, const LLTreeArgs& a, cudaStream_t st);
 cudaError_t launch_nvls_oneshot(int pol, const CommDev& c, const OneShotArgs& a, uint64_t slot_bytes, int lanes, int threads, cudaStream_t st);
+template <int RANKS>
+cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st);
 cudaError_t launch_wait_probe(const CommDev& c, int peer, unsigned long long timeout_ns, cudaStream_t st);
 }  // namespace ftk
 
@@ -118,6 +123,13 @@ struct DevPlanEntry {
   uint32_t npulls = 0, npushes = 0;
 };
 
+// Program of a world on one device, as asked for (see ft_local_world_run).
+struct WorldProgramEntry {
+  int algo, phase, lonely, ring;
+  std::vector<int> widths;
+  ft::WorldProgram program;
+};
+
 }  // namespace
 
 struct ft_comm {
@@ -159,6 +171,7 @@ struct ft_comm {
   int phase_nvls = 1;         // ft_reduce_scatter / ft_all_gather through the multimem kernels (flat shape, eligible tensor):
                               // 0 never, 1 where it measured faster (five ranks and more), 2 whenever possible     // all-reduce: 0 = rank r owns block r, else round-robin stripes of this many bytes
   std::map<std::string, DevPlanEntry> plans;
+  std::list<WorldProgramEntry> world_programs;   // rank 0 of a world on one device; one per shape and phase in use
   // ft_allreduce_host: chunk buffers in the heap + three streams, made on first use
   struct HostPipe {
     static constexpr int kDepth = 3;
@@ -455,6 +468,50 @@ int launch_ll_call(ft_comm* c, const Prepared& pr, const void* sendbuf, void* re
   cudaError_t e = ftk::launch_ll(pr.pol, c->dev, a, st);
   if (e != cudaSuccess) return fail(c, FT_ERR_CUDA, std::string("low-latency launch: ") + cudaGetErrorString(e));
   return FT_OK;
+}
+
+const ft::WorldProgram* world_program(ft_comm* c, int algo, int phase, const int* widths, int nw, int lonely, int ring) {
+  for (const WorldProgramEntry& w : c->world_programs)
+    if (w.algo == algo && w.phase == phase && w.lonely == lonely && w.ring == ring && (int)w.widths.size() == nw &&
+        std::equal(w.widths.begin(), w.widths.end(), widths))
+      return &w.program;
+  WorldProgramEntry w{algo, phase, lonely, ring, std::vector<int>(widths, widths + nw), {}};
+  ft::WorldProgramBuilder builder(c->world);
+  if (algo == FT_ALGO_PUSH) {
+    for (int b = 0; b < c->world; ++b) builder.flat(b, b, &w.program);
+  } else if (algo == FT_ALGO_ONESHOT || (algo == FT_ALGO_LL && nw == 0)) {
+    builder.flat(0, 0, &w.program);
+  } else {
+    const ft::Plan p = ft::build_plan(c->world, make_shape(c->world, widths, nw, lonely, ring));
+    if (p.ok()) w.program = builder.run(p, (ft::WorldPhase)phase);
+  }
+  c->world_programs.push_back(std::move(w));
+  return &c->world_programs.back().program;
+}
+
+template <int RANKS>
+cudaError_t world_launch(const ft::WorldProgram& wp, int pol, int world, const void* const* in, void* const* out, uint64_t bytes,
+                                uint64_t block_bytes, uint32_t es, float scale, cudaStream_t st) {
+  ftk::WorldArgs<RANKS> a;
+  uintptr_t all = block_bytes;
+  for (int r = 0; r < RANKS; ++r) {
+    a.out[r] = r < world ? out[r] : nullptr;
+    all |= r < world ? (uintptr_t)in[r] | (uintptr_t)out[r] : 0;
+  }
+  std::copy(wp.entries.begin(), wp.entries.end(), a.entry);
+  for (size_t k = 0; k < wp.steps.size(); ++k) {
+    const ftk::WorldStep& s = wp.steps[k];
+    a.src[k] = in[s.rank];
+    a.code[k] = (uint8_t)(s.start | s.pop << 1 | s.rounds << 2);
+    std::copy(s.store, s.store + ftk::kMaxRounds, a.store[k]);
+  }
+  a.total_bytes = bytes;
+  a.block_bytes = block_bytes;
+  a.es = es;
+  a.scale = scale;
+  // 32 bytes per thread once that leaves every SM a few CTAs; below, twice the threads hide more of the latency
+  const bool wide = all % 32 == 0 && bytes >= (2u << 20);
+  return ftk::launch_world<RANKS>(pol, a, (int)wp.entries.size(), wp.depth, wp.widest, wide, st);
 }
 
 }  // namespace
@@ -1121,6 +1178,64 @@ int ft_allreduce_emulate_ll(ft_comm* c, const void* sendbuf, void* recvbuf, size
   if (count == 0) return FT_OK;
   return launch_ll_call(c, pr, sendbuf, recvbuf, count, scale, (uint32_t)phase & 3u, false, call, (cudaStream_t)stream);
 }
+// The rules under which ft_local_world_run may take a call are those under which the per-rank calls it replaces would
+// succeed; whatever they would refuse, or would do differently, is left to them (FT_ERR_NOT_AVAILABLE).
+int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void* const* out, size_t count, int dtype, int op,
+                       const int* widths, int nw, int lonely, int ring, int algo, int phase, float scale, void* stream) {
+#ifdef FT_BOUNDS
+  return FT_ERR_NOT_AVAILABLE;   // the checked build is there to run the kernels that check
+#endif
+  if (!comms || n < 2 || n > ftk::kWorldRanks || !in || !out || !count || phase < 0 || phase > 2) return FT_ERR_NOT_AVAILABLE;
+  ft_comm* c = comms[0];
+  if (!c || !c->finalized || c->world != n || op < 0 || op >= FT_OP_COUNT) return FT_ERR_NOT_AVAILABLE;
+  const int pol = ftk::policy_id(op, dtype);
+  if (pol < 0) return FT_ERR_NOT_AVAILABLE;
+  const uint32_t es = (uint32_t)ft_dtype_size((ft_dtype)dtype);
+  const uint64_t bytes = (uint64_t)count * es;
+  int resident = 0;
+  for (int r = 0; r < n; ++r) {
+    const unsigned char *p = (const unsigned char*)in[r], *q = (const unsigned char*)out[r];
+    if (!comms[r] || !p || !q || (((uintptr_t)p | (uintptr_t)q) & 15)) return FT_ERR_NOT_AVAILABLE;
+    if (in_heap(comms[r], q, bytes)) {
+      if (q - local_base(comms[r]) != (const unsigned char*)out[0] - local_base(c)) return FT_ERR_NOT_AVAILABLE;
+      ++resident;
+    }
+    // results that overlap one another or an input other than exactly: only the per-rank order says what happens
+    for (int k = 0; k < n; ++k) {
+      const unsigned char *a = (const unsigned char*)in[k], *b = (const unsigned char*)out[k];
+      if (k != r && q < b + bytes && b < q + bytes) return FT_ERR_NOT_AVAILABLE;
+      if (q != a && q < a + bytes && a < q + bytes) return FT_ERR_NOT_AVAILABLE;
+    }
+  }
+  if (resident != 0 && resident != n) return FT_ERR_NOT_AVAILABLE;
+  const bool tree = algo == FT_ALGO_STAGED || (algo == FT_ALGO_LL && nw > 0);
+  const bool blocks = tree || algo == FT_ALGO_PUSH;
+  switch (algo) {
+    case FT_ALGO_STAGED: if (!resident && (phase != 0 || bytes > c->staging_bytes)) return FT_ERR_NOT_AVAILABLE; break;
+    case FT_ALGO_ONESHOT: if (bytes > c->staging_bytes) return FT_ERR_NOT_AVAILABLE; break;
+    case FT_ALGO_PUSH: if (!resident) return FT_ERR_NOT_AVAILABLE; break;
+    case FT_ALGO_LL: if (bytes > ftk::kLLMaxBytes) return FT_ERR_NOT_AVAILABLE; break;
+    default: return FT_ERR_NOT_AVAILABLE;
+  }
+  if (phase != 0 && algo != FT_ALGO_STAGED) return FT_ERR_NOT_AVAILABLE;
+  if (algo == FT_ALGO_LL && nw > 0) {   // the tagged-word form of a plan has its own limit on receive slots
+    DevPlanEntry* pe = nullptr;
+    if (get_plan(c, make_shape(n, widths, nw, lonely, ring), &pe) != FT_OK) { c->err.clear(); return FT_ERR_NOT_AVAILABLE; }
+    Prepared pr{pol, es, bytes, resident != 0};
+    if (!ll_tree_fits(c, pr, count, pe->nslots)) return FT_ERR_NOT_AVAILABLE;
+  }
+  const ft::WorldProgram* wp = world_program(c, algo, phase, widths, nw, lonely, ring);
+  const int cap = n <= 8 ? 8 : ftk::kWorldRanks;
+  if (!wp->ok || wp->depth > (n <= 8 ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap) return FT_ERR_NOT_AVAILABLE;
+  if (wp->entries.empty()) return FT_OK;
+  const uint64_t block_bytes = blocks ? pick_block_elems(count, n, es) * es : (bytes + 15) / 16 * 16;
+  // copies move raw words: 16-bit floats do not pass through fp32
+  const int kernel_pol = phase == 2 ? (int)ftk::POL_OR : pol;
+  const cudaError_t e = n <= 8 ? world_launch<8>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
+                               : world_launch<16>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream);
+  return e == cudaSuccess ? FT_OK : fail(c, FT_ERR_CUDA, std::string("world launch: ") + cudaGetErrorString(e));
+}
+
 void ft_comm_set_nvls_ctas_per_sm(ft_comm* c, int n) { if (c && n >= 1 && n <= 3) c->nvls_ctas_per_sm = n; }
 int ft_comm_set_nvls_config(ft_comm* c, int threads, int unroll, int weak, int max_lanes, size_t stripe_bytes) {
   if (!c) return FT_ERR_INVALID_ARG;

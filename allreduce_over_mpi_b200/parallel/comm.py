@@ -18,12 +18,14 @@ Reference counterpart: ``MPI_Allreduce_FT`` and its FT_TOPO / FT_LONELY configur
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 import uuid
 from typing import Sequence
 
 import torch
 
+from .. import _lib
 from .._lib import Choice, FlexTreeError, OPS, lib
 from ..ops.reduce import ft_dtype
 from ..utils import log
@@ -54,11 +56,14 @@ def tensor_from_ptr(ptr: int, shape, dtype: torch.dtype, device, owner=None) -> 
     return flat[:nbytes].view(dtype).view(*shape)
 
 
+_parse_shape = functools.lru_cache(maxsize=256)(Shape.parse)
+
+
 def _as_shape(shape, world) -> Shape | None:
     if shape is None or isinstance(shape, Shape):
         return shape
     if isinstance(shape, str):
-        return None if shape in ("auto", "") else Shape.parse(shape)
+        return None if shape in ("auto", "") else _parse_shape(shape)
     return Shape(tuple(int(x) for x in shape))
 
 
@@ -597,7 +602,19 @@ class FlexTreeComm(_CommBase):
 
 
 class _LocalRank(_CommBase):
-    pass
+    _world_handles: list | None = None   # the world's native handles, void as soon as one rank is closed
+
+    def close(self):
+        if self._world_handles is not None:
+            self._world_handles.clear()
+        super().close()
+
+
+@functools.lru_cache(maxsize=256)
+def _owned_ranges(world: int, shape: Shape, numel: int, elem_size: int) -> tuple:
+    """Per rank, the element ranges of the blocks it holds complete after a reduce-scatter."""
+    B = planner.block_elems_for(numel, world, elem_size)
+    return tuple(tuple((min(numel, b * B), min(numel, (b + 1) * B)) for b in planner.owned_blocks(world, shape, r)) for r in range(world))
 
 
 class LocalWorld:
@@ -605,9 +622,14 @@ class LocalWorld:
 
     ``devices`` lists one CUDA device per rank.  With distinct devices the ranks' kernels really
     run concurrently and rendezvous over NVLink.  With every rank on the SAME device the world is
-    *emulated*: each stage of the plan is launched rank after rank on one stream with the
-    rendezvous switched off, so kernels never wait on one another.
+    *emulated*: one launch evaluates the plan over all ranks' data (:attr:`fused`), or each stage of the
+    plan is launched rank after rank on one stream with the rendezvous switched off.  Either way no kernel
+    waits on another, and the results are the same bits.
     """
+
+    #: Emulated worlds: one launch over all ranks' data where the call allows it.  Off: every call goes stage by
+    #: stage, rank by rank, through the kernels that several devices would run.
+    fused = True
 
     def __init__(self, world: int, devices: Sequence[int] | None = None, heap_bytes: int = 64 << 20,
                  staging_bytes: int = 16 << 20, mem: str = "ipc"):
@@ -629,6 +651,19 @@ class LocalWorld:
         if code:
             raise FlexTreeError(code, lib().ft_comm_last_error(self.ranks[0]._h).decode())
         self._emu_call = 0
+        self._handles = [c._h.value for c in self.ranks]
+        for c in self.ranks:
+            c._world_handles = self._handles
+
+    def _run_fused(self, tensors, outs, op, shape: Shape | None, algo: int, phase: int, scale: float) -> bool:
+        """The whole call in one launch (ft_local_world_run); False: not a call it takes."""
+        widths, lonely, ring = (shape.widths, shape.lonely, int(shape.ring)) if shape is not None else ((), 0, 0)
+        code = (_lib._native or _lib.native()).local_world_run(self._handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)
+        if code is None:
+            return True
+        if code is not NotImplemented:
+            raise FlexTreeError(code, lib().ft_comm_last_error(self.ranks[0]._h).decode())
+        return False
 
     def all_reduce(self, tensors: Sequence[torch.Tensor], op: str = "sum", shape=None, algo: str = "staged",
                    scale: float = 1.0, outs: Sequence[torch.Tensor] | None = None):
@@ -643,6 +678,8 @@ class LocalWorld:
                 with torch.cuda.device(c.device):
                     c.all_reduce(tensors[r], op=op, shape=shp if algo == "staged" or (algo == "ll" and shape is not None) else None,
                                  algo=algo, scale=scale, out=outs[r])
+            return outs
+        if self.fused and self._run_fused(tensors, outs, op, shp if shape is not None or algo == "staged" else None, ALGOS.get(algo, -1), 0, scale):
             return outs
         L = lib()
         dt = ft_dtype(tensors[0].dtype)
@@ -717,6 +754,8 @@ class LocalWorld:
                     else:
                         c.reduce_scatter(tensors[r], op=op, shape=shp, scale=scale)
             return shp
+        if self.fused and self._run_fused(tensors, tensors, op, shp, ALGOS["staged"], 2 if gather else 1, scale):
+            return shp
         nstages = planner.plan_num_stages(world, shp)
         if nstages < 0:
             raise FlexTreeError(4, f"invalid FT_TOPO {shp} ({planner.validate_shape(world, shp)})")
@@ -734,6 +773,10 @@ class LocalWorld:
     def reduce_scatter(self, tensors: Sequence[torch.Tensor], op: str = "sum", shape=None, scale: float = 1.0):
         """Reduce-scatter half alone; returns, per rank, the views of the blocks it holds complete."""
         shp = self._phase(tensors, False, op, shape, scale)
+        t0 = tensors[0]
+        views = (_lib._native or _lib.native()).narrow_all(tensors, _owned_ranges(self.world, shp, t0.numel(), t0.element_size()))
+        if views is not NotImplemented:
+            return views
         out = []
         for r, c in enumerate(self.ranks):
             flat = tensors[r].view(-1)

@@ -1,0 +1,92 @@
+"""A world on one device: the one-launch form against the kernels that several devices would run.
+
+The tests of test_comm_emulated_gpu.py call whatever ``LocalWorld`` runs by default, the one-launch form; they are
+collected here a second time with it switched off, so that the multi-GPU kernels stay covered on one GPU."""
+import pytest
+import torch
+
+import test_comm_emulated_gpu as emulated
+from allreduce_over_mpi_b200.ops import launch_count
+from allreduce_over_mpi_b200.parallel.comm import LocalWorld
+from allreduce_over_mpi_b200.parallel.planner import Shape
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class TestStageByStage:
+    @pytest.fixture(autouse=True)
+    def unfused(self, monkeypatch):
+        monkeypatch.setattr(LocalWorld, "fused", False)
+
+    for _name in dir(emulated):
+        if _name.startswith("test_"):
+            locals()[_name] = staticmethod(getattr(emulated, _name))
+
+
+def both(world, make, call):
+    """The results of `call(world, tensors)` with and without the one-launch form, and how many launches it took."""
+    got = []
+    for fused in (True, False):
+        w = LocalWorld(world, heap_bytes=4 << 20, staging_bytes=4 << 20)
+        w.fused = fused
+        ts = make(w)
+        before = launch_count()
+        res = call(w, ts)
+        torch.cuda.synchronize()
+        got.append(([t.clone() for t in res], launch_count() - before))
+        w.close()
+    (a, launches), (b, _) = got
+    assert all(torch.equal(x.view(torch.uint8), y.view(torch.uint8)) for x, y in zip(a, b))
+    return launches
+
+
+def tensors(world, count, dtype, heap):
+    def make(w):
+        g = torch.Generator(device=DEV).manual_seed(count)
+        out = []
+        for c in w.ranks:
+            x = (torch.randn(count, generator=g, device=DEV) * 20).to(dtype)
+            out.append(c.alloc(count, dtype).copy_(x) if heap else x)
+        return out
+    return make
+
+
+@pytest.mark.parametrize("text", emulated.SHAPES + ["ring16", "2*2*2*2"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_every_shape_same_bits(text, dtype):
+    n = Shape.parse(text).world
+    for count in (35, 4099, 600_000):
+        for heap in (False, True):
+            make = tensors(n, count, dtype, heap)
+            assert both(n, make, lambda w, ts: w.all_reduce(ts, op="avg", shape=text)) == 1
+            if heap:
+                assert both(n, make, lambda w, ts: (w.reduce_scatter(ts, op="avg", shape=text), ts)[1]) == 1
+                assert both(n, make, lambda w, ts: w.all_gather(ts, shape=text)) == 1
+            elif count <= 4099:
+                assert both(n, make, lambda w, ts: w.all_reduce(ts, shape=text, algo="ll", outs=[torch.empty_like(t) for t in ts])) == 1
+
+
+@pytest.mark.parametrize("algo", ["oneshot", "ll", "push"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float64, torch.int64, torch.uint8])
+def test_flat_algorithms_same_bits(algo, dtype):
+    for world in (2, 7, 8, 11):
+        for count in (1, 20_001):
+            make = tensors(world, count, dtype, algo == "push")
+            assert both(world, make, lambda w, ts: w.all_reduce(ts, op="avg" if dtype.is_floating_point else "sum", algo=algo)) == 1
+
+
+def test_calls_it_does_not_take_go_stage_by_stage():
+    base = torch.randn(4, 2048, device=DEV)
+    shifted = lambda w: [b[1:2000] for b in base.clone()]   # noqa: E731 - off a 16-byte boundary
+    assert both(4, shifted, lambda w, ts: w.all_reduce(ts, shape="2*2")) > 1
+
+    def overlapping(w):   # rank 1's result starts inside rank 0's input
+        flat = base.clone().view(-1)
+        return [flat[0:1024], flat[2048:3072], flat[512:1536], flat[4096:5120]]
+    assert both(2, overlapping, lambda w, ts: w.all_reduce(ts[:2], shape="2", outs=ts[2:])) > 1
+    w = LocalWorld(2, heap_bytes=1 << 20, staging_bytes=1 << 20)
+    w.ranks[1].close()
+    with pytest.raises(Exception):
+        w.all_reduce([base[0], base[1]], shape="2")
+    w.close()
