@@ -151,7 +151,7 @@ def lib() -> C.CDLL:
 
 
 #: entry points that the native call path (csrc/python/ft_torch.cpp) calls
-_NATIVE = ("ft_reduce_nway", "ft_reduce_nway_scaled", "ft_local_world_run")
+_NATIVE = ("ft_reduce_nway", "ft_reduce_nway_scaled", "ft_local_world_run", "ft_host_pipe_reduce")
 
 
 def native():

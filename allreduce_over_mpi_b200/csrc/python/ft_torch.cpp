@@ -35,6 +35,8 @@ int (*p_reduce_nway_scaled)(int, int, const void* const*, void*, int, size_t, fl
 
 int (*p_local_world_run)(void* const*, int, const void* const*, void* const*, size_t, int, int, const int*, int, int, int, int, int, float, void*) = nullptr;
 
+int (*p_host_pipe_reduce)(void*, int, int, const void* const*, int, const int*, void* const*, int, size_t, void*) = nullptr;
+
 PyObject* other() { Py_RETURN_NOTIMPLEMENTED; }
 
 int dtype_of(at::ScalarType t) {
@@ -191,6 +193,52 @@ PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Py_RETURN_NONE;
 }
 
+// Plain, contiguous CPU tensors that share type and size with *first (set by the first one).  Returns their number, or 0.
+int gather_host(PyObject* seq, const void** ptr, const at::Tensor** first) {
+  const bool list = PyList_CheckExact(seq);
+  if (!list && !PyTuple_CheckExact(seq)) return 0;
+  const Py_ssize_t n = list ? PyList_GET_SIZE(seq) : PyTuple_GET_SIZE(seq);
+  if (n < 1 || n > FT_MAX_FANIN) return 0;
+  for (Py_ssize_t k = 0; k < n; ++k) {
+    PyObject* o = list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k);
+    if (!THPVariable_CheckExact(o)) return 0;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cpu() || t.layout() != at::kStrided || !t.is_contiguous()) return 0;
+    if (!*first) *first = &t;
+    else if (t.scalar_type() != (*first)->scalar_type() || t.numel() != (*first)->numel()) return 0;
+    ptr[k] = t.const_data_ptr();
+  }
+  return (int)n;
+}
+
+// host_pipe_run(pipeline, device, inputs, fanins, outs, op): on the current stream of `device`.  None when done.
+PyObject* host_pipe_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 6 || !p_host_pipe_reduce || !PyList_CheckExact(args[3])) return other();
+  const void *src[FT_MAX_FANIN], *dst[FT_MAX_FANIN];
+  int fanin[FT_MAX_FANIN];
+  const at::Tensor* t0 = nullptr;
+  const int n_in = gather_host(args[2], src, &t0), n_out = n_in ? gather_host(args[4], dst, &t0) : 0;
+  if (!n_out || PyList_GET_SIZE(args[3]) != n_out) return other();
+  for (int j = 0; j < n_out; ++j) fanin[j] = (int)PyLong_AsLong(PyList_GET_ITEM(args[3], j));
+  void* pipe = PyLong_AsVoidPtr(args[0]);
+  const long device = PyLong_AsLong(args[1]);
+  const int op = op_of(args[5]), dt = dtype_of(t0->scalar_type());
+  if (!pipe || op < 0 || dt < 0 || PyErr_Occurred()) { PyErr_Clear(); return other(); }
+  int code = 0;
+  Py_BEGIN_ALLOW_THREADS
+  try {
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    code = p_host_pipe_reduce(pipe, op, dt, src, n_in, fanin, const_cast<void* const*>(dst), n_out, (size_t)t0->numel(),
+                              c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream());
+  } catch (...) {
+    code = -1;
+  }
+  Py_END_ALLOW_THREADS
+  if (code < 0) return other();
+  if (code) return PyLong_FromLong(code);
+  Py_RETURN_NONE;
+}
+
 // narrow_all(tensors, ranges): for each tensor the list of its flat [lo, hi) views; ranges[k] is a tuple of (lo, hi).
 PyObject* narrow_all(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const void* ptr[FT_MAX_FANIN];
@@ -223,7 +271,7 @@ PyObject* bind(PyObject*, PyObject* d) {
     return !PyErr_Occurred();
   };
   if (!get("ft_reduce_nway", p_reduce_nway) || !get("ft_reduce_nway_scaled", p_reduce_nway_scaled) ||
-      !get("ft_local_world_run", p_local_world_run))
+      !get("ft_local_world_run", p_local_world_run) || !get("ft_host_pipe_reduce", p_host_pipe_reduce))
     return nullptr;
   Py_RETURN_NONE;
 }
@@ -234,6 +282,7 @@ PyMethodDef methods[] = {
     {"reduce_nway_scaled", (PyCFunction)(void (*)(void))reduce_nway_scaled, METH_FASTCALL, "reduce_nway_scaled(tensors, scale, out_dtype, out)"},
     {"local_world_run", (PyCFunction)(void (*)(void))local_world_run, METH_FASTCALL,
      "local_world_run(handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)"},
+    {"host_pipe_run", (PyCFunction)(void (*)(void))host_pipe_run, METH_FASTCALL, "host_pipe_run(pipeline, device, inputs, fanins, outs, op)"},
     {"narrow_all", (PyCFunction)(void (*)(void))narrow_all, METH_FASTCALL, "narrow_all(tensors, ranges)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ft_torch", "native call path of the Python entry points", -1, methods};

@@ -6,6 +6,9 @@
 // time.  Here the vectors are cut into chunks that rotate through a small ring of device buffers on
 // three streams: while chunk k is being reduced, chunk k+1 arrives and the results of chunk k-1
 // leave, so a step costs about max(bytes in, bytes out) / link rate instead of their sum.
+//
+// Operands in pinned memory need none of that: one kernel reads and writes them over the link (kernels/host_prefix.cu).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -13,6 +16,8 @@
 #include <vector>
 
 #include "../api/flextree.h"
+#include "../kernels/host_prefix.h"
+#include "../kernels/pol_ids.h"
 
 struct ft_host_pipe {
   static constexpr int kDepth = 3;
@@ -37,6 +42,59 @@ int fail(ft_host_pipe* p, int code, const std::string& what) {
     cudaError_t e_ = (call);                                                                          \
     if (e_ != cudaSuccess) return fail(p, FT_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
+
+// Address the GPU may use for `bytes` bytes of host memory at p; null unless all of them lie in one pinned allocation.
+// Asked on every call: memory that was pinned a moment ago may have been freed since.
+unsigned char* pinned_address(const void* p, size_t bytes) {
+  using Fn = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Fn get = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return (Fn)fn;
+  }();
+  if (!get) return nullptr;
+  CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  unsigned int type = 0;
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  void* to[4] = {&type, &dev, &start, &size};
+  if (get(4, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return nullptr;
+  if (type != CU_MEMORYTYPE_HOST || !dev || !start) return nullptr;
+  const uintptr_t at = (uintptr_t)p;
+  if (at < start || at + bytes > start + size) return nullptr;
+  return (unsigned char*)(uintptr_t)dev;
+}
+
+// The call as one kernel; FT_ERR_NOT_AVAILABLE when some operand is not pinned or not on a 16-byte boundary.
+int run_direct(int op, int dtype, const void* const* src, const int* fanin, void* const* dst, int n_out, size_t bytes, size_t es,
+               cudaStream_t st) {
+  const int pol = ftk::policy_id(op, dtype);
+  if (pol < 0) return FT_ERR_NOT_AVAILABLE;
+  ftk::HostPrefixArgs a;
+  a.n_in = 0;
+  for (int j = 0; j < n_out; ++j)
+    if (fanin[j] > a.n_in) a.n_in = fanin[j];
+  for (int k = 0; k < a.n_in; ++k)
+    if (((uintptr_t)src[k] & 15) || !(a.in[k] = pinned_address(src[k], bytes))) return FT_ERR_NOT_AVAILABLE;
+  int filled = 0;
+  for (int k = 0; k < a.n_in; ++k) {
+    a.first[k] = (uint8_t)filled;
+    for (int j = 0; j < n_out; ++j) {
+      if (fanin[j] != k + 1) continue;
+      if (((uintptr_t)dst[j] & 15) || !(a.out[filled++] = pinned_address(dst[j], bytes))) return FT_ERR_NOT_AVAILABLE;
+    }
+  }
+  a.first[a.n_in] = (uint8_t)filled;
+  a.bytes = bytes;
+  a.es = (uint32_t)es;
+  const cudaError_t e = ftk::launch_host_prefix(pol, a, st);
+  return e == cudaSuccess ? FT_OK : FT_ERR_CUDA;
+}
 }  // namespace
 
 extern "C" {
@@ -92,6 +150,8 @@ int ft_host_pipe_reduce(ft_host_pipe* p, int op, int dtype, const void* const* h
     if (fanin[j] < 1 || fanin[j] > n_in) return fail(p, FT_ERR_INVALID_ARG, "fan-in outside 1..n_in");
   if (len == 0) return FT_OK;
   HP_CUDA(p, cudaSetDevice(p->device));
+  if (const int rc = run_direct(op, dtype, host_src, fanin, host_dst, n_out, len * es, es, (cudaStream_t)stream); rc != FT_ERR_NOT_AVAILABLE)
+    return rc == FT_OK ? rc : fail(p, rc, cudaGetErrorString(cudaGetLastError()));
   constexpr int D = ft_host_pipe::kDepth;
   const size_t per = p->chunk_bytes / es;
   cudaStream_t user = (cudaStream_t)stream;

@@ -125,10 +125,11 @@ class HostReducePipeline:
     """n-way reductions of vectors that live in pinned HOST memory, streamed through one GPU.
 
     ``run(inputs, fanins, outs)`` computes ``outs[j] = inputs[0] (op) ... (op) inputs[fanins[j]-1]`` for every j.
-    The vectors are cut into chunks; the host-to-device copy of chunk k+1, the reductions of chunk k and the
-    device-to-host copy of chunk k-1 run at the same time on three streams (native: csrc/runtime/host_pipeline.cpp),
-    so a call costs about max(bytes in, bytes out) over the PCIe rate, where copy in / kernel / copy out one after
-    the other (what the reference's benchmark does, vector_add/vector_add.cu:81-136) costs their sum.
+    Pinned vectors on 16-byte boundaries go through one kernel that reads and writes them over PCIe
+    (csrc/kernels/host_prefix.cu).  Others are cut into chunks; the host-to-device copy of chunk k+1, the reductions of
+    chunk k and the device-to-host copy of chunk k-1 run at the same time on three streams (csrc/runtime/host_pipeline.cpp).
+    Either way a call costs about max(bytes in, bytes out) over the PCIe rate, where copy in / kernel / copy out one
+    after the other (what the reference's benchmark does, vector_add/vector_add.cu:81-136) costs their sum.
     """
 
     def __init__(self, device=None, chunk_bytes: int = 16 << 20, max_inputs: int = 8, max_outputs: int = 4):
@@ -146,6 +147,12 @@ class HostReducePipeline:
             stream: torch.cuda.Stream | None = None) -> Sequence[torch.Tensor]:
         """Asynchronous for pinned tensors: the results are complete once ``stream`` (default: the current
         stream of the pipeline's device) has been synchronised."""
+        if stream is None and self._h:
+            code = (_lib._native or _lib.native()).host_pipe_run(self._h.value, self.device.index or 0, inputs, fanins, outs, op)
+            if code is None:
+                return outs
+            if code is not NotImplemented:
+                check(code, lib().ft_host_pipe_last_error(self._h).decode())
         t0 = inputs[0]
         for t in list(inputs) + list(outs):
             if t.is_cuda or not t.is_contiguous() or t.dtype != t0.dtype or t.numel() != t0.numel():

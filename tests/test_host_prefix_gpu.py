@@ -1,0 +1,44 @@
+"""Prefix reductions of host vectors: pinned and aligned (one kernel over PCIe) or not (chunked copies), same results."""
+import pytest
+import torch
+
+from allreduce_over_mpi_b200.ops import HostReducePipeline, launch_count, reduce_nway
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype,op", [(torch.float32, "sum"), (torch.bfloat16, "sum"), (torch.float64, "sum"), (torch.int16, "sum"),
+                                      (torch.uint8, "band"), (torch.int64, "band")])
+@pytest.mark.parametrize("n,fanins", [(1, [1]), (8, [2, 3, 4, 8]), (9, [9, 1, 9]), (12, [5])])
+def test_pinned_pageable_and_unaligned(dtype, op, n, fanins):
+    for length in (1, 15, 4099, 70_003):
+        g = torch.Generator().manual_seed(length)
+        vecs = [torch.randint(0, 100, (length,), generator=g).to(dtype) for _ in range(n)]
+        want = [reduce_nway([v.to(DEV) for v in vecs[:f]], op=op).cpu() for f in fanins]
+        pipe = HostReducePipeline(device=DEV, chunk_bytes=64 << 10, max_inputs=n, max_outputs=len(fanins))
+        for kind in ("pinned", "pageable", "unaligned", "mixed"):
+            pin = kind in ("pinned", "unaligned")
+            off = 1 if kind == "unaligned" else 0
+            hin = [torch.empty(length + off, dtype=dtype, pin_memory=pin or (kind == "mixed" and k == 0))[off:].copy_(v) for k, v in enumerate(vecs)]
+            flat = [torch.zeros(length + 16 + off, dtype=dtype, pin_memory=pin) for _ in fanins]
+            outs = [f[off:length + off] for f in flat]
+            before = launch_count()
+            pipe.run(hin, fanins, outs, op=op)
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, w) for o, w in zip(outs, want)), (kind, length)
+            assert not any(f[length + off:].any() for f in flat)
+            if kind == "pinned":
+                assert launch_count() == before + 1
+        pipe.close()
+
+
+def test_in_place_and_own_stream():
+    hin = [torch.randn(100_003).pin_memory() for _ in range(3)]
+    want = (hin[0].to(DEV) + hin[1].to(DEV) + hin[2].to(DEV)).cpu()
+    pipe = HostReducePipeline(device=DEV, max_inputs=3, max_outputs=1)
+    st = torch.cuda.Stream()
+    pipe.run(hin, [3], [hin[1]], stream=st)
+    st.synchronize()
+    assert torch.equal(hin[1], want)
+    pipe.close()
