@@ -21,11 +21,11 @@ template <int POL>
 __global__ void __launch_bounds__(256) host_prefix_kernel(const __grid_constant__ HostPrefixArgs a) {
   using P = typename PolById<POL>::type;
   pdl_begin();
-  const uint64_t nvec = (a.bytes + 15) / 16;
+  const uint64_t nvec = a.bytes / 16, items = nvec + a.bytes % 16 / a.es;   // whole vectors, then single elements
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
-    const uint64_t off = i * 16;
-    const uint32_t valid = (uint32_t)(a.bytes - off < 16 ? a.bytes - off : 16);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += stride) {
+    const bool full = i < nvec;
+    const uint64_t off = full ? i * 16 : nvec * 16 + (i - nvec) * a.es;
     typename P::Acc acc;
     constexpr int G = 8;
     for (int k0 = 0; k0 < a.n_in; k0 += G) {
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) host_prefix_kernel(const __grid_constant_
       for (int g = 0; g < G; ++g)
         if (k0 + g < a.n_in) {
           const unsigned char* p = (const unsigned char*)a.in[k0 + g] + off;
-          v[g] = valid == 16 ? ld_stream(p) : ld_partial(p, valid, a.es);
+          v[g] = full ? ld_stream(p) : ld_element(p, a.es);
         }
 #pragma unroll
       for (int g = 0; g < G; ++g) {
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) host_prefix_kernel(const __grid_constant_
         else P::add(acc, v[g]);
         for (int j = a.first[k0 + g]; j < a.first[k0 + g + 1]; ++j) {   // the results that end with this input
           unsigned char* q = (unsigned char*)a.out[j] + off;
-          if (valid == 16) st_vec(q, P::fin(acc));
-          else st_partial(q, P::fin(acc), valid, a.es);
+          if (full) st_vec(q, P::fin(acc));
+          else st_element(q, P::fin(acc), a.es);
         }
       }
     }
@@ -53,9 +53,9 @@ __global__ void __launch_bounds__(256) host_prefix_kernel(const __grid_constant_
 
 template <int POL>
 static cudaError_t launch_t(const HostPrefixArgs& a, cudaStream_t st) {
-  const uint64_t nvec = (a.bytes + 15) / 16;
+  const uint64_t items = a.bytes / 16 + a.bytes % 16 / a.es;
   // 256 KB of loads in flight: 8 CTAs of 256 threads with eight inputs, more with fewer
-  uint64_t grid = 64 / (a.n_in < 8 ? a.n_in : 8), want = (nvec + 255) / 256;
+  uint64_t grid = 64 / (a.n_in < 8 ? a.n_in : 8), want = (items + 255) / 256;
   if (grid > want) grid = want;
   ft_count_launch(1);
   return launch_pdl(host_prefix_kernel<POL>, (unsigned)grid, 256, 0, st, a);

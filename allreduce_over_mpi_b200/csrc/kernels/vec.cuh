@@ -62,6 +62,24 @@ __device__ __forceinline__ uint4 ld_partial(const void* p, uint32_t nbytes, uint
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// One element in the low bytes of a vector (the rest zero), and back: the vector policies work on it as on any vector.
+// The elements behind the last whole vector of a message go this way, one thread each, so that their loads are in
+// flight together (ld_partial / st_partial walk a partial vector byte by byte in one thread).
+__device__ __forceinline__ uint4 ld_element(const void* p, uint32_t es) {
+  uint32_t x = 0, y = 0;
+  if (es == 8) asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "l"(p) : "memory");
+  else if (es == 4) asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  else if (es == 2) { uint16_t h; asm volatile("ld.global.L1::no_allocate.u16 %0, [%1];" : "=h"(h) : "l"(p) : "memory"); x = h; }
+  else asm volatile("ld.global.L1::no_allocate.u8 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  return make_uint4(x, y, 0, 0);
+}
+__device__ __forceinline__ void st_element(void* p, uint4 v, uint32_t es) {
+  if (es == 8) asm volatile("st.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+  else if (es == 4) *(volatile uint32_t*)p = v.x;
+  else if (es == 2) *(volatile uint16_t*)p = (uint16_t)v.x;
+  else *(volatile uint8_t*)p = (uint8_t)v.x;
+}
+
 // ---- element types --------------------------------------------------------------------
 template <int DT> struct ElemOf;
 template <> struct ElemOf<FT_U8> { using type = uint8_t; };

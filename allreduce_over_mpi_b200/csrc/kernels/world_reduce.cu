@@ -6,6 +6,8 @@
 // rank, eight loads in flight, evaluates the block's program (planner/world_program.hpp: the plan's own order of
 // additions and roundings) in registers and stores the copies that change.  The program sits in the kernel's
 // parameters, so nothing has to be fetched before the first load; all its branches are uniform across the grid's CTA.
+#include <algorithm>
+
 #include "../api/flextree.h"
 #include "pdl.cuh"
 #include "vec.cuh"
@@ -40,15 +42,6 @@ __device__ __forceinline__ void world_store(unsigned char* p, bool ok, const uin
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q st.global.v4.u32 [%0], {%1,%2,%3,%4};\n\t}"
                  ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"((uint32_t)ok) : "memory");
 }
-// The last vector of the message, where fewer than V * 16 bytes hold data (one thread per launch): 16 bytes of it.
-// (By value: an array handed over by address would leave the registers.)
-__device__ __noinline__ uint4 tail_load(const unsigned char* p, int valid, uint32_t es) {
-  return ld_partial(p, valid > 16 ? 16u : (valid > 0 ? (uint32_t)valid : 0u), es);
-}
-__device__ __noinline__ void tail_store(unsigned char* p, int valid, uint32_t es, uint4 v) {
-  if (valid > 0) st_partial(p, v, valid > 16 ? 16u : (uint32_t)valid, es);
-}
-
 // blockIdx.y: the program entry.  V: 16-byte vectors per thread and rank; DEPTH: accumulators the program puts aside
 // (0: one flat sum, no step but the first does more than add); G: steps whose loads are in flight together; RANKS: size
 // of the parameters.  At most 128 registers, so that four CTAs of 128 threads fit an SM: with 144 and CTAs of 256 only
@@ -60,11 +53,13 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
   const int first = a.entry[blockIdx.y].first, nsteps = a.entry[blockIdx.y].nsteps;
   const uint32_t mask = (uint32_t)a.entry[blockIdx.y].mask;
   const uint64_t lo = (uint64_t)a.entry[blockIdx.y].block * a.block_bytes;
-  const uint64_t off = lo + ((uint64_t)blockIdx.x * kWorldThreads + threadIdx.x) * (V * 16);
   const uint64_t end = lo + a.block_bytes < a.total_bytes ? lo + a.block_bytes : a.total_bytes;
+  if (lo >= end) return;
+  // whole vectors first, then the elements behind the last one, a thread each
+  const uint64_t i = (uint64_t)blockIdx.x * kWorldThreads + threadIdx.x, whole = (end - lo) / (V * 16);
+  const bool full = i < whole;
+  const uint64_t off = lo + (full ? i * (V * 16) : whole * (V * 16) + (i - whole) * a.es);
   if (off >= end) return;
-  const uint32_t valid = (uint32_t)(end - off < V * 16 ? end - off : V * 16);
-  const bool full = valid == V * 16;
   typename P::Acc acc[V], aside[DEPTH > 0 ? DEPTH : 1][V];
   for (int k0 = 0; k0 < nsteps; k0 += G) {
     uint4 v[G][V];
@@ -73,8 +68,7 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
     if (!full) {
 #pragma unroll
       for (int g = 0; g < G; ++g)
-        for (int h = 0; h < V; ++h)
-          if (k0 + g < nsteps) v[g][h] = tail_load((const unsigned char*)a.src[first + k0 + g] + off + h * 16, (int)valid - h * 16, a.es);
+        if (k0 + g < nsteps) v[g][0] = ld_element((const unsigned char*)a.src[first + k0 + g] + off, a.es);
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -103,9 +97,7 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
         const uint32_t to = a.store[first + k0 + g][r];
         if (to != kNoStore) {
           if (full) world_store<V>((unsigned char*)a.out[to] + off, true, w);
-          else
-#pragma unroll
-            for (int h = 0; h < V; ++h) tail_store((unsigned char*)a.out[to] + off + h * 16, (int)valid - h * 16, a.es, w[h]);
+          else st_element((unsigned char*)a.out[to] + off, w[0], a.es);
         }
         const bool pop = r + 1 < rounds || (code & 2);
 #pragma unroll
@@ -129,15 +121,15 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
   for (int r = 0; r < RANKS; ++r) world_store<V>((unsigned char*)a.out[r] + off, full && (mask >> r & 1), w);
   if (!full)
     for (int r = 0; r < RANKS; ++r)
-#pragma unroll
-      for (int h = 0; h < V; ++h)
-        if (mask >> r & 1) tail_store((unsigned char*)a.out[r] + off + h * 16, (int)valid - h * 16, a.es, w[h]);
+      if (mask >> r & 1) st_element((unsigned char*)a.out[r] + off, w[0], a.es);
 }
 
 template <int POL, int V, int DEPTH, int G, int RANKS>
 static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t st) {
-  const uint64_t region = a.block_bytes < a.total_bytes ? a.block_bytes : a.total_bytes;
-  const uint64_t per = (region + (uint64_t)kWorldThreads * V * 16 - 1) / ((uint64_t)kWorldThreads * V * 16);
+  // threads of the longest block: the first one's vectors, or the last one's vectors and elements
+  const uint64_t last = (a.total_bytes - 1) % a.block_bytes + 1;
+  const uint64_t most = std::max(a.total_bytes > a.block_bytes ? a.block_bytes / (V * 16) : 0, last / (V * 16) + last % (V * 16) / a.es);
+  const uint64_t per = (most + kWorldThreads - 1) / kWorldThreads;
   if (per == 0 || per > 0x7fffffffull) return cudaErrorInvalidValue;
   ft_count_launch(1);
   return launch_pdl(world_reduce_kernel<POL, V, DEPTH, G, RANKS>, dim3((unsigned)per, (unsigned)entries), kWorldThreads, 0, st, a);

@@ -191,7 +191,7 @@ def e2e_nway(a, vecs, step_bytes) -> dict:
     d2h = sum(h.numel() * h.element_size() for h in host_out)
     return {"value": round(step_bytes / (ms * 1e-3) / 1e9, 1), "unit": "GB/s", "ms_per_step": round(ms, 3),
             "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "steps": steps, "max_abs_err": err,
-            "api": "ops.HostReducePipeline.run (pinned host in, pinned host out, chunked and overlapped)",
+            "api": "ops.HostReducePipeline.run (pinned host in, pinned host out, both directions of PCIe at once)",
             "chunk_bytes": a.e2e_chunk}
 
 
