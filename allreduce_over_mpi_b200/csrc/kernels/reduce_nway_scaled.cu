@@ -1,17 +1,19 @@
 // out = scale * sum_k src[k] on one GPU, fp32 accumulation, fp32 or bf16 in and out (gradient averaging with the cast
 // fused into the store).
 //
-// HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, up to
-// eight sources in flight, the grid covers the vector once, edges in a CTA of their own, dependent launch.  The unit
+// HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, four
+// sources in flight, the grid covers the vector once, edges in a CTA of their own, dependent launch.  The unit
 // is 8 fp32 or 16 bf16 elements, whatever the output type, so that the source side (n streams to one) stays on 256-bit
 // loads.  fp32 -> bf16, 8 sources of 6.5 M: 38.9 us (5.7 TB/s, a strided loop with 16-byte loads of one source at a
-// time) -> 33.7 us (6.6 TB/s).
+// time) -> 33.0 us (6.8 TB/s).
 #include "../api/flextree.h"
 #include "pdl.cuh"
 #include "reduce_nway.cuh"
 #include "vec.cuh"
 
 namespace ftk {
+
+constexpr int kThreads = 128;
 
 template <bool WIDE>
 __device__ __forceinline__ void load32(const unsigned char* p, uint4& a, uint4& b) {
@@ -49,7 +51,7 @@ __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, f
 // WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
 // 32); not WIDE: 128-bit ones.
 template <bool IN_BF16, bool OUT_BF16, bool WIDE, int GROUP>
-__global__ void __launch_bounds__(256) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, float scale) {
+__global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, float scale) {
   constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
   pdl_begin();
   const int edge_ctas = a.edge != 0;
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(256) reduce_nway_scaled_kernel(const __grid_co
       scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), scale);
     return;
   }
-  const unsigned long long i = (unsigned long long)(blockIdx.x - edge_ctas) * 256 + threadIdx.x;
+  const unsigned long long i = (unsigned long long)(blockIdx.x - edge_ctas) * kThreads + threadIdx.x;
   if (i >= a.nvec) return;
   float acc[E];
 #pragma unroll
@@ -128,13 +130,14 @@ static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int
   a.edge = (uint16_t)(len - a.nbody);
   for (int k = 0; k < a.n; ++k) a.src[k] = (const unsigned char*)a.src[k] + a.head * is;
   a.dst = (unsigned char*)a.dst + a.head * os;
-  const unsigned long long grid = (a.nvec + 255) / 256 + (a.edge != 0);
+  const unsigned long long grid = (a.nvec + kThreads - 1) / kThreads + (a.edge != 0);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-  // groups of four where there are no more sources: fewer registers, more CTAs on an SM
-  if (a.n <= 4) return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 4>, (unsigned)grid, 256, 0, st, a, scale)
-                            : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 4>, (unsigned)grid, 256, 0, st, a, scale);
-  return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 8>, (unsigned)grid, 256, 0, st, a, scale)
-              : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 8>, (unsigned)grid, 256, 0, st, a, scale);
+  // eight sources in flight pay from nine sources up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us
+  // with four, 24.7 with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four)
+  if (a.n <= 8) return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 4>, (unsigned)grid, kThreads, 0, st, a, scale)
+                            : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 4>, (unsigned)grid, kThreads, 0, st, a, scale);
+  return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 8>, (unsigned)grid, kThreads, 0, st, a, scale)
+              : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 8>, (unsigned)grid, kThreads, 0, st, a, scale);
 }
 
 cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st) {

@@ -25,8 +25,8 @@ __device__ __forceinline__ uint4 join(uint4 lo, uint4 hi, uint32_t shift) {
   return make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits), __funnelshift_r(w3, w4, bits));
 }
 
-template <int POL, int UNROLL, int GROUP>
-__global__ void __launch_bounds__(256) reduce_nway_shift_kernel(const __grid_constant__ NwayArgs a) {
+template <int POL, int UNROLL, int GROUP, int THREADS>
+__global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   pdl_begin();
   const int edge_ctas = a.edge != 0;
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) reduce_nway_shift_kernel(const __grid_con
     reduce_edges<POL, ScalarOp>(a);
     return;
   }
-  const unsigned long long base = (unsigned long long)(blockIdx.x - edge_ctas) * 256 * UNROLL + threadIdx.x;
+  const unsigned long long base = (unsigned long long)(blockIdx.x - edge_ctas) * THREADS * UNROLL + threadIdx.x;
   const bool last_lane = (threadIdx.x & 31) == 31;
   typename P::Acc acc[UNROLL];
   for (int k0 = 0; k0 < a.n; k0 += GROUP) {
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) reduce_nway_shift_kernel(const __grid_con
         const uint4* p = (const uint4*)((const unsigned char*)a.src[k0 + g] - shift);
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-          const unsigned long long i = base + u * 256;
+          const unsigned long long i = base + u * THREADS;
           // vector nvec exists for a shifted source: the last result takes part of it
           lo[g][u] = i < a.nvec || (shift && i == a.nvec) ? ld_stream(p + i) : make_uint4(0, 0, 0, 0);
           ex[g][u] = shift && last_lane && i < a.nvec ? ld_stream(p + i + 1) : make_uint4(0, 0, 0, 0);
@@ -72,15 +72,22 @@ __global__ void __launch_bounds__(256) reduce_nway_shift_kernel(const __grid_con
   }
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u)
-    if (base + u * 256 < a.nvec) st_vec_cs((uint4*)a.dst + base + u * 256, P::fin(acc[u]));
+    if (base + u * THREADS < a.nvec) st_vec_cs((uint4*)a.dst + base + u * THREADS, P::fin(acc[u]));
 }
 
+template <int POL, int UNROLL, int GROUP, int THREADS>
+static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
+  const unsigned long long grid = (a.nvec + THREADS * UNROLL - 1) / (THREADS * UNROLL) + (a.edge != 0);
+  if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
+  return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, a);
+}
+// Long vectors want many small CTAs with few registers, two vectors of two sources at a time: with 256 threads and two
+// vectors of four sources 100 MB of fp32 x4 took 117 us, so they take 77 (6.5 TB/s).  Below 3 MB the chip is not full and
+// one vector of four sources at a time has the shorter chain: fp32 x8 of 2 MB 5.1 us against 6.0.  (18 shapes measured,
+// 64 KB to 100 MB, 2 to 16 sources.)
 template <int POL>
 static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
-  constexpr int U = 2;
-  const unsigned long long grid = (a.nvec + 256 * U - 1) / (256 * U) + (a.edge != 0);
-  if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-  return launch_pdl(reduce_nway_shift_kernel<POL, U, 4>, (unsigned)grid, 256, 0, st, a);
+  return a.nvec >= (3u << 20) / 16 ? launch_t<POL, 2, 2, 64>(a, st) : launch_t<POL, 1, 4, 128>(a, st);
 }
 
 cudaError_t launch_shift(int pol, const NwayArgs& a, cudaStream_t st) {

@@ -94,12 +94,12 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
   }
 }
 
-// The default: 256 threads, one 32-byte unit each, up to eight sources in flight, evict-first stores, the grid
-// covers the vector once.  What bounds it is HBM; from 2 to 16 sources of 4 to 80 MB fp32 / bf16 / fp16 it is within
-// 3 % of the best of 16 configurations swept (128-512 threads, groups of 4 or 8, cache hints, persistent grids).
-// Groups of eight instead of four sources matter where the chip is not full: fp16 x16 of 1 Mi 9.6 -> 6.2 us,
-// bf16 x8 of 4 Mi 16.4 -> 14.4 us; with the dependent launch (pdl.cuh) 5.7 and 12.9.
-// fp32 x8 of 20 M: 104.5 -> 102.0 us, 7.06 TB/s.
+// The default: 128 threads, one 32-byte unit each, four sources in flight (eight from nine sources up), evict-first
+// stores, the grid covers the vector once.  What bounds it is HBM, or L2 below about 100 MB.  Over 2, 4, 8 and 16
+// sources of 16 KB to 256 MB in fp32, bf16 and fp16 it is 0.8 % from the best of 12 configurations on average and 8 % at
+// most (128-512 threads, groups of 4 and 8, three places for the dependent launch); 256 threads lose up to 26 % where
+// the grid fills the chip only once or twice (fp32 x8 of 1 M elements), and behave alike above.
+// fp32 x8 of 1 M: 4.0 us; of 10 M: 51.9 us (6.9 TB/s); of 64 Mi: 334 us (7.2 TB/s).
 //
 // Other configurations by code = U*1000 + LD*100 + ST*10 + T, with U units per thread per step, LD/ST as above,
 // T: 0 = 256 threads and one step per thread (the grid covers the vector), 1 = 512 threads likewise,
@@ -123,7 +123,7 @@ template <int POL, int NSRC, bool TUNING>
 static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t st) {
   const int t = code % 10;
   if (t != 0 && t != 1 && t != 3) return cudaErrorInvalidValue;
-  if (code == 0) return launch_t<POL, NSRC, 1, 0, 1, 256, 8>(a, 0, sms, st);
+  if (code == 0) return launch_t<POL, NSRC, 1, 0, 1, 128, NSRC == 0 ? 8 : 4>(a, 0, sms, st);
   if constexpr (TUNING) {
     switch (code / 10) {
       case 101: return launch_v<POL, NSRC, 1, 0, 1>(a, t, sms, st);
