@@ -356,7 +356,10 @@ static void layout_shift(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs
       const unsigned long long fits = whole ? whole - 1 : 0;
       if (fits < nvec) nvec = fits;
     }
-  if (!nvec) head = 0;
+  if (!nvec) {   // no body, and with it no vector behind the body for the kernel to look at
+    head = 0;
+    for (int k = 0; k < in.n; ++k) out->shift[k] = 0;
+  }
   out->nvec = nvec;
   out->nbody = nvec * 16 / unit;
   out->head = (uint16_t)(head / unit);

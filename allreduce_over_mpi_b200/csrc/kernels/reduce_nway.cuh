@@ -9,7 +9,7 @@
 namespace ftk {
 
 // One launch covers a whole vector: the body in 32- or 16-byte vectors, and the elements in front of and behind it
-// (the edges) one by one in a CTA of their own (block 0), so that neither a ragged length nor a slice that starts
+// (the edges) one by one in a CTA of their own (the last one), so that neither a ragged length nor a slice that starts
 // off a vector boundary costs a second launch or takes the rest of the vector off the vector loads.
 struct NwayArgs {
   const void* src[FT_MAX_FANIN];  // start of the body in every source

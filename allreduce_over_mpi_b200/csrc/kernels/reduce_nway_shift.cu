@@ -29,12 +29,7 @@ template <int POL, int UNROLL, int GROUP, int THREADS>
 __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   pdl_begin();
-  const int edge_ctas = a.edge != 0;
-  if (edge_ctas && blockIdx.x == 0) {
-    reduce_edges<POL, ScalarOp>(a);
-    return;
-  }
-  const unsigned long long base = (unsigned long long)(blockIdx.x - edge_ctas) * THREADS * UNROLL + threadIdx.x;
+  const unsigned long long base = (unsigned long long)blockIdx.x * THREADS * UNROLL + threadIdx.x;
   const bool last_lane = (threadIdx.x & 31) == 31;
   typename P::Acc acc[UNROLL];
   for (int k0 = 0; k0 < a.n; k0 += GROUP) {
@@ -73,6 +68,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u)
     if (base + u * THREADS < a.nvec) st_vec_cs((uint4*)a.dst + base + u * THREADS, P::fin(acc[u]));
+  if (a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
 }
 
 template <int POL, int UNROLL, int GROUP, int THREADS>

@@ -9,6 +9,8 @@
 //
 // Same job as the reference's reduce_sum_2 .. reduce_sum_8 kernels
 // (vector_add/reduce_sum_gpu.h:13-69), which move 4 bytes per thread.
+#include <type_traits>
+
 #include "pdl.cuh"
 #include "reduce_nway.cuh"
 #include "vec.cuh"
@@ -42,24 +44,62 @@ __device__ __forceinline__ void st32(void* p, const uint4& a, const uint4& b) {
                  ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
 }
 
-// One thread handles UNROLL 32-byte units per step, THREADS apart (every warp access is one
+// The default: one 32-byte unit per thread, 128 threads, the grid covers the vector once, evict-first stores.  NSRC > 0:
+// the fan-in is known at compile time; NSRC == 0: it is a.n (any value up to FT_MAX_FANIN).  Sources are taken GROUP at
+// a time (four, or eight from nine sources up): all loads of a group are issued before its first add.  How a thread
+// behind the end is kept from loading decides how many the compiler leaves in flight: a predicate on each load keeps a
+// group and more (72 registers, bf16 x8 of 4 M 11.7 us), leaving early 50 registers and 12.2 us, loading zeros instead
+// 40 registers and 14.1 us.  The edges, the job of the last CTA, come behind for the same reason: a branch in front of
+// the loads cost 3 to 5 %.
+//
+// What bounds it is HBM, or L2 below about 100 MB.  Over 2, 4, 8 and 16 sources of 16 KB to 256 MB in fp32, bf16 and fp16
+// it is 0.8 % from the best of 12 configurations on average and 8 % at most (128-512 threads, groups of 4 and 8, three
+// places for the dependent launch); 256 threads lose up to 26 % where the grid fills the chip only once or twice.
+// fp32 x8 of 1 M: 4.0 us; of 10 M: 51.9 us (6.9 TB/s); of 64 Mi: 334 us (7.2 TB/s).
+template <int POL, int NSRC, int THREADS, int GROUP>
+__global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
+  using P = typename PolById<POL>::type;
+  pdl_begin();
+  const unsigned long long i = (unsigned long long)blockIdx.x * THREADS + threadIdx.x;
+  const bool ok = i < a.nvec;
+  constexpr int G = (NSRC > 0 && NSRC < GROUP) ? NSRC : GROUP;
+  typename P::Acc al, ah;
+#pragma unroll
+  for (int g0 = 0; g0 < (NSRC > 0 ? NSRC : FT_MAX_FANIN); g0 += G) {
+    if (NSRC == 0 && g0 >= a.n) break;
+    uint4 lo[G], hi[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      if (ok && g0 + g < (NSRC > 0 ? NSRC : a.n)) ld32<0>((const unsigned char*)a.src[g0 + g] + i * 32, lo[g], hi[g]);
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      if (g0 + g < (NSRC > 0 ? NSRC : a.n)) {
+        if (g0 + g == 0) { P::init(al, lo[g]); P::init(ah, hi[g]); }
+        else { P::add(al, lo[g]); P::add(ah, hi[g]); }
+      }
+  }
+  if (ok) st32<1>((unsigned char*)a.dst + i * 32, P::fin(al), P::fin(ah));
+  if (!ok && a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
+}
+
+// The configurations that are asked for by number: one thread handles UNROLL 32-byte units per step, THREADS apart (every warp access is one
 // contiguous 1 KiB run).  The grid either covers the vector once (one step per thread) or is
 // capped and strides over it.  NSRC > 0: the fan-in is known at compile time; NSRC == 0: it is
 // a.n (any value up to FT_MAX_FANIN).  Sources are taken GROUP at a time: all loads of a group are
 // issued before its first add.
 template <int POL, int NSRC, int UNROLL, int LD, int ST, int THREADS, int GROUP>
-__global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
+__global__ void __launch_bounds__(THREADS) reduce_nway_strided_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   pdl_begin();
   const int edge_ctas = a.edge != 0;
-  if (edge_ctas && blockIdx.x == 0) {
+  if (edge_ctas && blockIdx.x == gridDim.x - 1) {
     reduce_edges<POL, ScalarOp>(a);
     return;
   }
   const unsigned long long n32 = a.nvec;
   const int nsrc = NSRC > 0 ? NSRC : a.n;
   const unsigned long long stride = (unsigned long long)(gridDim.x - edge_ctas) * THREADS * UNROLL;
-  for (unsigned long long base = (unsigned long long)(blockIdx.x - edge_ctas) * THREADS * UNROLL; base < n32; base += stride) {
+  for (unsigned long long base = (unsigned long long)blockIdx.x * THREADS * UNROLL; base < n32; base += stride) {
     unsigned long long idx[UNROLL];
     bool ok[UNROLL];
 #pragma unroll
@@ -94,14 +134,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
   }
 }
 
-// The default: 128 threads, one 32-byte unit each, four sources in flight (eight from nine sources up), evict-first
-// stores, the grid covers the vector once.  What bounds it is HBM, or L2 below about 100 MB.  Over 2, 4, 8 and 16
-// sources of 16 KB to 256 MB in fp32, bf16 and fp16 it is 0.8 % from the best of 12 configurations on average and 8 % at
-// most (128-512 threads, groups of 4 and 8, three places for the dependent launch); 256 threads lose up to 26 % where
-// the grid fills the chip only once or twice (fp32 x8 of 1 M elements), and behave alike above.
-// fp32 x8 of 1 M: 4.0 us; of 10 M: 51.9 us (6.9 TB/s); of 64 Mi: 334 us (7.2 TB/s).
-//
-// Other configurations by code = U*1000 + LD*100 + ST*10 + T, with U units per thread per step, LD/ST as above,
+// Configurations by code = U*1000 + LD*100 + ST*10 + T, with U units per thread per step, LD/ST as above,
 // T: 0 = 256 threads and one step per thread (the grid covers the vector), 1 = 512 threads likewise,
 //    3 = 512 threads x 4 CTAs per SM striding over the vector; groups of four sources.
 template <int POL, int NSRC, int UNROLL, int LD, int ST, int THREADS, int GROUP>
@@ -111,7 +144,7 @@ static cudaError_t launch_t(const NwayArgs& a, int ctas_per_sm, int sms, cudaStr
   if (ctas_per_sm && grid > (unsigned long long)sms * ctas_per_sm) grid = (unsigned long long)sms * ctas_per_sm;
   grid += a.edge != 0;
   if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-  return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, UNROLL, LD, ST, THREADS, GROUP>, (unsigned)grid, THREADS, 0, st, a);
+  return launch_pdl(reduce_nway_strided_kernel<POL, NSRC, UNROLL, LD, ST, THREADS, GROUP>, (unsigned)grid, THREADS, 0, st, a);
 }
 template <int POL, int NSRC, int UNROLL, int LD, int ST>
 static cudaError_t launch_v(const NwayArgs& a, int t, int sms, cudaStream_t st) {
@@ -123,7 +156,11 @@ template <int POL, int NSRC, bool TUNING>
 static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t st) {
   const int t = code % 10;
   if (t != 0 && t != 1 && t != 3) return cudaErrorInvalidValue;
-  if (code == 0) return launch_t<POL, NSRC, 1, 0, 1, 128, NSRC == 0 ? 8 : 4>(a, 0, sms, st);
+  if (code == 0) {
+    const unsigned long long grid = (a.nvec + 127) / 128 + (a.edge != 0);
+    if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
+    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, 128, NSRC == 0 ? 8 : 4>, (unsigned)grid, 128, 0, st, a);
+  }
   if constexpr (TUNING) {
     switch (code / 10) {
       case 101: return launch_v<POL, NSRC, 1, 0, 1>(a, t, sms, st);
