@@ -169,7 +169,13 @@ PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const void *in[FT_MAX_FANIN], *res[FT_MAX_FANIN];
   const at::Tensor *t0 = nullptr, *o0 = nullptr;
   if (n > FT_MAX_FANIN || nw > FT_MAX_FANIN) return other();
-  if (gather_inputs(args[1], in, &t0) != n || gather_inputs(args[2], res, &o0) != n) return other();
+  if (gather_inputs(args[1], in, &t0) != n) return other();
+  if (args[2] == args[1]) {
+    std::memcpy(res, in, sizeof(void*) * n);
+    o0 = t0;
+  } else if (gather_inputs(args[2], res, &o0) != n) {
+    return other();
+  }
   if (o0->scalar_type() != t0->scalar_type() || o0->numel() != t0->numel() || o0->device() != t0->device()) return other();
   for (Py_ssize_t k = 0; k < n; ++k) handles[k] = PyLong_AsVoidPtr(PyList_GET_ITEM(args[0], k));
   for (Py_ssize_t k = 0; k < nw; ++k) widths[k] = (int)PyLong_AsLong(PyTuple_GET_ITEM(args[4], k));

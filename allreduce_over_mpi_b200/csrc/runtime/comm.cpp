@@ -127,6 +127,7 @@ struct DevPlanEntry {
 struct WorldProgramEntry {
   int algo, phase, lonely, ring;
   std::vector<int> widths;
+  uint32_t nslots;   // receive slots of the plan's tagged-word form, whose limit holds here too
   ft::WorldProgram program;
 };
 
@@ -470,12 +471,12 @@ int launch_ll_call(ft_comm* c, const Prepared& pr, const void* sendbuf, void* re
   return FT_OK;
 }
 
-const ft::WorldProgram* world_program(ft_comm* c, int algo, int phase, const int* widths, int nw, int lonely, int ring) {
+const WorldProgramEntry* world_program(ft_comm* c, int algo, int phase, const int* widths, int nw, int lonely, int ring) {
   for (const WorldProgramEntry& w : c->world_programs)
     if (w.algo == algo && w.phase == phase && w.lonely == lonely && w.ring == ring && (int)w.widths.size() == nw &&
         std::equal(w.widths.begin(), w.widths.end(), widths))
-      return &w.program;
-  WorldProgramEntry w{algo, phase, lonely, ring, std::vector<int>(widths, widths + nw), {}};
+      return &w;
+  WorldProgramEntry w{algo, phase, lonely, ring, std::vector<int>(widths, widths + nw), 0, {}};
   ft::WorldProgramBuilder builder(c->world);
   if (algo == FT_ALGO_PUSH) {
     for (int b = 0; b < c->world; ++b) builder.flat(b, b, &w.program);
@@ -483,10 +484,13 @@ const ft::WorldProgram* world_program(ft_comm* c, int algo, int phase, const int
     builder.flat(0, 0, &w.program);
   } else {
     const ft::Plan p = ft::build_plan(c->world, make_shape(c->world, widths, nw, lonely, ring));
-    if (p.ok()) w.program = builder.run(p, (ft::WorldPhase)phase);
+    if (p.ok()) {
+      w.program = builder.run(p, (ft::WorldPhase)phase);
+      w.nslots = ft::build_dev_plan(p, c->rank).plan.nslots;
+    }
   }
   c->world_programs.push_back(std::move(w));
-  return &c->world_programs.back().program;
+  return &c->world_programs.back();
 }
 
 template <int RANKS>
@@ -1218,13 +1222,9 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
     default: return FT_ERR_NOT_AVAILABLE;
   }
   if (phase != 0 && algo != FT_ALGO_STAGED) return FT_ERR_NOT_AVAILABLE;
-  if (algo == FT_ALGO_LL && nw > 0) {   // the tagged-word form of a plan has its own limit on receive slots
-    DevPlanEntry* pe = nullptr;
-    if (get_plan(c, make_shape(n, widths, nw, lonely, ring), &pe) != FT_OK) { c->err.clear(); return FT_ERR_NOT_AVAILABLE; }
-    Prepared pr{pol, es, bytes, resident != 0};
-    if (!ll_tree_fits(c, pr, count, pe->nslots)) return FT_ERR_NOT_AVAILABLE;
-  }
-  const ft::WorldProgram* wp = world_program(c, algo, phase, widths, nw, lonely, ring);
+  const WorldProgramEntry* we = world_program(c, algo, phase, widths, nw, lonely, ring);
+  const ft::WorldProgram* wp = &we->program;
+  if (algo == FT_ALGO_LL && nw > 0 && !ll_tree_fits(c, Prepared{pol, es, bytes, resident != 0}, count, we->nslots)) return FT_ERR_NOT_AVAILABLE;
   const int cap = n <= 8 ? 8 : ftk::kWorldRanks;
   if (!wp->ok || wp->depth > (n <= 8 ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap) return FT_ERR_NOT_AVAILABLE;
   if (wp->entries.empty()) return FT_OK;

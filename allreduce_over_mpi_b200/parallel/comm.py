@@ -651,13 +651,14 @@ class LocalWorld:
         if code:
             raise FlexTreeError(code, lib().ft_comm_last_error(self.ranks[0]._h).decode())
         self._emu_call = 0
+        self._flat = Shape.flat(world)
         self._handles = [c._h.value for c in self.ranks]
         for c in self.ranks:
             c._world_handles = self._handles
 
     def _run_fused(self, tensors, outs, op, shape: Shape | None, algo: int, phase: int, scale: float) -> bool:
         """The whole call in one launch (ft_local_world_run); False: not a call it takes."""
-        widths, lonely, ring = (shape.widths, shape.lonely, int(shape.ring)) if shape is not None else ((), 0, 0)
+        widths, lonely, ring = (shape.widths, shape.lonely, shape.ring) if shape is not None else ((), 0, 0)
         code = (_lib._native or _lib.native()).local_world_run(self._handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)
         if code is None:
             return True
@@ -669,17 +670,18 @@ class LocalWorld:
                    scale: float = 1.0, outs: Sequence[torch.Tensor] | None = None):
         """Rank r reduces ``tensors[r]`` (in place unless ``outs`` is given)."""
         world = self.world
-        shp = _as_shape(shape, world) or Shape.flat(world)
+        shp = _as_shape(shape, world) or self._flat
         if op == "avg":
             op, scale = "sum", scale / world
+        if self.emulated and self.fused and self._run_fused(tensors, tensors if outs is None else outs, op,
+                                                            shp if shape is not None or algo == "staged" else None, ALGOS.get(algo, -1), 0, scale):
+            return list(tensors if outs is None else outs)
         outs = list(outs) if outs is not None else list(tensors)
         if not self.emulated:
             for r, c in enumerate(self.ranks):
                 with torch.cuda.device(c.device):
                     c.all_reduce(tensors[r], op=op, shape=shp if algo == "staged" or (algo == "ll" and shape is not None) else None,
                                  algo=algo, scale=scale, out=outs[r])
-            return outs
-        if self.fused and self._run_fused(tensors, outs, op, shp if shape is not None or algo == "staged" else None, ALGOS.get(algo, -1), 0, scale):
             return outs
         L = lib()
         dt = ft_dtype(tensors[0].dtype)
@@ -743,7 +745,7 @@ class LocalWorld:
 
     def _phase(self, tensors: Sequence[torch.Tensor], gather: bool, op: str, shape, scale: float):
         world = self.world
-        shp = _as_shape(shape, world) or Shape.flat(world)
+        shp = _as_shape(shape, world) or self._flat
         if op == "avg":
             op, scale = "sum", scale / world
         if not self.emulated or world == 1:
