@@ -336,6 +336,25 @@ static bool layout_wide(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs*
   out->dst = (unsigned char*)in.dst + head;
   return true;
 }
+// Cut it for the realigning kernel: the sources agree modulo 32, the result lies elsewhere.  The body is what the
+// result's whole 32-byte units between the first and the last whole unit of the sources hold.
+static bool layout_realign(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
+  const uintptr_t phase = (uintptr_t)in.src[0] & 31;
+  for (int k = 1; k < in.n; ++k)
+    if (((uintptr_t)in.src[k] & 31) != phase) return false;
+  const size_t first = (32 - phase) & 31;   // bytes in front of the sources' first whole unit
+  const size_t shift = (32 - (((uintptr_t)in.dst + first) & 31)) & 31, head = first + shift;
+  if (shift == 0 || bytes < first + 64) return false;
+  *out = in;
+  out->nvec = (bytes - first) / 32 - 1;
+  out->nbody = out->nvec * 32 / unit;
+  out->head = (uint16_t)(head / unit);
+  out->edge = (uint16_t)((bytes - out->nvec * 32) / unit);
+  out->shift[0] = (uint8_t)shift;
+  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
+  out->dst = (unsigned char*)in.dst + head;
+  return true;
+}
 // Cut it on the result's 16-byte boundaries for the shifted kernel.  A source that lies s bytes behind such a
 // boundary is read from s bytes before the body to 16 - s bytes behind it; the body is kept small enough for these
 // to be the vector's own bytes.  A vector too short for that is all edges.
@@ -378,8 +397,9 @@ static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
     if (layout_wide(a, bytes, unit, &b)) e = launch_wide(POL, b, variant, dev_info().sms, st);
     if (e == cudaErrorInvalidValue) {   // other phases, or no such configuration
       cudaGetLastError();
-      layout_shift(a, bytes, unit, &b);
-      e = launch_shift(POL, b, st);
+      const bool realign = layout_realign(a, bytes, unit, &b);
+      if (!realign) layout_shift(a, bytes, unit, &b);
+      e = launch_shift(POL, b, realign, st);
     }
     if (e != cudaSuccess) return cuda_fail(e, "reduce_nway launch");
     g_launches++;

@@ -18,14 +18,14 @@ struct NwayArgs {
   unsigned long long nbody;   // ... and in scalar units (see ScalarOp)
   int n;
   uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
-  uint8_t shift[FT_MAX_FANIN];  // shifted kernel: bytes by which source k's body lies behind a 16-byte boundary
+  uint8_t shift[FT_MAX_FANIN];  // shifted kernels: bytes by which source k's body lies behind a 16-byte (realign: 32-byte) boundary
 };
 
 // Kernels for pointers that agree modulo 32 (reduce_nway_wide.cu).  `code` selects a configuration (0: by size;
 // see launch_cfg there); returns cudaErrorInvalidValue when (policy, fan-in, code) has no instantiation.
 cudaError_t launch_wide(int pol, const NwayArgs& a, int code, int sms, cudaStream_t st);
-// Kernel for pointers that do not agree modulo 32 (reduce_nway_shift.cu).
-cudaError_t launch_shift(int pol, const NwayArgs& a, cudaStream_t st);
+// Kernels for pointers that do not agree modulo 32 (reduce_nway_shift.cu); `realign`: the sources do, the result does not.
+cudaError_t launch_shift(int pol, const NwayArgs& a, bool realign, cudaStream_t st);
 // out = scale * sum over `len` elements of whole vectors in `a` (reduce_nway_scaled.cu).
 cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st);
 

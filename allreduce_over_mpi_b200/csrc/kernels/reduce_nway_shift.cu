@@ -6,6 +6,12 @@
 // its own load and its right neighbour's (a warp shuffle; lane 31 loads the one vector more).  Memory bounds the
 // kernel: every byte is still read once, where the one-element loads this replaces moved 4 bytes an instruction.
 // The host keeps all loads inside the vectors (layout_shift in reduce_nway.cu).
+//
+// Where all sources lie at one phase and only the result at another (views summed into a new tensor), the second
+// kernel keeps 256-bit loads on the sources' boundaries and moves the RESULT across: one shuffle step per 32 bytes of
+// result instead of one per source.
+#include <type_traits>
+
 #include "pdl.cuh"
 #include "reduce_nway.cuh"
 #include "vec.cuh"
@@ -71,6 +77,69 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid
   if (a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
 }
 
+// 32 bytes from byte `shift` of the 64 in lo, hi.  `shift` is the same for the whole grid.
+__device__ __forceinline__ void join32(const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t shift, uint32_t (&out)[8]) {
+  const uint32_t bits = (shift & 3) * 8;
+  auto from = [&](auto words) {
+    constexpr int W = decltype(words)::value;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t a = W + k < 8 ? lo[(W + k) & 7] : hi[(W + k) & 7], b = W + k + 1 < 8 ? lo[(W + k + 1) & 7] : hi[(W + k + 1) & 7];
+      out[k] = __funnelshift_r(a, b, bits);
+    }
+  };
+  switch (shift >> 2) {
+    case 0: from(std::integral_constant<int, 0>{}); break;
+    case 1: from(std::integral_constant<int, 1>{}); break;
+    case 2: from(std::integral_constant<int, 2>{}); break;
+    case 3: from(std::integral_constant<int, 3>{}); break;
+    case 4: from(std::integral_constant<int, 4>{}); break;
+    case 5: from(std::integral_constant<int, 5>{}); break;
+    case 6: from(std::integral_constant<int, 6>{}); break;
+    default: from(std::integral_constant<int, 7>{}); break;
+  }
+}
+
+// A warp sums 32 units of 32 bytes on the sources' boundaries and stores the 31 units of the result between them; the
+// next warp sums the last one again (a hit in L2).  a.nvec: units of the result; shift[0]: bytes by which it lies behind
+// the sources' boundaries.  bf16 x8 of 4 M, sources one element off: 14.3 us by the kernel above, 12.0 here.
+template <int POL, int GROUP>
+__global__ void __launch_bounds__(128) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
+  using P = typename PolById<POL>::type;
+  pdl_begin();
+  const uint32_t lane = threadIdx.x & 31, shift = a.shift[0];
+  const unsigned long long i = ((unsigned long long)blockIdx.x * 4 + threadIdx.x / 32) * 31 + lane;
+  const bool ok = i <= a.nvec;   // one unit more than the result has
+  typename P::Acc al, ah;
+  for (int k0 = 0; k0 < a.n; k0 += GROUP) {
+    uint4 lo[GROUP], hi[GROUP];
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g)
+      if (ok && k0 + g < a.n) {
+        const unsigned char* p = (const unsigned char*)a.src[k0 + g] - shift + i * 32;
+        asm volatile("ld.global.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(lo[g].x), "=r"(lo[g].y), "=r"(lo[g].z), "=r"(lo[g].w), "=r"(hi[g].x), "=r"(hi[g].y), "=r"(hi[g].z), "=r"(hi[g].w)
+                     : "l"(p) : "memory");
+      }
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g)
+      if (k0 + g < a.n) {
+        if (k0 + g == 0) { P::init(al, lo[g]); P::init(ah, hi[g]); }
+        else { P::add(al, lo[g]); P::add(ah, hi[g]); }
+      }
+  }
+  const uint4 l = P::fin(al), h = P::fin(ah);
+  const uint32_t mine[8] = {l.x, l.y, l.z, l.w, h.x, h.y, h.z, h.w};
+  uint32_t next[8], w[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) next[k] = __shfl_down_sync(~0u, mine[k], 1);
+  join32(mine, next, shift, w);
+  if (lane < 31 && i < a.nvec)
+    asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"((unsigned char*)a.dst + i * 32), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+  if (a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
+}
+
 template <int POL, int UNROLL, int GROUP, int THREADS>
 static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
   const unsigned long long grid = (a.nvec + THREADS * UNROLL - 1) / (THREADS * UNROLL) + (a.edge != 0);
@@ -82,22 +151,28 @@ static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
 // one vector of four sources at a time has the shorter chain: fp32 x8 of 2 MB 5.1 us against 6.0.  (18 shapes measured,
 // 64 KB to 100 MB, 2 to 16 sources.)
 template <int POL>
-static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
+static cudaError_t launch_t(const NwayArgs& a, bool realign, cudaStream_t st) {
+  if (realign) {
+    const unsigned long long grid = (a.nvec + 4 * 31 - 1) / (4 * 31) + (a.edge != 0);
+    if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
+    return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, 128, 0, st, a)
+                    : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, 128, 0, st, a);
+  }
   return a.nvec >= (3u << 20) / 16 ? launch_t<POL, 2, 2, 64>(a, st) : launch_t<POL, 1, 4, 128>(a, st);
 }
 
-cudaError_t launch_shift(int pol, const NwayArgs& a, cudaStream_t st) {
+cudaError_t launch_shift(int pol, const NwayArgs& a, bool realign, cudaStream_t st) {
   switch (pol) {
-    case POL_ADD8: return launch_t<POL_ADD8>(a, st);
-    case POL_ADD16: return launch_t<POL_ADD16>(a, st);
-    case POL_ADD32: return launch_t<POL_ADD32>(a, st);
-    case POL_ADD64: return launch_t<POL_ADD64>(a, st);
-    case POL_OR: return launch_t<POL_OR>(a, st);
-    case POL_AND: return launch_t<POL_AND>(a, st);
-    case POL_F32: return launch_t<POL_F32>(a, st);
-    case POL_F64: return launch_t<POL_F64>(a, st);
-    case POL_BF16: return launch_t<POL_BF16>(a, st);
-    case POL_F16: return launch_t<POL_F16>(a, st);
+    case POL_ADD8: return launch_t<POL_ADD8>(a, realign, st);
+    case POL_ADD16: return launch_t<POL_ADD16>(a, realign, st);
+    case POL_ADD32: return launch_t<POL_ADD32>(a, realign, st);
+    case POL_ADD64: return launch_t<POL_ADD64>(a, realign, st);
+    case POL_OR: return launch_t<POL_OR>(a, realign, st);
+    case POL_AND: return launch_t<POL_AND>(a, realign, st);
+    case POL_F32: return launch_t<POL_F32>(a, realign, st);
+    case POL_F64: return launch_t<POL_F64>(a, realign, st);
+    case POL_BF16: return launch_t<POL_BF16>(a, realign, st);
+    case POL_F16: return launch_t<POL_F16>(a, realign, st);
     default: return cudaErrorInvalidValue;
   }
 }
