@@ -117,7 +117,9 @@ static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int
   constexpr unsigned long long E = IN_BF16 ? 16 : 8;
   constexpr size_t is = IN_BF16 ? 2 : 4, os = OUT_BF16 ? 2 : 4;
   bool wide = true;
-  int head = common_head(a, is, os, 32, IN_BF16 || !OUT_BF16 ? 32 : 16);
+  constexpr size_t da = IN_BF16 || !OUT_BF16 ? 32 : 16;
+  int head = len >= 4096 / is ? common_head(a, is, os, 128, da) : -1;   // whole lines: see layout_wide in reduce_nway.cu
+  if (head < 0) head = common_head(a, is, os, 32, da);
   if (head < 0) { wide = false; head = common_head(a, is, os, 16, 16); }
   if (head < 0) {
     const unsigned long long want = (len + 255) / 256, cap = (unsigned long long)sms * 8;
