@@ -50,7 +50,7 @@ __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, f
 
 // WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
 // 32); not WIDE: 128-bit ones.
-template <bool IN_BF16, bool OUT_BF16, bool WIDE, int GROUP>
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP>
 __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, float scale) {
   constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
   pdl_begin();
@@ -64,14 +64,15 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   float acc[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) acc[j] = 0.f;
-  for (int k0 = 0; k0 < a.n; k0 += GROUP) {
+  const int n = NSRC > 0 ? NSRC : a.n;
+  for (int k0 = 0; k0 < n; k0 += GROUP) {
     uint4 lo[GROUP], hi[GROUP];
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
-      if (k0 + g < a.n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
+      if (k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
-      if (k0 + g < a.n) {
+      if (k0 + g < n) {
         const uint32_t w[8] = {lo[g].x, lo[g].y, lo[g].z, lo[g].w, hi[g].x, hi[g].y, hi[g].z, hi[g].w};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -112,6 +113,21 @@ static int common_head(const NwayArgs& a, size_t is, size_t os, size_t sa, size_
   return -1;
 }
 
+// Two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up the loop is as good or
+// better (with the fan-in known the compiler keeps fewer loads in flight: bf16 x8 of 4 M 14.3 us, not 12.0).  Eight
+// sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with four, 24.7
+// with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four).
+template <bool IN_BF16, bool OUT_BF16, bool WIDE>
+static cudaError_t launch_n(const NwayArgs& a, unsigned grid, float scale, cudaStream_t st) {
+  switch (a.n) {
+    case 2: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 2, 2>, grid, kThreads, 0, st, a, scale);
+    case 3: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 3, 3>, grid, kThreads, 0, st, a, scale);
+    default: break;
+  }
+  return a.n <= 8 ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 4>, grid, kThreads, 0, st, a, scale)
+                  : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 8>, grid, kThreads, 0, st, a, scale);
+}
+
 template <bool IN_BF16, bool OUT_BF16>
 static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int sms, cudaStream_t st) {
   constexpr unsigned long long E = IN_BF16 ? 16 : 8;
@@ -133,12 +149,7 @@ static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int
   a.dst = (unsigned char*)a.dst + a.head * os;
   const unsigned long long grid = (a.nvec + kThreads - 1) / kThreads + (a.edge != 0);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-  // eight sources in flight pay from nine sources up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us
-  // with four, 24.7 with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four)
-  if (a.n <= 8) return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 4>, (unsigned)grid, kThreads, 0, st, a, scale)
-                            : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 4>, (unsigned)grid, kThreads, 0, st, a, scale);
-  return wide ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, true, 8>, (unsigned)grid, kThreads, 0, st, a, scale)
-              : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, false, 8>, (unsigned)grid, kThreads, 0, st, a, scale);
+  return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, scale, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, scale, st);
 }
 
 cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st) {
