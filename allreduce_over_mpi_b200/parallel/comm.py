@@ -652,6 +652,7 @@ class LocalWorld:
             raise FlexTreeError(code, lib().ft_comm_last_error(self.ranks[0]._h).decode())
         self._emu_call = 0
         self._flat = Shape.flat(world)
+        self._ranges: tuple = (None, 0, 0, ())
         self._handles = [c._h.value for c in self.ranks]
         for c in self.ranks:
             c._world_handles = self._handles
@@ -748,6 +749,8 @@ class LocalWorld:
         shp = _as_shape(shape, world) or self._flat
         if op == "avg":
             op, scale = "sum", scale / world
+        if self.emulated and self.fused and self._run_fused(tensors, tensors, op, shp, ALGOS["staged"], 2 if gather else 1, scale):
+            return shp
         if not self.emulated or world == 1:
             for r, c in enumerate(self.ranks):
                 with torch.cuda.device(c.device):
@@ -755,8 +758,6 @@ class LocalWorld:
                         c.all_gather(tensors[r], shape=shp)
                     else:
                         c.reduce_scatter(tensors[r], op=op, shape=shp, scale=scale)
-            return shp
-        if self.fused and self._run_fused(tensors, tensors, op, shp, ALGOS["staged"], 2 if gather else 1, scale):
             return shp
         nstages = planner.plan_num_stages(world, shp)
         if nstages < 0:
@@ -775,8 +776,11 @@ class LocalWorld:
     def reduce_scatter(self, tensors: Sequence[torch.Tensor], op: str = "sum", shape=None, scale: float = 1.0):
         """Reduce-scatter half alone; returns, per rank, the views of the blocks it holds complete."""
         shp = self._phase(tensors, False, op, shape, scale)
-        t0 = tensors[0]
-        views = (_lib._native or _lib.native()).narrow_all(tensors, _owned_ranges(self.world, shp, t0.numel(), t0.element_size()))
+        n, es = tensors[0].numel(), tensors[0].element_size()
+        last = self._ranges   # of the call before: a step asks for the same ones bucket after bucket
+        if last[0] is not shp or last[1] != n or last[2] != es:
+            last = self._ranges = (shp, n, es, _owned_ranges(self.world, shp, n, es))
+        views = (_lib._native or _lib.native()).narrow_all(tensors, last[3])
         if views is not NotImplemented:
             return views
         out = []
