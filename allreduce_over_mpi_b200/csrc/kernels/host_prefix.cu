@@ -7,8 +7,9 @@
 // 684 us here (33.6 MB in at 49 GB/s, 16.8 MB out at the same time; the copy engines alone, both ways at once without
 // a reduction: 720 us); 20 000 elements 59 -> 20 us, 1000 elements of two inputs 20 -> 4 us.
 //
-// A handful of CTAs fills the link (latency x rate is about 100 KB in flight; 8 to 592 CTAs measured, more only make
-// reads and writes collide: 681 us with 8 or 16, 771 us with 592), so the rest of the GPU stays free.
+// A handful of CTAs fills the link, so the rest of the GPU stays free: 1 MB of loads in flight.  Where the host memory is
+// near, 256 KB do (8 CTAs with eight inputs, 681 us), but from a farther socket they reach 41 GB/s only (809 us; 683 us
+// with 32 CTAs on either box).  Many more make reads and writes collide (592 CTAs 771 us).
 #include "pdl.cuh"
 #include "vec.cuh"
 #include "host_prefix.h"
@@ -54,8 +55,8 @@ __global__ void __launch_bounds__(256) host_prefix_kernel(const __grid_constant_
 template <int POL>
 static cudaError_t launch_t(const HostPrefixArgs& a, cudaStream_t st) {
   const uint64_t items = a.bytes / 16 + a.bytes % 16 / a.es;
-  // 256 KB of loads in flight: 8 CTAs of 256 threads with eight inputs, more with fewer
-  uint64_t grid = 64 / (a.n_in < 8 ? a.n_in : 8), want = (items + 255) / 256;
+  // 32 CTAs of 256 threads with eight inputs, more with fewer
+  uint64_t grid = 256 / (a.n_in < 8 ? a.n_in : 8), want = (items + 255) / 256;
   if (grid > want) grid = want;
   ft_count_launch(1);
   return launch_pdl(host_prefix_kernel<POL>, (unsigned)grid, 256, 0, st, a);
