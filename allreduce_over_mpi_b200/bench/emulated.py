@@ -39,6 +39,7 @@ def main(argv=None):
     in_heap = a.algo in ("staged", "push")
     heap = a.bytes + (1 << 20) if in_heap else 1 << 20
     w = LocalWorld(a.world, heap_bytes=heap, staging_bytes=max(a.bytes, 1 << 20) if not in_heap else 1 << 20)
+    w.fused = False   # the kernels that several devices would run, not the one-launch form
     g = torch.Generator(device="cuda").manual_seed(7)
     if in_heap:
         bufs = [c.alloc(count, dtype) for c in w.ranks]
