@@ -397,7 +397,7 @@ static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
   if (variant == 0 || variant >= 1000) {
     NwayArgs b;
     e = cudaErrorInvalidValue;
-    if (layout_wide(a, bytes, unit, &b)) e = launch_wide(POL, b, variant, dev_info().sms, st);
+    if (layout_wide(a, bytes, unit, &b)) e = launch_wide(POL, b, variant, variant ? dev_info().sms : 0, st);
     if (e == cudaErrorInvalidValue) {   // other phases, or no such configuration
       cudaGetLastError();
       const bool realign = layout_realign(a, bytes, unit, &b);

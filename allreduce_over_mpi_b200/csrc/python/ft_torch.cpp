@@ -17,6 +17,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -255,6 +256,9 @@ PyObject* narrow_all(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   PyObject* all = PyList_New(n);
   for (int k = 0; all && k < n; ++k) {
     const at::Tensor& t = THPVariable_Unpack(PyList_GET_ITEM(args[0], k));
+    // nothing to record for a tensor without a gradient: past the autograd layer, but not past the one that makes it a view
+    std::optional<at::AutoDispatchBelowAutograd> below;
+    if (!t.requires_grad() && !t._fw_grad(0).defined()) below.emplace();
     PyObject* ranges = PyTuple_GET_ITEM(args[1], k);
     PyObject* mine = PyList_New(PyTuple_GET_SIZE(ranges));
     PyList_SET_ITEM(all, k, mine);
