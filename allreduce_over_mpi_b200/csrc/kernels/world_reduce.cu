@@ -148,7 +148,9 @@ static cudaError_t launch_v(const WorldArgs<RANKS>& a, int entries, int depth, i
       if (depth == 0) return steps <= 4 ? launch_t<POL, V, 0, 4, RANKS>(a, entries, st) : launch_t<POL, V, 0, 8, RANKS>(a, entries, st);
       if (depth == 1) return steps <= 4 ? launch_t<POL, V, 1, 4, RANKS>(a, entries, st) : launch_t<POL, V, 1, 8, RANKS>(a, entries, st);
     }
-    return launch_t<POL, V, 2, 8, RANKS>(a, entries, st);
+    // two values put aside: 32 bytes of 16-bit floats are 16 accumulators each and spill (2*2*2 over eight bf16 buckets of
+    // 25 MB 74.8 us, 70.1 with 16 bytes a thread; fp32 65.1 us with 16 and 64.3 with 32)
+    return launch_t<POL, POL == POL_BF16 || POL == POL_F16 ? 1 : V, 2, 8, RANKS>(a, entries, st);
   }
 }
 template <int POL, int RANKS>
