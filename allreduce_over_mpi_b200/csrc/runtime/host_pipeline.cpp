@@ -70,7 +70,9 @@ unsigned char* pinned_address(const void* p, size_t bytes) {
   return (unsigned char*)(uintptr_t)dev;
 }
 
-// The call as one kernel; FT_ERR_NOT_AVAILABLE when some operand is not pinned or not on a 16-byte boundary.
+// The call as one kernel; FT_ERR_NOT_AVAILABLE when some operand is not pinned or not on a 16-byte boundary, or when a
+// result overlaps an input or another result: the chunked path reads all inputs of a chunk before it writes and writes
+// the results in the caller's order, and what it does there stays what happens.
 int run_direct(int op, int dtype, const void* const* src, const int* fanin, void* const* dst, int n_out, size_t bytes, size_t es,
                cudaStream_t st) {
   const int pol = ftk::policy_id(op, dtype);
@@ -79,6 +81,15 @@ int run_direct(int op, int dtype, const void* const* src, const int* fanin, void
   a.n_in = 0;
   for (int j = 0; j < n_out; ++j)
     if (fanin[j] > a.n_in) a.n_in = fanin[j];
+  const auto overlap = [&](const void* x, const void* y) {
+    return (uintptr_t)x < (uintptr_t)y + bytes && (uintptr_t)y < (uintptr_t)x + bytes;
+  };
+  for (int j = 0; j < n_out; ++j) {
+    for (int i = 0; i < j; ++i)
+      if (overlap(dst[i], dst[j])) return FT_ERR_NOT_AVAILABLE;
+    for (int k = 0; k < a.n_in; ++k)
+      if (overlap(src[k], dst[j])) return FT_ERR_NOT_AVAILABLE;
+  }
   for (int k = 0; k < a.n_in; ++k)
     if (((uintptr_t)src[k] & 15) || !(a.in[k] = pinned_address(src[k], bytes))) return FT_ERR_NOT_AVAILABLE;
   int filled = 0;

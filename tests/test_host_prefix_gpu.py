@@ -42,3 +42,16 @@ def test_in_place_and_own_stream():
     st.synchronize()
     assert torch.equal(hin[1], want)
     pipe.close()
+
+
+def test_results_over_later_inputs_and_over_one_another():
+    """Every input of a chunk is read before any result is written, and the last of two results in one place stays."""
+    host = [torch.randn(5003) for _ in range(12)]
+    hin = [h.pin_memory() for h in host]
+    want = [reduce_nway([h.to(DEV) for h in host[:f]]).cpu() for f in (5, 12, 3)]
+    pipe = HostReducePipeline(device=DEV, max_inputs=12, max_outputs=3)
+    both = torch.empty(5003).pin_memory()
+    pipe.run(hin, [5, 12, 3], [hin[10], both, both])
+    torch.cuda.synchronize()
+    assert torch.equal(hin[10], want[0]) and torch.equal(both, want[2])
+    pipe.close()
