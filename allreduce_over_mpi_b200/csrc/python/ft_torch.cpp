@@ -170,7 +170,7 @@ PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   int widths[FT_MAX_FANIN];
   const void *in[FT_MAX_FANIN], *res[FT_MAX_FANIN];
   const at::Tensor *t0 = nullptr, *o0 = nullptr;
-  if (n > FT_MAX_FANIN || nw > FT_MAX_FANIN) return other();
+  if (n < 1 || n > FT_MAX_FANIN || nw > FT_MAX_FANIN) return other();   // no handles: a closed world
   if (gather_inputs(args[1], in, &t0) != n) return other();
   if (args[2] == args[1]) {
     std::memcpy(res, in, sizeof(void*) * n);
