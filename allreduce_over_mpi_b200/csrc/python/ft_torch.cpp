@@ -11,6 +11,8 @@
 //   an int                                                       the library's status, the call failed;
 //   NotImplemented                                               anything out of the ordinary (CPU tensors, tensor
 //       subclasses, mixed types or sizes, ...): the caller's Python path checks it and reports it in words.
+// A C++ exception (a tensor without memory inside vmap, a dispatch mode that raises, ...) becomes the Python exception
+// it would be in torch: guarded() stands between every function and the interpreter.
 //
 // libflextree.so is not linked: its entry points arrive as addresses through bind(), so that the checked
 // build (FT_LIB=bounds) and the normal one share this module.
@@ -23,7 +25,9 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <cstring>
 #include <optional>
@@ -63,11 +67,16 @@ int op_of(PyObject* o) {
   return !std::strcmp(s, "sum") ? FT_SUM : !std::strcmp(s, "band") ? FT_BAND : -1;
 }
 
-// A plain, contiguous tensor on a CUDA device; null for anything else.
-const at::Tensor* plain_cuda(PyObject* o) {
+// A plain, contiguous tensor; null for anything else.
+const at::Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  return t.defined() && t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() ? &t : nullptr;
+  return t.defined() && t.layout() == at::kStrided && t.is_contiguous() ? &t : nullptr;
+}
+// ... on a CUDA device.
+const at::Tensor* plain_cuda(PyObject* o) {
+  const at::Tensor* t = plain(o);
+  return t && t->is_cuda() ? t : nullptr;
 }
 
 // n tensors that share type, size and device.  Returns n, or 0.
@@ -208,13 +217,11 @@ int gather_host(PyObject* seq, const void** ptr, const at::Tensor** first) {
   const Py_ssize_t n = list ? PyList_GET_SIZE(seq) : PyTuple_GET_SIZE(seq);
   if (n < 1 || n > FT_MAX_FANIN) return 0;
   for (Py_ssize_t k = 0; k < n; ++k) {
-    PyObject* o = list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k);
-    if (!THPVariable_CheckExact(o)) return 0;
-    const at::Tensor& t = THPVariable_Unpack(o);
-    if (!t.defined() || !t.is_cpu() || t.layout() != at::kStrided || !t.is_contiguous()) return 0;
-    if (!*first) *first = &t;
-    else if (t.scalar_type() != (*first)->scalar_type() || t.numel() != (*first)->numel()) return 0;
-    ptr[k] = t.const_data_ptr();
+    const at::Tensor* t = plain(list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k));
+    if (!t || !t->is_cpu()) return 0;
+    if (!*first) *first = t;
+    else if (t->scalar_type() != (*first)->scalar_type() || t->numel() != (*first)->numel()) return 0;
+    ptr[k] = t->const_data_ptr();
   }
   return (int)n;
 }
@@ -249,27 +256,38 @@ PyObject* host_pipe_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 // narrow_all(tensors, ranges): for each tensor the list of its flat [lo, hi) views; ranges[k] is a tuple of (lo, hi).
 PyObject* narrow_all(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  const void* ptr[FT_MAX_FANIN];
-  const at::Tensor* t0 = nullptr;
   if (nargs != 2 || !PyList_CheckExact(args[0]) || !PyTuple_CheckExact(args[1])) return other();
-  const int n = gather_inputs(args[0], ptr, &t0);
-  if (!n || PyTuple_GET_SIZE(args[1]) != n) return other();
-  PyObject* all = PyList_New(n);
-  for (int k = 0; all && k < n; ++k) {
-    const at::Tensor& t = THPVariable_Unpack(PyList_GET_ITEM(args[0], k));
+  const Py_ssize_t n = PyList_GET_SIZE(args[0]);
+  if (n < 1 || PyTuple_GET_SIZE(args[1]) != n) return other();
+  THPObjectPtr all(PyList_New(n));
+  if (!all) return nullptr;
+  int64_t numel = -1;   // one size for all, as the ranges are
+  for (Py_ssize_t k = 0; k < n; ++k) {
+    // looked up for each tensor: a dispatch mode runs Python code below, which may change the list
+    const at::Tensor* p = k < PyList_GET_SIZE(args[0]) ? plain(PyList_GET_ITEM(args[0], k)) : nullptr;
+    PyObject* ranges = PyTuple_GET_ITEM(args[1], k);
+    if (!p || !PyTuple_CheckExact(ranges)) return other();
+    const at::Tensor t = *p;
+    if (k == 0) numel = t.numel();
+    else if (t.numel() != numel) return other();
     // nothing to record for a tensor without a gradient: past the autograd layer, but not past the one that makes it a view
     std::optional<at::AutoDispatchBelowAutograd> below;
     if (!t.requires_grad() && !t._fw_grad(0).defined()) below.emplace();
-    PyObject* ranges = PyTuple_GET_ITEM(args[1], k);
     PyObject* mine = PyList_New(PyTuple_GET_SIZE(ranges));
-    PyList_SET_ITEM(all, k, mine);
+    if (!mine) return nullptr;
+    PyList_SET_ITEM(all.get(), k, mine);
     for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(ranges); ++j) {
-      const int64_t lo = PyLong_AsLongLong(PyTuple_GET_ITEM(PyTuple_GET_ITEM(ranges, j), 0));
-      const int64_t hi = PyLong_AsLongLong(PyTuple_GET_ITEM(PyTuple_GET_ITEM(ranges, j), 1));
-      PyList_SET_ITEM(mine, j, THPVariable_Wrap(t.as_strided({hi - lo}, {1}, t.storage_offset() + lo)));
+      PyObject* range = PyTuple_GET_ITEM(ranges, j);
+      if (!PyTuple_CheckExact(range) || PyTuple_GET_SIZE(range) != 2) return other();
+      const int64_t lo = PyLong_AsLongLong(PyTuple_GET_ITEM(range, 0)), hi = PyLong_AsLongLong(PyTuple_GET_ITEM(range, 1));
+      if (PyErr_Occurred()) return nullptr;
+      if (lo < 0 || hi < lo || hi > numel) return other();
+      PyObject* view = THPVariable_Wrap(t.as_strided({hi - lo}, {1}, t.storage_offset() + lo));
+      if (!view) return nullptr;
+      PyList_SET_ITEM(mine, j, view);
     }
   }
-  return all;
+  return all.release();
 }
 
 // bind({name: address}): entry points of the libflextree build this process uses.
@@ -287,14 +305,25 @@ PyObject* bind(PyObject*, PyObject* d) {
   Py_RETURN_NONE;
 }
 
+// No C++ exception may leave through the interpreter's C frames.
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  return F(self, args, nargs);
+  END_HANDLE_TH_ERRORS
+}
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+constexpr PyMethodDef method(const char* name, const char* doc) {
+  return {name, (PyCFunction)(void (*)(void))guarded<F>, METH_FASTCALL, doc};
+}
+
 PyMethodDef methods[] = {
     {"bind", bind, METH_O, "bind({name: address})"},
-    {"reduce_nway", (PyCFunction)(void (*)(void))reduce_nway, METH_FASTCALL, "reduce_nway(tensors, op, out, variant)"},
-    {"reduce_nway_scaled", (PyCFunction)(void (*)(void))reduce_nway_scaled, METH_FASTCALL, "reduce_nway_scaled(tensors, scale, out_dtype, out)"},
-    {"local_world_run", (PyCFunction)(void (*)(void))local_world_run, METH_FASTCALL,
-     "local_world_run(handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)"},
-    {"host_pipe_run", (PyCFunction)(void (*)(void))host_pipe_run, METH_FASTCALL, "host_pipe_run(pipeline, device, inputs, fanins, outs, op)"},
-    {"narrow_all", (PyCFunction)(void (*)(void))narrow_all, METH_FASTCALL, "narrow_all(tensors, ranges)"},
+    method<reduce_nway>("reduce_nway", "reduce_nway(tensors, op, out, variant)"),
+    method<reduce_nway_scaled>("reduce_nway_scaled", "reduce_nway_scaled(tensors, scale, out_dtype, out)"),
+    method<local_world_run>("local_world_run", "local_world_run(handles, tensors, outs, op, widths, lonely, ring, algo, phase, scale)"),
+    method<host_pipe_run>("host_pipe_run", "host_pipe_run(pipeline, device, inputs, fanins, outs, op)"),
+    method<narrow_all>("narrow_all", "narrow_all(tensors, ranges)"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ft_torch", "native call path of the Python entry points", -1, methods};
 

@@ -33,3 +33,38 @@ try:
 except IndexError:
     print("refused")
 """) == "refused"
+
+
+def test_an_exception_in_torch_becomes_a_python_exception():
+    """Inside vmap a tensor has no memory: asking for its address throws, in C++."""
+    assert child("""
+try:
+    torch.vmap(lambda x: (N.host_pipe_run(1, 0, [x], [1], [x], "sum"), x)[1])(torch.zeros(2, 3))
+except RuntimeError as e:
+    print("storage" in str(e))
+""") == "True"
+
+
+def test_narrow_all_reports_what_its_views_raise():
+    """A dispatch mode that raises in the second view of the first tensor; without it, the views themselves."""
+    assert child("""
+from torch.utils._python_dispatch import TorchDispatchMode
+class Refuse(TorchDispatchMode):
+    calls = 0
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.calls += 1
+        if self.calls == 2:
+            raise KeyError("no more views")
+        return func(*args, **(kwargs or {}))
+t = [torch.arange(6.), torch.arange(6.).requires_grad_()]
+ranges = (((0, 2), (2, 6)), ((5, 6),))
+try:
+    with Refuse():
+        N.narrow_all(t, ranges)
+except KeyError as e:
+    print("raised")
+v = N.narrow_all(t, ranges)
+assert [x.tolist() for x in v[0]] == [[0, 1], [2, 3, 4, 5]] and v[1][0].tolist() == [5]
+assert v[0][1]._base is t[0] and not v[0][0].requires_grad and v[1][0].requires_grad
+assert N.narrow_all(t, (((0, 7),), ())) is NotImplemented and N.narrow_all([t[0], t[1][:2]], ((), ())) is NotImplemented
+""") == "raised"
