@@ -79,15 +79,30 @@ const at::Tensor* plain_cuda(PyObject* o) {
   return t && t->is_cuda() ? t : nullptr;
 }
 
+// References to the tensors of a call.  The calls give up the GIL, and the caller's lists are only borrowed: a thread that
+// changes one in the meantime would otherwise free the tensors whose memory the call is about to use.  Destroyed with
+// the GIL held.
+struct Kept {
+  PyObject* o[2 * FT_MAX_FANIN];
+  int n = 0;
+  Kept() = default;
+  Kept(const Kept&) = delete;
+  Kept& operator=(const Kept&) = delete;
+  ~Kept() { while (n) Py_DECREF(o[--n]); }
+  void add(PyObject* p) { Py_INCREF(p); o[n++] = p; }
+};
+
 // n tensors that share type, size and device.  Returns n, or 0.
-int gather_inputs(PyObject* seq, const void** src, const at::Tensor** first) {
+int gather_inputs(PyObject* seq, const void** src, const at::Tensor** first, Kept* kept) {
   const bool list = PyList_CheckExact(seq);
   if (!list && !PyTuple_CheckExact(seq)) return 0;
   const Py_ssize_t n = list ? PyList_GET_SIZE(seq) : PyTuple_GET_SIZE(seq);
   if (n < 1 || n > FT_MAX_FANIN) return 0;
   for (Py_ssize_t k = 0; k < n; ++k) {
-    const at::Tensor* t = plain_cuda(list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k));
+    PyObject* o = list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k);
+    const at::Tensor* t = plain_cuda(o);
     if (!t) return 0;
+    kept->add(o);
     if (k == 0) *first = t;
     else if (t->scalar_type() != (*first)->scalar_type() || t->numel() != (*first)->numel() || t->device() != (*first)->device()) return 0;
     src[k] = t->const_data_ptr();
@@ -107,7 +122,8 @@ PyObject* reduce_nway(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (nargs != 4 || !p_reduce_nway) return other();
   const void* src[FT_MAX_FANIN];
   const at::Tensor* t0 = nullptr;
-  const int n = gather_inputs(args[0], src, &t0);
+  Kept kept;   // (args[] themselves are held by the caller's frame)
+  const int n = gather_inputs(args[0], src, &t0, &kept);
   const int op = op_of(args[1]);
   if (!n || op < 0 || !PyLong_CheckExact(args[3])) return other();
   const int dt = dtype_of(t0->scalar_type());
@@ -139,7 +155,8 @@ PyObject* reduce_nway_scaled(PyObject*, PyObject* const* args, Py_ssize_t nargs)
   if (nargs != 4 || !p_reduce_nway_scaled) return other();
   const void* src[FT_MAX_FANIN];
   const at::Tensor* t0 = nullptr;
-  const int n = gather_inputs(args[0], src, &t0);
+  Kept kept;   // (args[] themselves are held by the caller's frame)
+  const int n = gather_inputs(args[0], src, &t0, &kept);
   if (!n || !PyFloat_CheckExact(args[1])) return other();
   const float scale = (float)PyFloat_AS_DOUBLE(args[1]);
   const at::Tensor* dst = nullptr;
@@ -179,12 +196,13 @@ PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   int widths[FT_MAX_FANIN];
   const void *in[FT_MAX_FANIN], *res[FT_MAX_FANIN];
   const at::Tensor *t0 = nullptr, *o0 = nullptr;
+  Kept kept;
   if (n < 1 || n > FT_MAX_FANIN || nw > FT_MAX_FANIN) return other();   // no handles: a closed world
-  if (gather_inputs(args[1], in, &t0) != n) return other();
+  if (gather_inputs(args[1], in, &t0, &kept) != n) return other();
   if (args[2] == args[1]) {
     std::memcpy(res, in, sizeof(void*) * n);
     o0 = t0;
-  } else if (gather_inputs(args[2], res, &o0) != n) {
+  } else if (gather_inputs(args[2], res, &o0, &kept) != n) {
     return other();
   }
   if (o0->scalar_type() != t0->scalar_type() || o0->numel() != t0->numel() || o0->device() != t0->device()) return other();
@@ -211,14 +229,16 @@ PyObject* local_world_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 // Plain, contiguous CPU tensors that share type and size with *first (set by the first one).  Returns their number, or 0.
-int gather_host(PyObject* seq, const void** ptr, const at::Tensor** first) {
+int gather_host(PyObject* seq, const void** ptr, const at::Tensor** first, Kept* kept) {
   const bool list = PyList_CheckExact(seq);
   if (!list && !PyTuple_CheckExact(seq)) return 0;
   const Py_ssize_t n = list ? PyList_GET_SIZE(seq) : PyTuple_GET_SIZE(seq);
   if (n < 1 || n > FT_MAX_FANIN) return 0;
   for (Py_ssize_t k = 0; k < n; ++k) {
-    const at::Tensor* t = plain(list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k));
+    PyObject* o = list ? PyList_GET_ITEM(seq, k) : PyTuple_GET_ITEM(seq, k);
+    const at::Tensor* t = plain(o);
     if (!t || !t->is_cpu()) return 0;
+    kept->add(o);
     if (!*first) *first = t;
     else if (t->scalar_type() != (*first)->scalar_type() || t->numel() != (*first)->numel()) return 0;
     ptr[k] = t->const_data_ptr();
@@ -232,7 +252,8 @@ PyObject* host_pipe_run(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const void *src[FT_MAX_FANIN], *dst[FT_MAX_FANIN];
   int fanin[FT_MAX_FANIN];
   const at::Tensor* t0 = nullptr;
-  const int n_in = gather_host(args[2], src, &t0), n_out = n_in ? gather_host(args[4], dst, &t0) : 0;
+  Kept kept;
+  const int n_in = gather_host(args[2], src, &t0, &kept), n_out = n_in ? gather_host(args[4], dst, &t0, &kept) : 0;
   if (!n_out || PyList_GET_SIZE(args[3]) != n_out) return other();
   for (int j = 0; j < n_out; ++j) fanin[j] = (int)PyLong_AsLong(PyList_GET_ITEM(args[3], j));
   void* pipe = PyLong_AsVoidPtr(args[0]);

@@ -5,6 +5,8 @@ import subprocess
 import sys
 from pathlib import Path
 
+import pytest
+
 ROOT = Path(__file__).resolve().parents[1]
 
 
@@ -68,3 +70,50 @@ assert [x.tolist() for x in v[0]] == [[0, 1], [2, 3, 4, 5]] and v[1][0].tolist()
 assert v[0][1]._base is t[0] and not v[0][0].requires_grad and v[1][0].requires_grad
 assert N.narrow_all(t, (((0, 7),), ())) is NotImplemented and N.narrow_all([t[0], t[1][:2]], ((), ())) is NotImplemented
 """) == "raised"
+
+
+@pytest.mark.gpu
+def test_tensors_of_a_call_outlive_the_lists_they_came_in():
+    """While a call runs without the GIL, another thread may change the caller's lists.  The library's entry points are
+    replaced by ones that do just that, and look whether the tensors are still there; nothing is launched."""
+    assert child("""
+import ctypes as C, gc, weakref
+from allreduce_over_mpi_b200._lib import _NATIVE
+i, sz, vp, f = C.c_int, C.c_size_t, C.c_void_p, C.c_float
+sig = {"ft_reduce_nway": (i, i, vp, vp, i, sz, i, vp), "ft_reduce_nway_scaled": (i, i, vp, vp, i, sz, f, vp),
+       "ft_local_world_run": (vp, i, vp, vp, sz, i, i, vp, i, i, i, i, i, f, vp),
+       "ft_host_pipe_reduce": (vp, i, i, vp, i, vp, vp, i, sz, vp)}
+seen = {}
+def fake(name):
+    def run(*_):
+        for l in lists:
+            l.clear()
+        gc.collect()
+        seen[name] = all(w() is not None for w in watched)
+        return 0
+    return C.CFUNCTYPE(i, *sig[name])(run)
+keep = {name: fake(name) for name in _NATIVE}
+N.bind({name: C.cast(k, C.c_void_p).value for name, k in keep.items()})
+def call(fn, device, count):
+    global lists, watched
+    lists = [[torch.zeros(64, device=device) for _ in range(2)] for _ in range(count)]
+    watched = [weakref.ref(t) for l in lists for t in l]
+    fn(*lists)
+    assert all(w() is None for w in watched)      # and no longer than the call
+call(lambda a: N.reduce_nway(a, "sum", None, 0), "cuda", 1)
+call(lambda a: N.reduce_nway_scaled(a, 1.0, None, None), "cuda", 1)
+call(lambda a, b: N.local_world_run([1, 2], a, b, "sum", (2,), 0, 0, 1, 0, 1.0), "cuda", 2)
+call(lambda a, b: N.host_pipe_run(1, 0, a, [2, 2], b, "sum"), "cpu", 2)
+print(sorted(seen) == sorted(_NATIVE) and all(seen.values()))
+""") == "True"
+
+
+@pytest.mark.gpu
+def test_a_reduction_inside_vmap_is_refused():
+    assert child("""
+from allreduce_over_mpi_b200.ops import reduce_nway
+try:
+    torch.vmap(lambda x: reduce_nway([x, x]))(torch.zeros(2, 8, device="cuda"))
+except RuntimeError as e:
+    print("storage" in str(e))
+""") == "True"
