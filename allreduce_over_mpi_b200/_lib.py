@@ -155,16 +155,14 @@ _NATIVE = ("ft_reduce_nway", "ft_reduce_nway_scaled", "ft_local_world_run", "ft_
 
 
 def native():
-    """The native call path of the CUDA entry points (lib/_ft_torch.so), bound to the loaded library."""
+    """The native call path of the CUDA entry points (lib/_ft_torch-*.so, built on first use), bound to the loaded library."""
     global _native
     if _native is None:
         import importlib.util
         import torch  # noqa: F401 - its libraries have to be in the process first
         L = lib()
-        path = LIB_PATH.with_name("_ft_torch.so")
-        if not path.exists():
-            from .build import build_ext
-            path = build_ext()
+        from .build import build_ext
+        path = build_ext()
         spec = importlib.util.spec_from_file_location("_ft_torch", path)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)

@@ -12,6 +12,9 @@ cost_model/CMakeLists.txt, vector_add/Makefile, which targets sm_35..sm_86 only)
 from __future__ import annotations
 
 import concurrent.futures as cf
+import contextlib
+import fcntl
+import hashlib
 import os
 import shutil
 import subprocess
@@ -22,7 +25,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "csrc" / "build"
 LIB = PKG / "lib" / "libflextree.so"
-EXT = PKG / "lib" / "_ft_torch.so"
+EXT_SOURCES = (CSRC / "python" / "ft_torch.cpp", CSRC / "api" / "ft_types.h")
 
 NVCC = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -58,10 +61,44 @@ def compile_one(src: Path, verbose: bool, obj_dir: Path = OBJ, defines: tuple = 
     return obj, r.stderr
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile what changed and link; returns the path of the shared library."""
-    OBJ.mkdir(parents=True, exist_ok=True)
+@contextlib.contextmanager
+def _lock():
+    """One build at a time in this tree, whatever the number of ranks that find something missing."""
     LIB.parent.mkdir(parents=True, exist_ok=True)
+    with open(LIB.parent / ".build.lock", "w") as f:
+        fcntl.flock(f, fcntl.LOCK_EX)
+        yield
+
+
+def _produce(cmd: list, out: Path, what: str) -> Path:
+    """Run a compiler or linker on a file of its own and put the result in place whole: a process that finds `out` may
+    load it at once, and one that has the file before it in use keeps that."""
+    part = out.with_name(f".{out.name}.{os.getpid()}")
+    try:
+        r = subprocess.run([*cmd, "-o", str(part)], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"{what} failed:\n{r.stdout}\n{r.stderr}")
+        os.replace(part, out)
+    finally:
+        part.unlink(missing_ok=True)
+    return out
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Compile what changed and link, with the tools and the native call path; returns the path of the shared library."""
+    build_lib(force, verbose)
+    build_ext(force)
+    return LIB
+
+
+def build_lib(force: bool = False, verbose: bool = False) -> Path:
+    """libflextree.so and the tools."""
+    with _lock():
+        return _build_lib(force, verbose)
+
+
+def _build_lib(force: bool, verbose: bool) -> Path:
+    OBJ.mkdir(parents=True, exist_ok=True)
     hm = headers_mtime()
     srcs = sources()
     todo = []
@@ -76,13 +113,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 logs.append(log)
     objs = [OBJ / (s.stem + ".o") for s in srcs]
     if todo or not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):
-        cmd = [NVCC, *ARCH, "-shared", "-cudart", "static", "-o", str(LIB), *map(str, objs),
-               "-Xcompiler", "-fopenmp", "-lpthread", "-ldl", "-lrt"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        _produce([NVCC, *ARCH, "-shared", "-cudart", "static", *map(str, objs), "-Xcompiler", "-fopenmp", "-lpthread", "-ldl", "-lrt"], LIB, "link")
     build_tools()
-    build_ext(force)
     if verbose:
         print("\n".join(logs))
     return LIB
@@ -95,6 +127,11 @@ def build_bounds(force: bool = False) -> Path:
     """The debugging build: the same sources with -DFT_BOUNDS, linked as lib/libflextree_bounds.so.  Its collective
     kernels test every run of heap bytes against the heap size before touching it (csrc/kernels/comm_bounds.h);
     select it with FT_LIB=bounds in the environment of the process that loads the library."""
+    with _lock():
+        return _build_bounds(force)
+
+
+def _build_bounds(force: bool) -> Path:
     obj_dir = PKG / "csrc" / "build_bounds"
     obj_dir.mkdir(parents=True, exist_ok=True)
     hm = headers_mtime()
@@ -106,11 +143,8 @@ def build_bounds(force: bool = False) -> Path:
             list(ex.map(lambda s: compile_one(s, False, obj_dir, ("-DFT_BOUNDS",)), todo))
     objs = [obj_dir / (s.stem + ".o") for s in srcs]
     if todo or not BOUNDS_LIB.exists():
-        cmd = [NVCC, *ARCH, "-shared", "-cudart", "static", "-o", str(BOUNDS_LIB), *map(str, objs),
-               "-Xcompiler", "-fopenmp", "-lpthread", "-ldl", "-lrt"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        _produce([NVCC, *ARCH, "-shared", "-cudart", "static", *map(str, objs), "-Xcompiler", "-fopenmp", "-lpthread", "-ldl", "-lrt"],
+                 BOUNDS_LIB, "link")
     return BOUNDS_LIB
 
 
@@ -133,35 +167,51 @@ def build_tools() -> list[Path]:
     return out
 
 
+def ext_path() -> Path:
+    """Where the native call path for this interpreter, this torch and these sources lies.  The name says what it was
+    compiled from and for: an edit, or another torch beside this one, looks for another file."""
+    import torch
+    h = hashlib.sha256(str(torch.version.git_version).encode())
+    for p in EXT_SOURCES:
+        h.update(p.read_bytes())
+    return LIB.with_name(f"_ft_torch-{sys.implementation.cache_tag}-torch{torch.__version__}-{h.hexdigest()[:16]}.so")
+
+
 def build_ext(force: bool = False) -> Path:
     """The native call path of the Python entry points (csrc/python/ft_torch.cpp), a CPython module on torch's C++
     headers.  It holds no kernels and does not link libflextree: the loader hands it the entry points."""
     import sysconfig
     import torch
-    src = CSRC / "python" / "ft_torch.cpp"
-    if not force and EXT.exists() and EXT.stat().st_mtime >= max(src.stat().st_mtime, (CSRC / "api" / "ft_types.h").stat().st_mtime):
-        return EXT
+    ext = ext_path()
+    if ext.exists() and not force:
+        return ext
     root = Path(torch.__file__).resolve().parent
     cuda = Path(NVCC).resolve().parent.parent
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
-           "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"], str(src), "-o", str(EXT),
-           "-L", str(root / "lib"), f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"{src.name} failed to build:\n{r.stdout}\n{r.stderr}")
-    return EXT
+    src = EXT_SOURCES[0]
+    with _lock():
+        if ext.exists() and not force:   # built by the process that had the lock before
+            return ext
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+               "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"], str(src),
+               "-L", str(root / "lib"), f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+        _produce(cmd, ext, src.name)
+        for old in ext.parent.glob(ext.name.rpartition("-")[0] + "-*.so"):   # of earlier sources, for the same torch
+            if old != ext:
+                old.unlink(missing_ok=True)
+        return ext
 
 
 def ensure_built() -> Path:
-    """Build if the library is missing or older than its sources (needs nvcc)."""
+    """Build the library if it is missing or older than its sources (needs nvcc).  The native call path is looked for,
+    and built, where it is loaded (``_lib.native``)."""
     if LIB.exists():
         newest = max([s.stat().st_mtime for s in sources()] + [headers_mtime()])
-        if LIB.stat().st_mtime >= newest and EXT.exists():
+        if LIB.stat().st_mtime >= newest:
             return LIB
         if not os.path.exists(NVCC):
             return LIB
-    return build()
+    return build_lib()
 
 
 if __name__ == "__main__":
