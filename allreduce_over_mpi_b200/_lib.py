@@ -154,19 +154,36 @@ def lib() -> C.CDLL:
 _NATIVE = ("ft_reduce_nway", "ft_reduce_nway_scaled", "ft_local_world_run", "ft_host_pipe_reduce")
 
 
+class _NoNative:
+    """In place of the native call path where it cannot be built or loaded (no compiler or Python headers, a torch
+    without CUDA, ...): it takes no call, so that each goes through Python and ctypes to the same library."""
+
+    @staticmethod
+    def _hand_back(*args):
+        return NotImplemented
+
+    reduce_nway = reduce_nway_scaled = local_world_run = host_pipe_run = narrow_all = _hand_back
+
+
 def native():
-    """The native call path of the CUDA entry points (lib/_ft_torch-*.so, built on first use), bound to the loaded library."""
+    """The native call path of the CUDA entry points (lib/_ft_torch-*.so, built on first use), bound to the loaded library.
+    It only makes calls cheaper: where it is not to be had, that is said once and the calls take the longer way."""
     global _native
     if _native is None:
         import importlib.util
         import torch  # noqa: F401 - its libraries have to be in the process first
         L = lib()
-        from .build import build_ext
-        path = build_ext()
-        spec = importlib.util.spec_from_file_location("_ft_torch", path)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in _NATIVE})
+        try:
+            from .build import build_ext
+            spec = importlib.util.spec_from_file_location("_ft_torch", build_ext())
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+        except (ImportError, OSError, RuntimeError) as e:
+            import warnings
+            warnings.warn(f"flextree: no native call path, calls cost the host some 15 us more ({e})", RuntimeWarning, stacklevel=3)
+            mod = _NoNative
+        else:
+            mod.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in _NATIVE})
         _native = mod
     return _native
 
