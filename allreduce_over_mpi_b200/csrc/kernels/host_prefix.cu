@@ -14,8 +14,6 @@
 #include "vec.cuh"
 #include "host_prefix.h"
 
-extern "C" void ft_count_launch(uint64_t n);
-
 namespace ftk {
 
 template <int POL>
@@ -58,7 +56,6 @@ static cudaError_t launch_t(const HostPrefixArgs& a, cudaStream_t st) {
   // 32 CTAs of 256 threads with eight inputs, more with fewer
   uint64_t grid = 256 / (a.n_in < 8 ? a.n_in : 8), want = (items + 255) / 256;
   if (grid > want) grid = want;
-  ft_count_launch(1);
   return launch_pdl(host_prefix_kernel<POL>, (unsigned)grid, 256, 0, st, a);
 }
 

@@ -1,4 +1,4 @@
-// Programmatic dependent launch for the short kernels.
+// Launching: what every launch does afterwards, and programmatic dependent launch for the short kernels.
 //
 // Between two kernels of a stream lie about 2 us in which nothing runs: the second one is set up only when the first
 // has completed.  A kernel launched with launch_pdl() is set up when the CTAs of the one before it have left; it calls
@@ -11,8 +11,19 @@
 // with it behind the loads, 2.3 without.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
+
+extern "C" void ft_count_launch(uint64_t n);   // see ft_launch_count()
 
 namespace ftk {
+
+// Behind every launch, with what it answered.  Counts it if it went out; if not, takes the error away from the runtime,
+// which would hand it to the next caller that asks whether ITS launch went well.
+inline cudaError_t launched(cudaError_t e) {
+  if (e == cudaSuccess) ft_count_launch(1);
+  else cudaGetLastError();
+  return e;
+}
 
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -30,7 +41,7 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned threads, s
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  return launched(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 }  // namespace ftk

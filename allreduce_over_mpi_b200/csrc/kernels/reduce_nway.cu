@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "../api/flextree.h"
+#include "pdl.cuh"
 #include "reduce_nway.cuh"
 #include "vec.cuh"
 
@@ -124,8 +125,7 @@ static cudaError_t launch_narrow(const NwayArgs& a, cudaStream_t st) {
   const unsigned long long nwords = a.nvec * 4;   // the aligned part, in 4-byte words (a multiple of 4)
   const unsigned long long threads = nwords / WORDS;
   reduce_nway_narrow_kernel<POL, WORDS><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(a, nwords);
-  g_launches++;
-  return cudaGetLastError();
+  return launched(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------- scalar path
@@ -270,8 +270,7 @@ static cudaError_t launch_vec(const NwayArgs& a, int threads, int ctas_per_sm, c
   int grid = (int)(want < cap ? want : cap);
   if (grid < 1) grid = 1;
   reduce_nway_vec_kernel<POL, UNROLL, GROUP><<<grid, threads, 0, st>>>(a);
-  g_launches++;
-  return cudaGetLastError();
+  return launched(cudaGetLastError());
 }
 
 template <int POL>
@@ -280,8 +279,7 @@ static cudaError_t launch_scalar(const NwayArgs& a, unsigned long long first_uni
   unsigned long long want = (a.nbody - first_unit + 255) / 256;
   unsigned long long cap = (unsigned long long)dev_info().sms * 8;
   reduce_nway_scalar_kernel<POL><<<(int)(want < cap ? want : cap), 256, 0, st>>>(a, first_unit);
-  g_launches++;
-  return cudaGetLastError();
+  return launched(cudaGetLastError());
 }
 
 static int* tma_error_flag() {
@@ -315,8 +313,7 @@ static cudaError_t launch_tma(const NwayArgs& a, cudaStream_t st) {
   int grid = (int)(ntiles < cap ? ntiles : cap);
   if (grid < 1) grid = 1;
   reduce_nway_tma_kernel<POL, STAGES><<<grid, 256, smem, st>>>(a, tile_vecs, tma_error_flag());
-  g_launches++;
-  return cudaGetLastError();
+  return launched(cudaGetLastError());
 }
 
 // Cut the vector for the 32-byte kernel: possible when every pointer has the same offset from a 32-byte boundary
@@ -399,14 +396,11 @@ static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
     e = cudaErrorInvalidValue;
     if (layout_wide(a, bytes, unit, &b)) e = launch_wide(POL, b, variant, variant ? dev_info().sms : 0, st);
     if (e == cudaErrorInvalidValue) {   // other phases, or no such configuration
-      cudaGetLastError();
       const bool realign = layout_realign(a, bytes, unit, &b);
       if (!realign) layout_shift(a, bytes, unit, &b);
       e = launch_shift(POL, b, realign, st);
     }
-    if (e != cudaSuccess) return cuda_fail(e, "reduce_nway launch");
-    g_launches++;
-    return FT_OK;
+    return e == cudaSuccess ? FT_OK : cuda_fail(e, "reduce_nway launch");
   }
   // the configurations that are asked for by number: 16-byte accesses where every pointer allows them, a second
   // launch for the rest
@@ -492,8 +486,7 @@ int ft_scale_inplace(int dtype, void* buf, size_t len, float scale, void* stream
     case POL_BF16: scale_inplace_kernel<POL_BF16><<<grid, 256, 0, st>>>(buf, nvec, len, scale); break;
     default: scale_inplace_kernel<POL_F16><<<grid, 256, 0, st>>>(buf, nvec, len, scale); break;
   }
-  g_launches++;
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launched(cudaGetLastError());
   return e == cudaSuccess ? FT_OK : cuda_fail(e, "scale launch");
 }
 
@@ -543,7 +536,6 @@ int ft_reduce_nway_scaled(int in_dtype, int out_dtype, const void* const* src, v
   a.dst = dst;
   a.n = n;
   const cudaError_t e = launch_scaled(in_dtype == FT_BF16, out_dtype == FT_BF16, a, len, scale, dev_info().sms, (cudaStream_t)stream);
-  g_launches++;
   return e == cudaSuccess ? FT_OK : cuda_fail(e, "reduce_nway_scaled launch");
 }
 

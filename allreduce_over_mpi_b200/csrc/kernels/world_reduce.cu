@@ -13,8 +13,6 @@
 #include "vec.cuh"
 #include "world_dev.h"
 
-extern "C" void ft_count_launch(uint64_t n);
-
 namespace ftk {
 
 constexpr int kWorldThreads = 128;
@@ -131,7 +129,6 @@ static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t
   const uint64_t most = std::max(a.total_bytes > a.block_bytes ? a.block_bytes / (V * 16) : 0, last / (V * 16) + last % (V * 16) / a.es);
   const uint64_t per = (most + kWorldThreads - 1) / kWorldThreads;
   if (per == 0 || per > 0x7fffffffull) return cudaErrorInvalidValue;
-  ft_count_launch(1);
   return launch_pdl(world_reduce_kernel<POL, V, DEPTH, G, RANKS>, dim3((unsigned)per, (unsigned)entries), kWorldThreads, 0, st, a);
 }
 

@@ -74,7 +74,7 @@ unsigned char* pinned_address(const void* p, size_t bytes) {
 // result overlaps an input or another result: the chunked path reads all inputs of a chunk before it writes and writes
 // the results in the caller's order, and what it does there stays what happens.
 int run_direct(int op, int dtype, const void* const* src, const int* fanin, void* const* dst, int n_out, size_t bytes, size_t es,
-               cudaStream_t st) {
+               cudaStream_t st, cudaError_t* err) {
   const int pol = ftk::policy_id(op, dtype);
   if (pol < 0) return FT_ERR_NOT_AVAILABLE;
   ftk::HostPrefixArgs a;
@@ -103,8 +103,8 @@ int run_direct(int op, int dtype, const void* const* src, const int* fanin, void
   a.first[a.n_in] = (uint8_t)filled;
   a.bytes = bytes;
   a.es = (uint32_t)es;
-  const cudaError_t e = ftk::launch_host_prefix(pol, a, st);
-  return e == cudaSuccess ? FT_OK : FT_ERR_CUDA;
+  *err = ftk::launch_host_prefix(pol, a, st);
+  return *err == cudaSuccess ? FT_OK : FT_ERR_CUDA;
 }
 }  // namespace
 
@@ -161,8 +161,9 @@ int ft_host_pipe_reduce(ft_host_pipe* p, int op, int dtype, const void* const* h
     if (fanin[j] < 1 || fanin[j] > n_in) return fail(p, FT_ERR_INVALID_ARG, "fan-in outside 1..n_in");
   if (len == 0) return FT_OK;
   HP_CUDA(p, cudaSetDevice(p->device));
-  if (const int rc = run_direct(op, dtype, host_src, fanin, host_dst, n_out, len * es, es, (cudaStream_t)stream); rc != FT_ERR_NOT_AVAILABLE)
-    return rc == FT_OK ? rc : fail(p, rc, cudaGetErrorString(cudaGetLastError()));
+  cudaError_t err = cudaSuccess;
+  if (const int rc = run_direct(op, dtype, host_src, fanin, host_dst, n_out, len * es, es, (cudaStream_t)stream, &err); rc != FT_ERR_NOT_AVAILABLE)
+    return rc == FT_OK ? rc : fail(p, rc, std::string("host prefix launch: ") + cudaGetErrorString(err));
   constexpr int D = ft_host_pipe::kDepth;
   const size_t per = p->chunk_bytes / es;
   cudaStream_t user = (cudaStream_t)stream;
