@@ -7,6 +7,7 @@ namespace ftk {
 
 constexpr int kWorldRanks = 16;      // ranks, and entries of a program, that fit the kernel's parameters
 constexpr int kMaxRounds = 4;        // copies that may be finished after one step
+constexpr int kWorldGroup = 8;       // steps whose sources the kernel looks up together, also behind the last one
 constexpr uint8_t kNoStore = 0xff;
 
 // Take the next value: start an accumulator with it (a running one is put aside) or add it.  Then `rounds` times:
@@ -28,7 +29,8 @@ template <int RANKS>
 struct WorldArgs {
   void* out[RANKS];
   WorldEntry entry[RANKS];
-  const void* src[RANKS * RANKS];      // of step k: the copy it takes (any valid pointer behind the last step)
+  // of step k: the copy it takes; behind the last step rank 0's, which the kernel looks up and does not read
+  const void* src[RANKS * RANKS + kWorldGroup - 1];
   uint8_t code[RANKS * RANKS];
   uint8_t store[RANKS * RANKS][kMaxRounds];
   uint64_t total_bytes, block_bytes;

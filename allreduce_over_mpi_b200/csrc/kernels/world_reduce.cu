@@ -47,6 +47,7 @@ __device__ __forceinline__ void world_store(unsigned char* p, bool ok, const uin
 template <int POL, int V, int DEPTH, int G, int RANKS>
 __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __grid_constant__ WorldArgs<RANKS> a) {
   using P = typename PolById<POL>::type;
+  static_assert(G <= kWorldGroup, "the parameters are filled for this many");
   pdl_begin();
   const int first = a.entry[blockIdx.y].first, nsteps = a.entry[blockIdx.y].nsteps;
   const uint32_t mask = (uint32_t)a.entry[blockIdx.y].mask;

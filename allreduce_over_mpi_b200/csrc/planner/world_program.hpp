@@ -11,6 +11,7 @@
 // that the results are the same bits.  Plans it cannot linearise (a block that ends in two different expressions, a
 // nesting deeper than the kernel's stack) come back with ok = false and are run stage by stage.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <vector>
@@ -27,6 +28,21 @@ struct WorldProgram {
   std::vector<ftk::WorldEntry> entries;      // one per block and pass over it
   std::vector<ftk::WorldStep> steps;         // entries[i] uses steps [first, first + nsteps)
 };
+
+// What the kernel gets of a program for the inputs of a call.  False: more than its parameters hold.
+template <int RANKS>
+bool fill_world_steps(const WorldProgram& wp, const void* const* in, ftk::WorldArgs<RANKS>* a) {
+  if (wp.entries.size() > (std::size_t)RANKS || wp.steps.size() > (std::size_t)RANKS * RANKS) return false;
+  std::copy(wp.entries.begin(), wp.entries.end(), a->entry);
+  for (std::size_t k = 0; k < wp.steps.size(); ++k) {
+    const ftk::WorldStep& s = wp.steps[k];
+    a->src[k] = in[s.rank];
+    a->code[k] = (uint8_t)(s.start | s.pop << 1 | s.rounds << 2);
+    std::copy(s.store, s.store + ftk::kMaxRounds, a->store[k]);
+  }
+  std::fill_n(a->src + wp.steps.size(), ftk::kWorldGroup - 1, in[0]);
+  return true;
+}
 
 enum class WorldPhase { all, reduce_scatter, all_gather };
 

@@ -502,13 +502,7 @@ cudaError_t world_launch(const ft::WorldProgram& wp, int pol, int world, const v
     a.out[r] = r < world ? out[r] : nullptr;
     all |= r < world ? (uintptr_t)in[r] | (uintptr_t)out[r] : 0;
   }
-  std::copy(wp.entries.begin(), wp.entries.end(), a.entry);
-  for (size_t k = 0; k < wp.steps.size(); ++k) {
-    const ftk::WorldStep& s = wp.steps[k];
-    a.src[k] = in[s.rank];
-    a.code[k] = (uint8_t)(s.start | s.pop << 1 | s.rounds << 2);
-    std::copy(s.store, s.store + ftk::kMaxRounds, a.store[k]);
-  }
+  if (!ft::fill_world_steps(wp, in, &a)) return cudaErrorInvalidValue;   // (asked by the caller)
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
   a.es = es;

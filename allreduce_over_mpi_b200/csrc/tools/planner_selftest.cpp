@@ -3,7 +3,8 @@
 //     g++ -std=c++17 -O1 -g -fsanitize=thread planner_selftest.cpp -o t -lpthread && ./t threads
 // It builds the plan of every executable shape up to 24 ranks, runs the static race check and the
 // snapshot executor against a double-precision sum, exercises the candidate enumerators and the
-// cost models, checks the device tables (and that damaged ones are refused) and the heap allocator, and (argument "threads") runs the thread-per-rank executor with its flag protocol,
+// cost models, checks the device tables (and that damaged ones are refused), the one-pass programs of a world on one
+// device and the heap allocator, and (argument "threads") runs the thread-per-rank executor with its flag protocol,
 // including a silent rank that must produce time-outs rather than a hang.
 // The reference has no sanitizer builds (its flags are -Wall -Wextra only, allreduce_over_mpi/CMakeLists.txt:5).
 #include <sys/wait.h>
@@ -20,6 +21,7 @@
 #include "../planner/cpu_executor.hpp"
 #include "../planner/policy.hpp"
 #include "../planner/proc_world.hpp"
+#include "../planner/world_program.hpp"
 #include "../runtime/dev_plan.hpp"
 #include "../runtime/heap_alloc.hpp"
 #include "../runtime/fd_channel.cpp"   // descriptor passing over abstract unix sockets: plain host code, compiled in here
@@ -445,9 +447,85 @@ static void thread_world_small_message_twins() {
   }
 }
 
+// One pass over the copies of all ranks, as world_reduce_kernel does it for one element of each block: in place, the
+// inputs read as late as the program asks for them, no more values put aside than the program says.
+static char rank_copy[ftk::kWorldRanks];   // the ranks' "addresses"
+template <int RANKS>
+static void run_world_args(const ftk::WorldArgs<RANKS>& a, int entries, int depth, uint16_t (*copy)[ftk::kWorldRanks]) {
+  const auto at = [&](const void* rank, int block) -> uint16_t& { return copy[(const char*)rank - rank_copy][block]; };
+  for (int e = 0; e < entries; ++e) {
+    const ftk::WorldEntry& en = a.entry[e];
+    float acc = 0;
+    std::vector<float> aside(depth > 0 ? depth : 1, 0.f);
+    for (int k = en.first; k < en.first + en.nsteps; ++k) {
+      const float v = ft::bf16_to_float({at(a.src[k], en.block)});
+      if (depth == 0) { acc = k == en.first ? v : acc + v; continue; }
+      if (a.code[k] & 1) {
+        aside.insert(aside.begin(), acc);
+        aside.pop_back();
+        acc = v;
+      } else {
+        acc += v;
+      }
+      const int rounds = a.code[k] >> 2;
+      for (int r = 0; r < rounds; ++r) {
+        const ft::bf16_t w = ft::float_to_bf16(acc);
+        if (a.store[k][r] != ftk::kNoStore) at(a.out[a.store[k][r]], en.block) = w.bits;
+        acc = ft::bf16_to_float(w);
+        if (r + 1 < rounds || (a.code[k] & 2)) {
+          acc = aside[0] + acc;
+          aside.erase(aside.begin());
+          aside.push_back(0.f);
+        }
+      }
+    }
+    for (int r = 0; r < RANKS; ++r)
+      if (en.mask >> r & 1) at(a.out[r], en.block) = ft::float_to_bf16(acc).bits;
+  }
+}
+template <int RANKS>
+static bool world_program_as_plan(int n, const ft::Plan& p, ft::WorldPhase phase) {
+  const ft::WorldProgram wp = ft::WorldProgramBuilder(n).run(p, phase);
+  if (!wp.ok || wp.depth > (RANKS == 8 ? 2 : 3)) return false;
+  const void* in[RANKS];
+  ftk::WorldArgs<RANKS> a;
+  std::memset((void*)&a, 0xab, sizeof a);
+  for (int r = 0; r < RANKS; ++r) in[r] = a.out[r] = rank_copy + r;
+  if (!ft::fill_world_steps(wp, in, &a)) return false;
+  for (const ftk::WorldEntry& e : wp.entries)   // the kernel looks up whole groups of steps
+    for (int k = 0; k < (e.nsteps + ftk::kWorldGroup - 1) / ftk::kWorldGroup * ftk::kWorldGroup; ++k) {
+      EXPECT((const void* const*)&a.src[e.first + k] < (const void* const*)(&a.src + 1));
+      EXPECT(a.src[e.first + k] >= in[0] && a.src[e.first + k] <= in[n - 1]);
+    }
+  uint16_t got[ftk::kWorldRanks][ftk::kWorldRanks] = {}, want[ftk::kWorldRanks][ftk::kWorldRanks] = {};
+  void* bufs[ftk::kWorldRanks];
+  for (int r = 0; r < n; ++r) {
+    for (int b = 0; b < n; ++b) want[r][b] = got[r][b] = ft::float_to_bf16((float)std::sin(r * 131 + b * 7 + 1)).bits;
+    bufs[r] = want[r];
+  }
+  const int half = p.num_stages / 2;
+  EXPECT(ft::run_plan_snapshot(p, FT_SUM, FT_BF16, bufs, n, 1, phase == ft::WorldPhase::all_gather ? half : 0,
+                               phase == ft::WorldPhase::reduce_scatter ? half : -1) == FT_OK);
+  run_world_args(a, (int)wp.entries.size(), wp.depth, got);
+  EXPECT(!std::memcmp(got, want, sizeof got));
+  return true;
+}
+static void world_programs() {
+  int shapes = 0, taken = 0;
+  for (int n = 2; n <= ftk::kWorldRanks; ++n)
+    for (const ft::Shape& s : ft::executable_shapes(n)) {
+      const ft::Plan p = ft::build_plan(n, s);
+      for (ft::WorldPhase phase : {ft::WorldPhase::all, ft::WorldPhase::reduce_scatter, ft::WorldPhase::all_gather}) {
+        ++shapes;
+        taken += n <= 8 ? world_program_as_plan<8>(n, p, phase) : world_program_as_plan<16>(n, p, phase);
+      }
+    }
+  EXPECT(shapes > 250 && taken == shapes);
+}
+
 int main(int argc, char** argv) {
   const bool threads = argc > 1 && !std::strcmp(argv[1], "threads");
-  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
+  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
   thread_world(false);
   thread_world_phases();
   thread_world_small_message_twins();
