@@ -4,20 +4,21 @@ from __future__ import annotations
 import torch
 
 from ..models.gpt2 import GPT2, GPT2Config
+from ..ops import HostReducePipeline, launch_count, reduce_nway, reduce_nway_scaled
 from .comm import LocalWorld
 from .ddp import FlexTreeDDP
 
 
-def smoke_comm_and_model(dev: torch.device) -> None:
-    # four ranks emulated on this GPU: tree 2*2 and one-shot, checked against a plain sum
+def smoke_worlds(dev: torch.device, fused: bool) -> None:
+    """Worlds of four and five ranks on this GPU: a tree, one-shot, tagged words, reduce + push and a lonely layout, each
+    in one launch of the kernel for worlds on one device (``fused``) or through the kernels that several GPUs run."""
     w = LocalWorld(4, devices=[dev.index] * 4, heap_bytes=4 << 20, staging_bytes=1 << 20)
+    w.fused = fused
+    before = launch_count()
     xs = [torch.full((10_000,), float(r + 1), device=dev) for r in range(4)]
     w.all_reduce(xs, shape="2*2")
     ys = [torch.full((999,), float(r + 1), device=dev).bfloat16() for r in range(4)]
     w.all_reduce(ys, algo="oneshot")
-    torch.cuda.synchronize(dev)
-    assert all(bool((x == 10).all()) for x in xs) and all(bool((y == 10).all()) for y in ys)
-    # the low-latency push protocol, the flat reduce + push kernel (heap tensors) and a lonely layout, same world
     zs = [torch.full((777,), float(r + 1), device=dev) for r in range(4)]
     w.all_reduce(zs, algo="ll")
     ps = [w.ranks[r].alloc(4096, torch.bfloat16) for r in range(4)]
@@ -25,17 +26,24 @@ def smoke_comm_and_model(dev: torch.device) -> None:
         p.fill_(float(r + 1))
     w.all_reduce(ps, algo="push", op="avg")
     torch.cuda.synchronize(dev)
+    assert all(bool((x == 10).all()) for x in xs) and all(bool((y == 10).all()) for y in ys)
     assert all(bool((z == 10).all()) for z in zs) and all(bool((p == 2.5).all()) for p in ps)
+    assert (launch_count() - before == 4) == fused, "the other form ran"
     w.close()
     w5 = LocalWorld(5, devices=[dev.index] * 5, heap_bytes=1 << 20, staging_bytes=1 << 20)
+    w5.fused = fused
     ls = [torch.full((1000,), float(r + 1), device=dev) for r in range(5)]
     w5.all_reduce(ls, shape="2*2+1")
     torch.cuda.synchronize(dev)
     assert all(bool((x == 15).all()) for x in ls)
     w5.close()
+
+
+def smoke_comm_and_model(dev: torch.device) -> None:
+    for fused in (True, False):
+        smoke_worlds(dev, fused)
     # single-GPU n-way reduce: 8 bytes per thread (fp32, fan-in 4), 32-byte accesses, the scaled / casting kernel,
     # and the pipeline for operands in host memory
-    from ..ops import HostReducePipeline, reduce_nway, reduce_nway_scaled
     fs = [torch.randn(1 << 16, device=dev) for _ in range(4)]
     want = torch.stack(fs).sum(0)
     assert torch.allclose(reduce_nway(fs), want, atol=1e-5)                  # 32-byte accesses (the default)

@@ -1,11 +1,14 @@
 """A world on one device: the one-launch form against the kernels that several devices would run.
 
-The tests of test_comm_emulated_gpu.py call whatever ``LocalWorld`` runs by default, the one-launch form; they are
-collected here a second time with it switched off, so that the multi-GPU kernels stay covered on one GPU."""
+The tests of test_comm_emulated_gpu.py, and those of test_y_comm_extras_gpu.py on worlds of several ranks, call whatever
+``LocalWorld`` runs by default, the one-launch form; they are collected here a second time with it switched off, so that
+the multi-GPU kernels stay covered on one GPU: their sums, the guard blocks behind the tensors they write, and the
+stage ranges of the two halves (everything a rank does not own is NaN before the gather)."""
 import pytest
 import torch
 
 import test_comm_emulated_gpu as emulated
+import test_y_comm_extras_gpu as extras
 from allreduce_over_mpi_b200.ops import launch_count
 from allreduce_over_mpi_b200.parallel.comm import LocalWorld
 from allreduce_over_mpi_b200.parallel.planner import Shape
@@ -17,11 +20,18 @@ DEV = "cuda:0"
 class TestStageByStage:
     @pytest.fixture(autouse=True)
     def unfused(self, monkeypatch):
+        def refuse(*_):
+            raise AssertionError("the one-launch form was asked")
         monkeypatch.setattr(LocalWorld, "fused", False)
+        monkeypatch.setattr(LocalWorld, "_run_fused", refuse)
 
     for _name in dir(emulated):
         if _name.startswith("test_"):
             locals()[_name] = staticmethod(getattr(emulated, _name))
+    for _name in ("test_reduce_scatter_and_all_gather_alone", "test_phases_refuse_tensors_outside_the_heap",
+                  "test_guard_blocks_behind_heap_tensors_stay_intact", "test_unaligned_slice_of_a_heap_tensor_goes_through_the_slots",
+                  "test_heap_free_and_reuse"):
+        locals()[_name] = staticmethod(getattr(extras, _name))
 
 
 def both(world, make, call):
