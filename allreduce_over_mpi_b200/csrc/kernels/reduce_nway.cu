@@ -316,77 +316,6 @@ static cudaError_t launch_tma(const NwayArgs& a, cudaStream_t st) {
   return launched(cudaGetLastError());
 }
 
-// Cut the vector for the 32-byte kernel: possible when every pointer has the same offset from a 32-byte boundary
-// (a slice of a flat buffer reduced into the same slice of another, or whole tensors).
-static bool layout_wide(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
-  uintptr_t differ = 0;
-  for (int k = 0; k < in.n; ++k) differ |= (uintptr_t)in.src[k] ^ (uintptr_t)in.dst;
-  if (differ & 31) return false;
-  // The body starts on a 128-byte line where that is possible, or each 1 KiB request of a warp touches nine lines
-  // instead of eight: bf16 x2 of 4 M one element off, in L2, took 3.2 us from the next 32 bytes and 2.9 from the next line.
-  const size_t to = (differ & 127) == 0 && bytes >= 4096 ? 128 : 32;
-  const size_t head = (to - ((uintptr_t)in.dst & (to - 1))) & (to - 1);
-  if (bytes < head + 32) return false;
-  *out = in;
-  out->nvec = (bytes - head) / 32;
-  out->nbody = out->nvec * 32 / unit;
-  out->head = (uint16_t)(head / unit);
-  out->edge = (uint16_t)((bytes - out->nvec * 32) / unit);
-  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
-  out->dst = (unsigned char*)in.dst + head;
-  return true;
-}
-// Cut it for the realigning kernel: the sources agree modulo 32, the result lies elsewhere.  The body is what the
-// result's whole 32-byte units between the first and the last whole unit of the sources hold.
-static bool layout_realign(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
-  const uintptr_t phase = (uintptr_t)in.src[0] & 31;
-  for (int k = 1; k < in.n; ++k)
-    if (((uintptr_t)in.src[k] & 31) != phase) return false;
-  const size_t first = (32 - phase) & 31;   // bytes in front of the sources' first whole unit
-  const size_t shift = (32 - (((uintptr_t)in.dst + first) & 31)) & 31, head = first + shift;
-  if (shift == 0 || bytes < first + 64) return false;
-  *out = in;
-  out->nvec = (bytes - first) / 32 - 1;
-  out->nbody = out->nvec * 32 / unit;
-  out->head = (uint16_t)(head / unit);
-  out->edge = (uint16_t)((bytes - out->nvec * 32) / unit);
-  out->shift[0] = (uint8_t)shift;
-  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
-  out->dst = (unsigned char*)in.dst + head;
-  return true;
-}
-// Cut it on the result's 16-byte boundaries for the shifted kernel.  A source that lies s bytes behind such a
-// boundary is read from s bytes before the body to 16 - s bytes behind it; the body is kept small enough for these
-// to be the vector's own bytes.  A vector too short for that is all edges.
-static void layout_shift(const NwayArgs& in, size_t bytes, size_t unit, NwayArgs* out) {
-  *out = in;
-  size_t head = (16 - ((uintptr_t)in.dst & 15)) & 15, widest = 0;
-  bool any = false;
-  for (int k = 0; k < in.n; ++k) {
-    out->shift[k] = (uint8_t)(((uintptr_t)in.src[k] + head) & 15);
-    any = any || out->shift[k];
-    if (out->shift[k] > widest) widest = out->shift[k];
-  }
-  if (widest > head) head += 16;
-  unsigned long long nvec = bytes > head ? (bytes - head) / 16 : 0;
-  for (int k = 0; k < in.n; ++k)
-    if (out->shift[k]) {
-      const unsigned long long whole = (bytes > head ? bytes - head + out->shift[k] : 0) / 16;
-      const unsigned long long fits = whole ? whole - 1 : 0;
-      if (fits < nvec) nvec = fits;
-    }
-  if (!nvec) {   // no body, and with it no vector behind the body for the kernel to look at
-    head = 0;
-    for (int k = 0; k < in.n; ++k) out->shift[k] = 0;
-  }
-  out->nvec = nvec;
-  out->nbody = nvec * 16 / unit;
-  out->head = (uint16_t)(head / unit);
-  out->edge = (uint16_t)((bytes - nvec * 16) / unit);
-  for (int k = 0; k < in.n; ++k) out->src[k] = (const unsigned char*)in.src[k] + head;
-  out->dst = (unsigned char*)in.dst + head;
-}
-
 template <int POL>
 static int run_policy(NwayArgs& a, size_t bytes, int variant, cudaStream_t st) {
   const size_t unit = sizeof(typename ScalarOp<POL>::elem);

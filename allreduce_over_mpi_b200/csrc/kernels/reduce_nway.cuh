@@ -1,25 +1,13 @@
-// Argument block of the single-GPU n-way reduction kernels (reduce_nway.cu, reduce_nway_wide.cu,
-// reduce_nway_shift.cu, reduce_nway_scaled.cu).
+// The single-GPU n-way reduction kernels as reduce_nway.cu launches them (reduce_nway_wide.cu, reduce_nway_shift.cu,
+// reduce_nway_scaled.cu), and the part they share.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../api/ft_types.h"
+#include "nway_layout.h"
 
 namespace ftk {
-
-// One launch covers a whole vector: the body in 32- or 16-byte vectors, and the elements in front of and behind it
-// (the edges) one by one in a CTA of their own (the last one), so that neither a ragged length nor a slice that starts
-// off a vector boundary costs a second launch or takes the rest of the vector off the vector loads.
-struct NwayArgs {
-  const void* src[FT_MAX_FANIN];  // start of the body in every source
-  void* dst;
-  unsigned long long nvec;    // body length, in the kernel's vectors
-  unsigned long long nbody;   // ... and in scalar units (see ScalarOp)
-  int n;
-  uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
-  uint8_t shift[FT_MAX_FANIN];  // shifted kernels: bytes by which source k's body lies behind a 16-byte (realign: 32-byte) boundary
-};
 
 // Kernels for pointers that agree modulo 32 (reduce_nway_wide.cu).  `code` selects a configuration (0: by size;
 // see launch_cfg there); returns cudaErrorInvalidValue when (policy, fan-in, code) has no instantiation.

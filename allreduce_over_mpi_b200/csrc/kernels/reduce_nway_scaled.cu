@@ -13,7 +13,7 @@
 
 namespace ftk {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = kWideThreads;
 
 template <bool WIDE>
 __device__ __forceinline__ void load32(const unsigned char* p, uint4& a, uint4& b) {
@@ -103,16 +103,6 @@ __global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __
     scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, scale);
 }
 
-// First element from which every source lies on a boundary of `sa` bytes and the output on one of `da`, or -1.
-static int common_head(const NwayArgs& a, size_t is, size_t os, size_t sa, size_t da) {
-  for (size_t h = 0; h < sa / is; ++h) {
-    bool ok = ((uintptr_t)a.dst + h * os) % da == 0;
-    for (int k = 0; ok && k < a.n; ++k) ok = ((uintptr_t)a.src[k] + h * is) % sa == 0;
-    if (ok) return (int)h;
-  }
-  return -1;
-}
-
 // Two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up the loop is as good or
 // better (with the fan-in known the compiler keeps fewer loads in flight: bf16 x8 of 4 M 14.3 us, not 12.0).  Eight
 // sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with four, 24.7
@@ -129,25 +119,14 @@ static cudaError_t launch_n(const NwayArgs& a, unsigned grid, float scale, cudaS
 }
 
 template <bool IN_BF16, bool OUT_BF16>
-static cudaError_t launch_t(NwayArgs a, unsigned long long len, float scale, int sms, cudaStream_t st) {
-  constexpr unsigned long long E = IN_BF16 ? 16 : 8;
-  constexpr size_t is = IN_BF16 ? 2 : 4, os = OUT_BF16 ? 2 : 4;
-  bool wide = true;
-  constexpr size_t da = IN_BF16 || !OUT_BF16 ? 32 : 16;
-  int head = len >= 4096 / is ? common_head(a, is, os, 128, da) : -1;   // whole lines: see layout_wide in reduce_nway.cu
-  if (head < 0) head = common_head(a, is, os, 32, da);
-  if (head < 0) { wide = false; head = common_head(a, is, os, 16, 16); }
-  if (head < 0) {
+static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, float scale, int sms, cudaStream_t st) {
+  NwayArgs a;
+  bool wide;
+  if (!layout_scaled(in, len, IN_BF16, OUT_BF16, &a, &wide)) {
     const unsigned long long want = (len + 255) / 256, cap = (unsigned long long)sms * 8;
-    return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, a, len, scale);
+    return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, in, len, scale);
   }
-  a.nvec = len >= head + E ? (len - head) / E : 0;   // shorter: all edges
-  a.nbody = a.nvec * E;
-  a.head = (uint16_t)(a.nvec ? head : 0);
-  a.edge = (uint16_t)(len - a.nbody);
-  for (int k = 0; k < a.n; ++k) a.src[k] = (const unsigned char*)a.src[k] + a.head * is;
-  a.dst = (unsigned char*)a.dst + a.head * os;
-  const unsigned long long grid = (a.nvec + kThreads - 1) / kThreads + (a.edge != 0);
+  const unsigned long long grid = nway_grid(a, kThreads);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
   return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, scale, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, scale, st);
 }

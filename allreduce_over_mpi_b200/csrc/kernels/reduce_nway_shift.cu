@@ -5,7 +5,7 @@
 // bytes behind a boundary there is read with aligned 16-byte loads, and each lane puts its vector together from
 // its own load and its right neighbour's (a warp shuffle; lane 31 loads the one vector more).  Memory bounds the
 // kernel: every byte is still read once, where the one-element loads this replaces moved 4 bytes an instruction.
-// The host keeps all loads inside the vectors (layout_shift in reduce_nway.cu).
+// The host keeps all loads inside the vectors (layout_shift in nway_layout.h).
 //
 // Where all sources lie at one phase and only the result at another (views summed into a new tensor), the second
 // kernel keeps 256-bit loads on the sources' boundaries and moves the RESULT across: one shuffle step per 32 bytes of
@@ -104,11 +104,11 @@ __device__ __forceinline__ void join32(const uint32_t (&lo)[8], const uint32_t (
 // next warp sums the last one again (a hit in L2).  a.nvec: units of the result; shift[0]: bytes by which it lies behind
 // the sources' boundaries.  bf16 x8 of 4 M, sources one element off: 14.3 us by the kernel above, 12.0 here.
 template <int POL, int GROUP>
-__global__ void __launch_bounds__(128) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
+__global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   pdl_begin();
   const uint32_t lane = threadIdx.x & 31, shift = a.shift[0];
-  const unsigned long long i = ((unsigned long long)blockIdx.x * 4 + threadIdx.x / 32) * 31 + lane;
+  const unsigned long long i = (unsigned long long)blockIdx.x * kRealignPerCta + threadIdx.x / 32 * 31 + lane;
   const bool ok = i <= a.nvec;   // one unit more than the result has
   typename P::Acc al, ah;
   for (int k0 = 0; k0 < a.n; k0 += GROUP) {
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(128) reduce_nway_realign_kernel(const __grid_c
 
 template <int POL, int UNROLL, int GROUP, int THREADS>
 static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
-  const unsigned long long grid = (a.nvec + THREADS * UNROLL - 1) / (THREADS * UNROLL) + (a.edge != 0);
+  const unsigned long long grid = nway_grid(a, THREADS * UNROLL);
   if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
   return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, a);
 }
@@ -153,12 +153,12 @@ static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
 template <int POL>
 static cudaError_t launch_t(const NwayArgs& a, bool realign, cudaStream_t st) {
   if (realign) {
-    const unsigned long long grid = (a.nvec + 4 * 31 - 1) / (4 * 31) + (a.edge != 0);
+    const unsigned long long grid = nway_grid(a, kRealignPerCta);
     if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-    return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, 128, 0, st, a)
-                    : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, 128, 0, st, a);
+    return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, kRealignThreads, 0, st, a)
+                    : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, kRealignThreads, 0, st, a);
   }
-  return a.nvec >= (3u << 20) / 16 ? launch_t<POL, 2, 2, 64>(a, st) : launch_t<POL, 1, 4, 128>(a, st);
+  return shift_long(a) ? launch_t<POL, 2, 2, 64>(a, st) : launch_t<POL, 1, 4, 128>(a, st);
 }
 
 cudaError_t launch_shift(int pol, const NwayArgs& a, bool realign, cudaStream_t st) {

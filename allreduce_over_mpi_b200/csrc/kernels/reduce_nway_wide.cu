@@ -157,9 +157,9 @@ static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t
   const int t = code % 10;
   if (t != 0 && t != 1 && t != 3) return cudaErrorInvalidValue;
   if (code == 0) {
-    const unsigned long long grid = (a.nvec + 127) / 128 + (a.edge != 0);
+    const unsigned long long grid = nway_grid(a, kWideThreads);
     if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, 128, NSRC == 0 ? 8 : 4>, (unsigned)grid, 128, 0, st, a);
+    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4>, (unsigned)grid, kWideThreads, 0, st, a);
   }
   if constexpr (TUNING) {
     switch (code / 10) {

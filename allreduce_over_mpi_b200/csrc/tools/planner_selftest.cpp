@@ -4,7 +4,7 @@
 // It builds the plan of every executable shape up to 24 ranks, runs the static race check and the
 // snapshot executor against a double-precision sum, exercises the candidate enumerators and the
 // cost models, checks the device tables (and that damaged ones are refused), the one-pass programs of a world on one
-// device and the heap allocator, and (argument "threads") runs the thread-per-rank executor with its flag protocol,
+// device, every access of the single-GPU reductions and the heap allocator, and (argument "threads") runs the thread-per-rank executor with its flag protocol,
 // including a silent rank that must produce time-outs rather than a hang.
 // The reference has no sanitizer builds (its flags are -Wall -Wextra only, allreduce_over_mpi/CMakeLists.txt:5).
 #include <sys/wait.h>
@@ -16,6 +16,7 @@
 #include <thread>
 #include <vector>
 
+#include "../kernels/nway_layout.h"
 #include "../planner/config.hpp"
 #include "../planner/cost_model.hpp"
 #include "../planner/cpu_executor.hpp"
@@ -523,9 +524,137 @@ static void world_programs() {
   EXPECT(shapes > 250 && taken == shapes);
 }
 
+// Every access of every thread of the single-GPU reductions, for the way the host cuts the vectors: reads inside the
+// sources and on the boundaries the instructions need, each element of the result written once.
+struct NwayReplay {
+  ftk::NwayArgs whole, a;      // before and after the cut
+  size_t is, os, len;          // bytes of an element of the sources, of the result; elements
+  std::vector<uint8_t> written;
+  bool good = true;
+  void need(bool ok) { good = good && ok; }
+  void read(int k, const void* p, size_t bytes, size_t align) {
+    const uintptr_t lo = (uintptr_t)whole.src[k];
+    need((uintptr_t)p % align == 0 && (uintptr_t)p >= lo && (uintptr_t)p + bytes <= lo + len * is);
+  }
+  void write(const void* p, size_t bytes, size_t align) {
+    const uintptr_t lo = (uintptr_t)whole.dst;
+    const bool in = (uintptr_t)p % align == 0 && (uintptr_t)p >= lo && (uintptr_t)p + bytes <= lo + len * os;
+    need(in);
+    for (size_t b = 0; in && b < bytes; ++b) need(++written[(uintptr_t)p - lo + b] == 1);
+  }
+  const unsigned char* src(int k, long long bytes) const { return (const unsigned char*)((uintptr_t)a.src[k] + bytes); }
+  const unsigned char* dst(long long bytes) const { return (const unsigned char*)((uintptr_t)a.dst + bytes); }
+  void edges(int thread, int threads) {
+    for (int e = thread; e < a.edge; e += threads) {
+      const long long i = e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head));
+      for (int k = 0; k < a.n; ++k) read(k, src(k, i * (long long)is), is, is);
+      write(dst(i * (long long)os), os, os);
+    }
+  }
+  // wide and scaled kernels: 32 bytes of every source a thread, `out` bytes of the result
+  void wide(size_t load, size_t out, size_t store) {
+    const unsigned long long grid = ftk::nway_grid(a, ftk::kWideThreads);
+    need(grid > 0);
+    for (unsigned long long cta = 0; cta < grid; ++cta)
+      for (unsigned t = 0; t < ftk::kWideThreads; ++t) {
+        const unsigned long long i = cta * ftk::kWideThreads + t;
+        if (i < a.nvec) {
+          for (int k = 0; k < a.n; ++k) read(k, src(k, i * 32), 32, load);
+          write(dst(i * out), out, store);
+        } else if (cta == grid - 1) {
+          edges(t, ftk::kWideThreads);
+        }
+      }
+  }
+  void realign() {
+    const unsigned long long grid = ftk::nway_grid(a, ftk::kRealignPerCta);
+    need(grid > 0 && a.shift[0] > 0 && a.shift[0] < 32);
+    for (unsigned long long cta = 0; cta < grid; ++cta)
+      for (unsigned t = 0; t < ftk::kRealignThreads; ++t) {
+        const unsigned lane = t & 31;
+        const unsigned long long i = cta * ftk::kRealignPerCta + t / 32 * 31 + lane;
+        if (i <= a.nvec)
+          for (int k = 0; k < a.n; ++k) read(k, src(k, (long long)(i * 32) - a.shift[0]), 32, 32);
+        if (lane < 31 && i < a.nvec) write(dst(i * 32), 32, 32);   // from this unit's sum and the next lane's: i + 1 <= nvec
+        if (a.edge && cta == grid - 1) edges(t, ftk::kRealignThreads);
+      }
+  }
+  void shift() {
+    const unsigned threads = ftk::shift_long(a) ? 64 : 128, unroll = ftk::shift_long(a) ? 2 : 1;
+    const unsigned long long grid = ftk::nway_grid(a, threads * unroll);
+    need(grid > 0);
+    for (unsigned long long cta = 0; cta < grid; ++cta)
+      for (unsigned t = 0; t < threads; ++t) {
+        for (unsigned u = 0; u < unroll; ++u) {
+          const unsigned long long i = cta * threads * unroll + u * threads + t;
+          for (int k = 0; k < a.n; ++k) {
+            const long long s = a.shift[k];
+            if (i < a.nvec || (s && i == a.nvec)) read(k, src(k, (long long)(i * 16) - s), 16, 16);
+            if (s && t % 32 == 31 && i < a.nvec) read(k, src(k, (long long)(i * 16 + 16) - s), 16, 16);
+          }
+          if (i < a.nvec) write(dst(i * 16), 16, 16);
+        }
+        if (a.edge && cta == grid - 1) edges(t, threads);
+      }
+  }
+  bool done() {
+    for (int k = 0; k < a.n; ++k)   // source and result are cut at the same element
+      need(((uintptr_t)a.src[k] - (uintptr_t)whole.src[k]) * os == ((uintptr_t)a.dst - (uintptr_t)whole.dst) * is);
+    for (uint8_t w : written) need(w == 1);
+    return good;
+  }
+};
+static int nway_kernel_seen[5];   // wide, realign, shift, scaled wide, scaled narrow
+static bool replay_nway(const ftk::NwayArgs& in, size_t unit, size_t len) {
+  NwayReplay r{in, in, unit, unit, len, std::vector<uint8_t>(len * unit)};
+  // the order of run_policy() in reduce_nway.cu
+  if (ftk::layout_wide(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[0]; r.wide(32, 32, 32); }
+  else if (ftk::layout_realign(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[1]; r.realign(); }
+  else { ++nway_kernel_seen[2]; ftk::layout_shift(in, len * unit, unit, &r.a); r.shift(); }
+  return r.done();
+}
+static bool replay_scaled(const ftk::NwayArgs& in, bool in_bf16, bool out_bf16, size_t len) {
+  const size_t is = in_bf16 ? 2 : 4, os = out_bf16 ? 2 : 4;
+  NwayReplay r{in, in, is, os, len, std::vector<uint8_t>(len * os)};
+  bool wide = false;
+  if (!ftk::layout_scaled(in, len, in_bf16, out_bf16, &r.a, &wide)) return true;   // an element at a time
+  ++nway_kernel_seen[wide ? 3 : 4];
+  r.wide(wide ? 32 : 16, 32 / is * os, wide && 32 / is * os >= 32 ? 32 : 16);
+  return r.done();
+}
+static void nway_layouts() {
+  const auto at = [](int vector, size_t offset) { return (void*)(((uintptr_t)(vector + 1) << 32) + offset); };
+  for (size_t unit : {1, 2, 4, 8}) {
+    const size_t offsets[] = {0, unit, 16 - unit, 16, 16 + unit, 32 - unit, 32, 96 + unit, 128 - unit};
+    std::vector<size_t> lens;
+    for (size_t bytes = unit; bytes <= 216; bytes += unit) lens.push_back(bytes / unit);
+    for (size_t edge : {2048, 3968, 4096, 7936, 8192})   // CTAs of the kernels, and the size from which a body starts on a line
+      for (long long off : {-40, -8, 0, 8, 40, 168}) lens.push_back((size_t)((long long)edge + off) / unit);
+    for (size_t d : offsets)
+      for (size_t s0 : offsets)
+        for (size_t s1 : offsets) {
+          ftk::NwayArgs in{};
+          in.n = 2;
+          in.dst = at(0, d); in.src[0] = at(1, s0); in.src[1] = at(2, s1);
+          for (size_t len : lens) EXPECT(replay_nway(in, unit, len));
+          if (unit != 2 && unit != 4) continue;
+          for (bool out_bf16 : {false, true})
+            if (d % (out_bf16 ? 2 : 4) == 0)
+              for (size_t len : lens) EXPECT(replay_scaled(in, unit == 2, out_bf16, len));
+        }
+    for (size_t bytes : {(3u << 20) - 40, 3u << 20, (3u << 20) + 56}) {   // where the shifted kernel changes its CTAs
+      ftk::NwayArgs in{};
+      in.n = 3;
+      in.dst = at(0, unit); in.src[0] = at(1, 0); in.src[1] = at(2, 24); in.src[2] = at(3, 16 - unit);
+      EXPECT(replay_nway(in, unit, bytes / unit));
+    }
+  }
+  for (int seen : nway_kernel_seen) EXPECT(seen > 1000);
+}
+
 int main(int argc, char** argv) {
   const bool threads = argc > 1 && !std::strcmp(argv[1], "threads");
-  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
+  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); nway_layouts(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
   thread_world(false);
   thread_world_phases();
   thread_world_small_message_twins();
