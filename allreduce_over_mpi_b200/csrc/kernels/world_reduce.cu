@@ -48,6 +48,7 @@ template <int POL, int V, int DEPTH, int G, int RANKS>
 __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __grid_constant__ WorldArgs<RANKS> a) {
   using P = typename PolById<POL>::type;
   static_assert(G <= kWorldGroup, "the parameters are filled for this many");
+  const void* const* out = a.ptr + a.kSteps;
   pdl_begin();
   const int first = a.entry[blockIdx.y].first, nsteps = a.entry[blockIdx.y].nsteps;
   const uint32_t mask = (uint32_t)a.entry[blockIdx.y].mask;
@@ -63,11 +64,11 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
   for (int k0 = 0; k0 < nsteps; k0 += G) {
     uint4 v[G][V];
 #pragma unroll
-    for (int g = 0; g < G; ++g) world_load<V>((const unsigned char*)a.src[first + k0 + g] + off, full && k0 + g < nsteps, v[g]);
+    for (int g = 0; g < G; ++g) world_load<V>((const unsigned char*)a.ptr[first + k0 + g] + off, full && k0 + g < nsteps, v[g]);
     if (!full) {
 #pragma unroll
       for (int g = 0; g < G; ++g)
-        if (k0 + g < nsteps) v[g][0] = ld_element((const unsigned char*)a.src[first + k0 + g] + off, a.es);
+        if (k0 + g < nsteps) v[g][0] = ld_element((const unsigned char*)a.ptr[first + k0 + g] + off, a.es);
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -95,8 +96,8 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
         for (int h = 0; h < V; ++h) w[h] = P::fin(acc[h]);
         const uint32_t to = a.store[first + k0 + g][r];
         if (to != kNoStore) {
-          if (full) world_store<V>((unsigned char*)a.out[to] + off, true, w);
-          else st_element((unsigned char*)a.out[to] + off, w[0], a.es);
+          if (full) world_store<V>((unsigned char*)out[to] + off, true, w);
+          else st_element((unsigned char*)out[to] + off, w[0], a.es);
         }
         const bool pop = r + 1 < rounds || (code & 2);
 #pragma unroll
@@ -117,10 +118,10 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
 #pragma unroll
   for (int h = 0; h < V; ++h) w[h] = a.entry[blockIdx.y].scaled ? P::fins(acc[h], a.scale) : P::fin(acc[h]);
 #pragma unroll
-  for (int r = 0; r < RANKS; ++r) world_store<V>((unsigned char*)a.out[r] + off, full && (mask >> r & 1), w);
+  for (int r = 0; r < RANKS; ++r) world_store<V>((unsigned char*)out[r] + off, full && (mask >> r & 1), w);
   if (!full)
     for (int r = 0; r < RANKS; ++r)
-      if (mask >> r & 1) st_element((unsigned char*)a.out[r] + off, w[0], a.es);
+      if (mask >> r & 1) st_element((unsigned char*)out[r] + off, w[0], a.es);
 }
 
 template <int POL, int V, int DEPTH, int G, int RANKS>

@@ -29,18 +29,21 @@ struct WorldProgram {
   std::vector<ftk::WorldStep> steps;         // entries[i] uses steps [first, first + nsteps)
 };
 
-// What the kernel gets of a program for the inputs of a call.  False: more than its parameters hold.
+// What the kernel gets of a program for the tensors of a call.  False: more than its parameters hold.
 template <int RANKS>
-bool fill_world_steps(const WorldProgram& wp, const void* const* in, ftk::WorldArgs<RANKS>* a) {
-  if (wp.entries.size() > (std::size_t)RANKS || wp.steps.size() > (std::size_t)RANKS * RANKS) return false;
+bool fill_world_args(const WorldProgram& wp, int world, const void* const* in, void* const* out, ftk::WorldArgs<RANKS>* a) {
+  constexpr std::size_t cap = ftk::WorldArgs<RANKS>::kSteps;
+  if (world > RANKS || wp.entries.size() > (std::size_t)RANKS || wp.steps.size() > cap) return false;
   std::copy(wp.entries.begin(), wp.entries.end(), a->entry);
-  for (std::size_t k = 0; k < wp.steps.size(); ++k) {
-    const ftk::WorldStep& s = wp.steps[k];
-    a->src[k] = in[s.rank];
+  std::size_t k = 0;
+  for (const ftk::WorldStep& s : wp.steps) {
+    a->ptr[k] = in[s.rank];
     a->code[k] = (uint8_t)(s.start | s.pop << 1 | s.rounds << 2);
     std::copy(s.store, s.store + ftk::kMaxRounds, a->store[k]);
+    ++k;
   }
-  std::fill_n(a->src + wp.steps.size(), ftk::kWorldGroup - 1, in[0]);
+  for (const std::size_t end = std::min(cap, k + ftk::kWorldGroup - 1); k < end; ++k) a->ptr[k] = in[0];
+  for (int r = 0; r < RANKS; ++r) a->ptr[cap + r] = r < world ? out[r] : nullptr;
   return true;
 }
 

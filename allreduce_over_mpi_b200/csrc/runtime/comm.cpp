@@ -498,11 +498,8 @@ cudaError_t world_launch(const ft::WorldProgram& wp, int pol, int world, const v
                                 uint64_t block_bytes, uint32_t es, float scale, cudaStream_t st) {
   ftk::WorldArgs<RANKS> a;
   uintptr_t all = block_bytes;
-  for (int r = 0; r < RANKS; ++r) {
-    a.out[r] = r < world ? out[r] : nullptr;
-    all |= r < world ? (uintptr_t)in[r] | (uintptr_t)out[r] : 0;
-  }
-  if (!ft::fill_world_steps(wp, in, &a)) return cudaErrorInvalidValue;   // (asked by the caller)
+  for (int r = 0; r < world; ++r) all |= (uintptr_t)in[r] | (uintptr_t)out[r];
+  if (!ft::fill_world_args(wp, world, in, out, &a)) return cudaErrorInvalidValue;   // (asked by the caller)
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
   a.es = es;

@@ -459,7 +459,7 @@ static void run_world_args(const ftk::WorldArgs<RANKS>& a, int entries, int dept
     float acc = 0;
     std::vector<float> aside(depth > 0 ? depth : 1, 0.f);
     for (int k = en.first; k < en.first + en.nsteps; ++k) {
-      const float v = ft::bf16_to_float({at(a.src[k], en.block)});
+      const float v = ft::bf16_to_float({at(a.ptr[k], en.block)});
       if (depth == 0) { acc = k == en.first ? v : acc + v; continue; }
       if (a.code[k] & 1) {
         aside.insert(aside.begin(), acc);
@@ -471,7 +471,7 @@ static void run_world_args(const ftk::WorldArgs<RANKS>& a, int entries, int dept
       const int rounds = a.code[k] >> 2;
       for (int r = 0; r < rounds; ++r) {
         const ft::bf16_t w = ft::float_to_bf16(acc);
-        if (a.store[k][r] != ftk::kNoStore) at(a.out[a.store[k][r]], en.block) = w.bits;
+        if (a.store[k][r] != ftk::kNoStore) at(a.ptr[a.kSteps + a.store[k][r]], en.block) = w.bits;
         acc = ft::bf16_to_float(w);
         if (r + 1 < rounds || (a.code[k] & 2)) {
           acc = aside[0] + acc;
@@ -481,22 +481,22 @@ static void run_world_args(const ftk::WorldArgs<RANKS>& a, int entries, int dept
       }
     }
     for (int r = 0; r < RANKS; ++r)
-      if (en.mask >> r & 1) at(a.out[r], en.block) = ft::float_to_bf16(acc).bits;
+      if (en.mask >> r & 1) at(a.ptr[a.kSteps + r], en.block) = ft::float_to_bf16(acc).bits;
   }
 }
 template <int RANKS>
 static bool world_program_as_plan(int n, const ft::Plan& p, ft::WorldPhase phase) {
   const ft::WorldProgram wp = ft::WorldProgramBuilder(n).run(p, phase);
   if (!wp.ok || wp.depth > (RANKS == 8 ? 2 : 3)) return false;
-  const void* in[RANKS];
+  void* in[RANKS];
   ftk::WorldArgs<RANKS> a;
   std::memset((void*)&a, 0xab, sizeof a);
-  for (int r = 0; r < RANKS; ++r) in[r] = a.out[r] = rank_copy + r;
-  if (!ft::fill_world_steps(wp, in, &a)) return false;
+  for (int r = 0; r < RANKS; ++r) in[r] = rank_copy + r;
+  if (!ft::fill_world_args(wp, n, in, in, &a)) return false;
   for (const ftk::WorldEntry& e : wp.entries)   // the kernel looks up whole groups of steps
-    for (int k = 0; k < (e.nsteps + ftk::kWorldGroup - 1) / ftk::kWorldGroup * ftk::kWorldGroup; ++k) {
-      EXPECT((const void* const*)&a.src[e.first + k] < (const void* const*)(&a.src + 1));
-      EXPECT(a.src[e.first + k] >= in[0] && a.src[e.first + k] <= in[n - 1]);
+    for (int k = e.first; k < e.first + (e.nsteps + ftk::kWorldGroup - 1) / ftk::kWorldGroup * ftk::kWorldGroup; ++k) {
+      EXPECT(k < a.kSteps + RANKS);
+      EXPECT((a.ptr[k] >= in[0] && a.ptr[k] <= in[n - 1]) || (k >= a.kSteps + n && !a.ptr[k]));
     }
   uint16_t got[ftk::kWorldRanks][ftk::kWorldRanks] = {}, want[ftk::kWorldRanks][ftk::kWorldRanks] = {};
   void* bufs[ftk::kWorldRanks];
