@@ -179,7 +179,8 @@ int ft_proc_allreduce(ft_proc_world* w, const int* widths, int nw, int lonely, i
 
 /* ---- single-GPU n-way reduction (reference: vector_add/reduce_sum_gpu.h) ---- */
 /* dst[i] = src[0][i] (op) ... (op) src[n-1][i], n in [1, FT_MAX_FANIN]; src/dst are device
- * pointers, `stream` a cudaStream_t.  variant: 0 auto, 1 vector loads, 2 TMA bulk pipeline.
+ * pointers, `stream` a cudaStream_t.  variant: 0 by alignment and size, in one launch;
+ * 1 8- or 16-byte vector loads; 2 TMA bulk pipeline; 11..24 and from 1000 up configurations for tuning.
  * Returns ft_status; CUDA launch errors map to FT_ERR_CUDA (see ft_last_cuda_error). */
 int ft_reduce_nway(int op, int dtype, const void* const* src, void* dst, int n, size_t len, int variant,
                    void* stream);

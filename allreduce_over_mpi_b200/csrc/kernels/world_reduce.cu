@@ -135,6 +135,9 @@ static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t
 }
 
 // No more loads in flight and values put aside than the program has: they cost registers, and those CTAs.
+// Integers have few programs worth a kernel of their own (one word a value, so the deepest form costs them nothing: eight
+// int32 buckets of 25 MB flat 63.8 us, 2*4 64.3, fp32 flat 63.6).  From nine ranks up every program runs the deepest form:
+// sixteen fp32 buckets flat 130 us (6.5 TB/s), 4*4 132, 2*2*2*2 141 (6.0 TB/s), in bf16 139, 151 and 166 us.
 template <int POL, int V, int RANKS>
 static cudaError_t launch_v(const WorldArgs<RANKS>& a, int entries, int depth, int steps, cudaStream_t st) {
   constexpr bool floats = POL == POL_F32 || POL == POL_BF16 || POL == POL_F16 || POL == POL_F64;

@@ -61,8 +61,9 @@ def reduce_nway(tensors: Sequence[torch.Tensor], op: str = "sum", out: torch.Ten
                 variant: int = 0, threads: int = 0) -> torch.Tensor:
     """Reduce ``tensors`` element-wise into ``out`` (allocated when omitted).
 
-    ``variant`` selects the device data path: 0/1 vector loads, 2 TMA bulk pipeline,
-    11..16 tuning configurations of the vector path (fp32 / bf16 only).
+    ``variant`` selects the device data path: 0 by the tensors' alignment and size, in one launch (256-bit accesses where
+    all of them lie at one offset from a 32-byte boundary); 1 8- or 16-byte vector loads, with a second launch for the
+    rest; 2 TMA bulk pipeline; 11..24 configurations of 1, and from 1000 up of 0, for tuning (some fan-ins in fp32 / bf16).
     """
     fast = (_lib._native or _lib.native()).reduce_nway(tensors, op, out, variant)
     if fast is not NotImplemented:

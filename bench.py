@@ -160,9 +160,9 @@ def bench_nway(a) -> dict:
 
 def e2e_nway(a, vecs, step_bytes) -> dict:
     """The same step end to end through the public API for operands in host memory
-    (``ops.HostReducePipeline``): every step copies the 8 input vectors from pinned host memory to the
-    device, reduces the four fan-ins and copies the four results back to pinned host memory.  The copies are
-    part of the timed region; the pipeline overlaps them chunk by chunk with each other and with the kernels."""
+    (``ops.HostReducePipeline``): every step brings the 8 input vectors from pinned host memory to the device, reduces
+    the four fan-ins and returns the four results to pinned host memory.  One kernel reads and writes them over PCIe,
+    both directions at once; all of it is part of the timed region."""
     import torch
     from allreduce_over_mpi_b200.ops import HostReducePipeline
     host_in = [torch.empty(v.shape, dtype=v.dtype).pin_memory() for v in vecs]
