@@ -13,10 +13,13 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <list>
 #include <map>
+#include <mutex>
 #include <vector>
 
 #include "../kernels/world_dev.h"
+#include "../runtime/dev_plan.hpp"
 #include "plan.hpp"
 
 namespace ft {
@@ -230,6 +233,52 @@ class WorldProgramBuilder {
   bool open_ = false;
   std::vector<Node> nodes_;
   std::map<std::pair<std::vector<int>, bool>, int> known_;
+};
+
+// What a call asks for: a plan, all copies summed in one order, or each block summed from its owner on.
+enum class WorldForm { plan, flat, rotated };
+
+// The programs of one world, each built by the first call that asks for it and kept: as many as shapes and phases in
+// use.  Calls may come from several threads.
+class WorldProgramCache {
+ public:
+  struct Entry {
+    WorldForm form;
+    WorldPhase phase;
+    Shape shape;
+    uint32_t nslots;   // receive slots of the plan's tagged-word form, whose limit holds for a call in one pass too
+    WorldProgram program;
+  };
+
+  // Null where there is no such plan, or none that runs in one pass; nothing is kept of those.
+  const Entry* get(int world, WorldForm form, WorldPhase phase, const int* widths, int nw, int lonely, bool ring) {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (const Entry& e : entries_)
+      if (e.form == form && e.phase == phase && e.shape.lonely == lonely && e.shape.ring == ring && (int)e.shape.widths.size() == nw &&
+          std::equal(e.shape.widths.begin(), e.shape.widths.end(), widths))
+        return &e;
+    Entry e{form, phase, Shape{std::vector<int>(widths, widths + nw), lonely, ring}, 0, {}};
+    WorldProgramBuilder builder(world);
+    if (form == WorldForm::plan) {
+      const Plan p = build_plan(world, nw > 0 ? e.shape : Shape::flat(world));
+      if (!p.ok()) return nullptr;
+      e.program = builder.run(p, phase);
+      e.nslots = build_dev_plan(p, 0).plan.nslots;
+    } else {
+      for (int b = 0; b < (form == WorldForm::rotated ? world : 1); ++b) builder.flat(b, b, &e.program);
+    }
+    if (!e.program.ok) return nullptr;
+    entries_.push_back(std::move(e));
+    return &entries_.back();
+  }
+  std::size_t size() {
+    std::lock_guard<std::mutex> lock(mu_);
+    return entries_.size();
+  }
+
+ private:
+  std::mutex mu_;
+  std::list<Entry> entries_;   // their addresses stay
 };
 
 }  // namespace ft

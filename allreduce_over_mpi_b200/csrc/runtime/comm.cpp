@@ -16,7 +16,6 @@
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
-#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -123,14 +122,6 @@ struct DevPlanEntry {
   uint32_t npulls = 0, npushes = 0;
 };
 
-// Program of a world on one device, as asked for (see ft_local_world_run).
-struct WorldProgramEntry {
-  int algo, phase, lonely, ring;
-  std::vector<int> widths;
-  uint32_t nslots;   // receive slots of the plan's tagged-word form, whose limit holds here too
-  ft::WorldProgram program;
-};
-
 }  // namespace
 
 struct ft_comm {
@@ -172,7 +163,7 @@ struct ft_comm {
   int phase_nvls = 1;         // ft_reduce_scatter / ft_all_gather through the multimem kernels (flat shape, eligible tensor):
                               // 0 never, 1 where it measured faster (five ranks and more), 2 whenever possible     // all-reduce: 0 = rank r owns block r, else round-robin stripes of this many bytes
   std::map<std::string, DevPlanEntry> plans;
-  std::list<WorldProgramEntry> world_programs;   // rank 0 of a world on one device; one per shape and phase in use
+  ft::WorldProgramCache world_programs;   // rank 0 of a world on one device
   // ft_allreduce_host: chunk buffers in the heap + three streams, made on first use
   struct HostPipe {
     static constexpr int kDepth = 3;
@@ -469,28 +460,6 @@ int launch_ll_call(ft_comm* c, const Prepared& pr, const void* sendbuf, void* re
   cudaError_t e = ftk::launch_ll(pr.pol, c->dev, a, st);
   if (e != cudaSuccess) return fail(c, FT_ERR_CUDA, std::string("low-latency launch: ") + cudaGetErrorString(e));
   return FT_OK;
-}
-
-const WorldProgramEntry* world_program(ft_comm* c, int algo, int phase, const int* widths, int nw, int lonely, int ring) {
-  for (const WorldProgramEntry& w : c->world_programs)
-    if (w.algo == algo && w.phase == phase && w.lonely == lonely && w.ring == ring && (int)w.widths.size() == nw &&
-        std::equal(w.widths.begin(), w.widths.end(), widths))
-      return &w;
-  WorldProgramEntry w{algo, phase, lonely, ring, std::vector<int>(widths, widths + nw), 0, {}};
-  ft::WorldProgramBuilder builder(c->world);
-  if (algo == FT_ALGO_PUSH) {
-    for (int b = 0; b < c->world; ++b) builder.flat(b, b, &w.program);
-  } else if (algo == FT_ALGO_ONESHOT || (algo == FT_ALGO_LL && nw == 0)) {
-    builder.flat(0, 0, &w.program);
-  } else {
-    const ft::Plan p = ft::build_plan(c->world, make_shape(c->world, widths, nw, lonely, ring));
-    if (p.ok()) {
-      w.program = builder.run(p, (ft::WorldPhase)phase);
-      w.nslots = ft::build_dev_plan(p, c->rank).plan.nslots;
-    }
-  }
-  c->world_programs.push_back(std::move(w));
-  return &c->world_programs.back();
 }
 
 template <int RANKS>
@@ -1180,7 +1149,7 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
 #ifdef FT_BOUNDS
   return FT_ERR_NOT_AVAILABLE;   // the checked build is there to run the kernels that check
 #endif
-  if (!comms || n < 2 || n > ftk::kWorldRanks || !in || !out || !count || phase < 0 || phase > 2) return FT_ERR_NOT_AVAILABLE;
+  if (!comms || n < 2 || n > ftk::kWorldRanks || !in || !out || !count || phase < 0 || phase > 2 || nw < 0 || (nw && !widths)) return FT_ERR_NOT_AVAILABLE;
   ft_comm* c = comms[0];
   if (!c || !c->finalized || c->world != n || op < 0 || op >= FT_OP_COUNT) return FT_ERR_NOT_AVAILABLE;
   const int pol = ftk::policy_id(op, dtype);
@@ -1213,11 +1182,14 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
     default: return FT_ERR_NOT_AVAILABLE;
   }
   if (phase != 0 && algo != FT_ALGO_STAGED) return FT_ERR_NOT_AVAILABLE;
-  const WorldProgramEntry* we = world_program(c, algo, phase, widths, nw, lonely, ring);
+  const ft::WorldForm form = tree ? ft::WorldForm::plan : algo == FT_ALGO_PUSH ? ft::WorldForm::rotated : ft::WorldForm::flat;
+  const ft::WorldProgramCache::Entry* we = tree ? c->world_programs.get(n, form, (ft::WorldPhase)phase, widths, nw, lonely, ring != 0)
+                                                : c->world_programs.get(n, form, ft::WorldPhase::all, nullptr, 0, 0, false);
+  if (!we) return FT_ERR_NOT_AVAILABLE;
   const ft::WorldProgram* wp = &we->program;
   if (algo == FT_ALGO_LL && nw > 0 && !ll_tree_fits(c, Prepared{pol, es, bytes, resident != 0}, count, we->nslots)) return FT_ERR_NOT_AVAILABLE;
   const int cap = n <= 8 ? 8 : ftk::kWorldRanks;
-  if (!wp->ok || wp->depth > (n <= 8 ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap) return FT_ERR_NOT_AVAILABLE;
+  if (wp->depth > (n <= 8 ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap) return FT_ERR_NOT_AVAILABLE;
   if (wp->entries.empty()) return FT_OK;
   const uint64_t block_bytes = blocks ? pick_block_elems(count, n, es) * es : (bytes + 15) / 16 * 16;
   // copies move raw words: 16-bit floats do not pass through fp32

@@ -524,6 +524,30 @@ static void world_programs() {
   EXPECT(shapes > 250 && taken == shapes);
 }
 
+// Threads that ask one world for programs at the same time get the same ones; shapes that are none leave nothing behind.
+static void world_program_cache() {
+  const int n = 12;
+  const std::vector<ft::Shape> shapes = ft::executable_shapes(n);
+  const ft::WorldPhase phases[] = {ft::WorldPhase::all, ft::WorldPhase::reduce_scatter, ft::WorldPhase::all_gather};
+  ft::WorldProgramCache cache;
+  std::vector<std::vector<const ft::WorldProgramCache::Entry*>> got(4);
+  std::vector<std::thread> th;
+  for (int t = 0; t < 4; ++t)
+    th.emplace_back([&, t] {
+      for (const ft::Shape& s : shapes)
+        for (ft::WorldPhase phase : phases)
+          got[t].push_back(cache.get(n, ft::WorldForm::plan, phase, s.widths.data(), (int)s.widths.size(), s.lonely, s.ring));
+      got[t].push_back(cache.get(n, ft::WorldForm::flat, ft::WorldPhase::all, nullptr, 0, 0, false));
+      got[t].push_back(cache.get(n, ft::WorldForm::rotated, ft::WorldPhase::all, nullptr, 0, 0, false));
+    });
+  for (auto& x : th) x.join();
+  for (int t = 0; t < 4; ++t) EXPECT(got[t] == got[0]);
+  for (const auto* e : got[0]) EXPECT(e && e->program.ok);
+  EXPECT(cache.size() == got[0].size());
+  const int wrong[] = {5, 2};
+  EXPECT(!cache.get(n, ft::WorldForm::plan, ft::WorldPhase::all, wrong, 2, 0, false) && cache.size() == got[0].size());
+}
+
 // Every access of every thread of the single-GPU reductions, for the way the host cuts the vectors: reads inside the
 // sources and on the boundaries the instructions need, each element of the result written once.
 struct NwayReplay {
@@ -655,6 +679,7 @@ static void nway_layouts() {
 int main(int argc, char** argv) {
   const bool threads = argc > 1 && !std::strcmp(argv[1], "threads");
   if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); nway_layouts(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
+  world_program_cache();
   thread_world(false);
   thread_world_phases();
   thread_world_small_message_twins();
