@@ -1,6 +1,8 @@
-// What the host hands to world_reduce_kernel (world_reduce.cu): one pass over the copies of all ranks of a world that
-// lives on one device.  Programs are built by planner/world_program.hpp.
+// What the host hands to the kernels that run one pass over the copies of all ranks of a world that lives on one device:
+// world_tree_kernel and world_copy_kernel (world_tree.cu) for floating sums and copies of up to eight ranks,
+// world_reduce_kernel (world_reduce.cu), which interprets its program, for the rest.  Programs are built by planner/world_program.hpp.
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 namespace ftk {
@@ -39,6 +41,62 @@ struct WorldArgs {
   uint32_t es;
   float scale;
   static_assert(RANKS >= kWorldGroup - 1, "a group that starts with the last step ends inside the table");
+};
+
+// ---- programs the tree kernel is compiled for -----------------------------------------------------------------------
+// A program's steps as one word: start | pop << 1 | rounds << 2 of step k in bits 4k .. 4k + 3.  As text: S starts, a
+// adds, r is a round, p a pop.
+constexpr int kTreeRanks = 8, kTreeRounds = 6;   // ranks, and rounds of one entry, of a program in this form
+constexpr uint32_t tree_code(const char* s) {
+  uint32_t code = 0;
+  for (int k = -1; *s; ++s) {
+    if (*s == 'S') code |= 1u << (4 * ++k);
+    else if (*s == 'a') ++k;
+    else if (*s == 'r') code += 4u << (4 * k);
+    else if (*s == 'p') code |= 2u << (4 * k);
+  }
+  return code;
+}
+// The shapes that the planner proposes for two to eight ranks: flat, trees of two or three levels, rings, and the trees
+// with lonely ranks (whose blocks follow two codes, by the group a lonely rank joins).
+struct WorldTree {
+  int ranks;
+  uint32_t code[2];   // in ascending order; the same twice where all blocks follow one
+};
+constexpr WorldTree tree(int ranks, const char* a, const char* b = nullptr) {
+  const uint32_t x = tree_code(a), y = b ? tree_code(b) : x;
+  return x < y ? WorldTree{ranks, {x, y}} : WorldTree{ranks, {y, x}};
+}
+constexpr WorldTree kWorldTrees[] = {
+    tree(2, "S a"), tree(3, "S a a"), tree(4, "S a a a"), tree(5, "S a a a a"), tree(6, "S a a a a a"), tree(7, "S a a a a a a"),
+    tree(8, "S a a a a a a a"),
+    tree(4, "S ar S arp"),                                        // 2*2
+    tree(6, "S ar S arp S arp"), tree(6, "S a ar S a arp"),       // 2*3, 3*2
+    tree(8, "S ar S arp S arp S arp"), tree(8, "S a a ar S a a arp"), tree(8, "S ar S arr S ar S arrp"),   // 2*4, 4*2, 2*2*2
+    tree(3, "S ar a"), tree(4, "S ar ar a"), tree(5, "S ar ar ar a"), tree(6, "S ar ar ar ar a"), tree(7, "S ar ar ar ar ar a"),
+    tree(8, "S ar ar ar ar ar ar a"),                             // rings
+    tree(5, "S a ar S arp", "S ar S a arp"),                      // 2*2+1
+    tree(7, "S a ar S arp S arp", "S ar S a arp S arp"),          // 2*3+1
+    tree(7, "S a a ar S a arp", "S a ar S a a arp"),              // 3*2+1
+    tree(8, "S a ar S a arp S arp", "S ar S a arp S a arp"),      // 2*3+2
+};
+constexpr int kFlatTrees = kTreeRanks - 1;   // the first ones: 2 .. 8 ranks in one sum
+constexpr int kWorldTreeCount = sizeof kWorldTrees / sizeof kWorldTrees[0];
+
+// One block's program beside its code: the rank of step k in bits 3k .. 3k + 2, the ranks that get the result in bits
+// 24 .. 31, the block in 32 .. 34, which of the two codes in 35, and from 36 on four bits a round: the rank whose copy ends
+// there, or 15.
+constexpr int kTreeMask = 24, kTreeBlock = 32, kTreeWhich = 35, kTreeStore = 36;
+
+// 216 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
+// cache after the other.
+struct WorldTreeArgs {
+  uint64_t entry[kTreeRanks];
+  const void* in[kTreeRanks];
+  void* out[kTreeRanks];
+  uint64_t total_bytes, block_bytes;
+  uint32_t es;
+  float scale;
 };
 
 }  // namespace ftk

@@ -134,51 +134,42 @@ static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t
   return launch_pdl(world_reduce_kernel<POL, V, DEPTH, G, RANKS>, dim3((unsigned)per, (unsigned)entries), kWorldThreads, 0, st, a);
 }
 
-// No more loads in flight and values put aside than the program has: they cost registers, and those CTAs.
-// Integers have few programs worth a kernel of their own (one word a value, so the deepest form costs them nothing: eight
-// int32 buckets of 25 MB flat 63.8 us, 2*4 64.3, fp32 flat 63.6).  From nine ranks up every program runs the deepest form:
-// sixteen fp32 buckets flat 130 us (6.5 TB/s), 4*4 132, 2*2*2*2 141 (6.0 TB/s), in bf16 139, 151 and 166 us.
-template <int POL, int V, int RANKS>
-static cudaError_t launch_v(const WorldArgs<RANKS>& a, int entries, int depth, int steps, cudaStream_t st) {
-  constexpr bool floats = POL == POL_F32 || POL == POL_BF16 || POL == POL_F16 || POL == POL_F64;
-  if constexpr (RANKS > 8) {
-    return launch_t<POL, V, 3, 8, RANKS>(a, entries, st);
-  } else {
-    if constexpr (POL == POL_OR)
-      if (steps == 1) return launch_t<POL, V, 0, 1, RANKS>(a, entries, st);
-    if constexpr (floats) {
-      if (depth == 0) return steps <= 4 ? launch_t<POL, V, 0, 4, RANKS>(a, entries, st) : launch_t<POL, V, 0, 8, RANKS>(a, entries, st);
-      if (depth == 1) return steps <= 4 ? launch_t<POL, V, 1, 4, RANKS>(a, entries, st) : launch_t<POL, V, 1, 8, RANKS>(a, entries, st);
-    }
-    // two values put aside: 32 bytes of 16-bit floats are 16 accumulators each and spill (2*2*2 over eight bf16 buckets of
-    // 25 MB 74.8 us, 70.1 with 16 bytes a thread; fp32 65.1 us with 16 and 64.3 with 32)
-    return launch_t<POL, POL == POL_BF16 || POL == POL_F16 ? 1 : V, 2, 8, RANKS>(a, entries, st);
-  }
-}
+// Of integers of up to eight ranks only the reduce-scatters of trees come here (one word a value, so the deepest form costs
+// nothing: eight int32 buckets of 25 MB flat 63.8 us, 2*4 64.3).  From nine ranks up, and for a floating sum of fewer
+// whose program is not compiled in, every program runs the deepest form: sixteen fp32 buckets flat 130 us (6.5 TB/s), 4*4
+// 132, 2*2*2*2 141 (6.0 TB/s), in bf16 139, 151 and 166 us.
 template <int POL, int RANKS>
-static cudaError_t launch_r(const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st) {
-  if constexpr (RANKS <= 8)
-    if (wide) return launch_v<POL, 2>(a, entries, depth, steps, st);
-  return launch_v<POL, 1>(a, entries, depth, steps, st);
+static cudaError_t launch_r(const WorldArgs<RANKS>& a, int entries, bool wide, cudaStream_t st) {
+  if constexpr (RANKS <= 8) {
+    return wide ? launch_t<POL, 2, 2, 8, RANKS>(a, entries, st) : launch_t<POL, 1, 2, 8, RANKS>(a, entries, st);
+  } else {
+    return launch_t<POL, 1, 3, 8, RANKS>(a, entries, st);
+  }
 }
 
 template <int RANKS>
-cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st) {
+cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, bool wide, cudaStream_t st) {
   switch (pol) {
-    case POL_ADD8: return launch_r<POL_ADD8>(a, entries, depth, steps, wide, st);
-    case POL_ADD16: return launch_r<POL_ADD16>(a, entries, depth, steps, wide, st);
-    case POL_ADD32: return launch_r<POL_ADD32>(a, entries, depth, steps, wide, st);
-    case POL_ADD64: return launch_r<POL_ADD64>(a, entries, depth, steps, wide, st);
-    case POL_OR: return launch_r<POL_OR>(a, entries, depth, steps, wide, st);
-    case POL_AND: return launch_r<POL_AND>(a, entries, depth, steps, wide, st);
-    case POL_F32: return launch_r<POL_F32>(a, entries, depth, steps, wide, st);
-    case POL_F64: return launch_r<POL_F64>(a, entries, depth, steps, wide, st);
-    case POL_BF16: return launch_r<POL_BF16>(a, entries, depth, steps, wide, st);
-    case POL_F16: return launch_r<POL_F16>(a, entries, depth, steps, wide, st);
-    default: return cudaErrorInvalidValue;
+    case POL_ADD8: return launch_r<POL_ADD8>(a, entries, wide, st);
+    case POL_ADD16: return launch_r<POL_ADD16>(a, entries, wide, st);
+    case POL_ADD32: return launch_r<POL_ADD32>(a, entries, wide, st);
+    case POL_ADD64: return launch_r<POL_ADD64>(a, entries, wide, st);
+    case POL_OR: return launch_r<POL_OR>(a, entries, wide, st);
+    case POL_AND: return launch_r<POL_AND>(a, entries, wide, st);
+    default: break;
   }
+  if constexpr (RANKS > 8) {
+    switch (pol) {
+      case POL_F32: return launch_r<POL_F32>(a, entries, wide, st);
+      case POL_F64: return launch_r<POL_F64>(a, entries, wide, st);
+      case POL_BF16: return launch_r<POL_BF16>(a, entries, wide, st);
+      case POL_F16: return launch_r<POL_F16>(a, entries, wide, st);
+      default: break;
+    }
+  }
+  return cudaErrorInvalidValue;
 }
-template cudaError_t launch_world<8>(int, const WorldArgs<8>&, int, int, int, bool, cudaStream_t);
-template cudaError_t launch_world<16>(int, const WorldArgs<16>&, int, int, int, bool, cudaStream_t);
+template cudaError_t launch_world<8>(int, const WorldArgs<8>&, int, bool, cudaStream_t);
+template cudaError_t launch_world<16>(int, const WorldArgs<16>&, int, bool, cudaStream_t);
 
 }  // namespace ftk

@@ -27,10 +27,68 @@ namespace ft {
 struct WorldProgram {
   bool ok = false;
   int depth = 0;                             // 0: plain sums; else the accumulators put aside at the same time, at least 1
-  int widest = 0;                            // steps of the longest entry
   std::vector<ftk::WorldEntry> entries;      // one per block and pass over it
   std::vector<ftk::WorldStep> steps;         // entries[i] uses steps [first, first + nsteps)
+  // The same for the kernels with programs compiled in, where there is one for this program (compact_world_program).
+  int tree = -1;                             // index into kWorldTrees
+  bool copies = false;                       // every entry is one step: copies only
+  bool partial = false;                      // some copy ends as a part of the sum
+  std::vector<uint64_t> words;               // WorldTreeArgs::entry
 };
+
+// Finds the compiled form of a finished program: all entries take every rank's copy once and follow one or two codes of
+// kWorldTrees, or are copies.  Leaves tree = -1 and copies = false where there is none.
+inline void compact_world_program(int world, WorldProgram* wp) {
+  if (!wp->ok || world > ftk::kTreeRanks || wp->entries.empty() || wp->entries.size() > (std::size_t)ftk::kTreeRanks) return;
+  std::vector<uint32_t> codes;
+  std::vector<uint64_t> words;
+  bool copies = true, whole = true, partial = false;
+  for (const ftk::WorldEntry& e : wp->entries) {
+    uint64_t word = (uint64_t)(e.mask & 0xff) << ftk::kTreeMask | (uint64_t)e.block << ftk::kTreeBlock;
+    uint32_t code = 0;
+    int rounds = 0;
+    copies = copies && e.nsteps == 1 && !e.scaled && wp->steps[e.first].rounds == 0;
+    whole = whole && e.nsteps == world && e.scaled;
+    if (e.nsteps > ftk::kTreeRanks || e.block >= ftk::kTreeRanks) return;
+    for (int k = 0; k < e.nsteps; ++k) {
+      const ftk::WorldStep& s = wp->steps[e.first + k];
+      if (s.rounds > 3 || rounds + s.rounds > ftk::kTreeRounds) return;
+      word |= (uint64_t)s.rank << (3 * k);
+      code |= (uint32_t)(s.start | s.pop << 1 | s.rounds << 2) << (4 * k);
+      for (int r = 0; r < s.rounds; ++r) {
+        partial = partial || s.store[r] != ftk::kNoStore;
+        word |= (uint64_t)(s.store[r] == ftk::kNoStore ? 15 : s.store[r]) << (ftk::kTreeStore + 4 * rounds++);
+      }
+    }
+    words.push_back(word);
+    codes.push_back(code);
+  }
+  if (copies) {
+    wp->copies = true;
+    wp->words = words;
+    return;
+  }
+  const uint32_t lo = *std::min_element(codes.begin(), codes.end()), hi = *std::max_element(codes.begin(), codes.end());
+  for (std::size_t i = 0; i < codes.size(); ++i) {
+    if (codes[i] != lo && codes[i] != hi) return;
+    if (codes[i] != lo) words[i] |= 1ull << ftk::kTreeWhich;
+  }
+  for (int t = 0; whole && t < ftk::kWorldTreeCount; ++t)
+    if (ftk::kWorldTrees[t].ranks == world && ftk::kWorldTrees[t].code[0] == lo && ftk::kWorldTrees[t].code[1] == hi) {
+      wp->tree = t;
+      wp->partial = partial;
+      wp->words = words;
+    }
+}
+
+// What the tree and copy kernels get of it for the tensors of a call.
+inline void fill_tree_args(const WorldProgram& wp, int world, const void* const* in, void* const* out, ftk::WorldTreeArgs* a) {
+  for (int r = 0; r < ftk::kTreeRanks; ++r) {
+    a->entry[r] = r < (int)wp.words.size() ? wp.words[r] : 0;
+    a->in[r] = r < world ? in[r] : nullptr;
+    a->out[r] = r < world ? out[r] : nullptr;
+  }
+}
 
 // What the kernel gets of a program for the tensors of a call.  False: more than its parameters hold.
 template <int RANKS>
@@ -102,7 +160,6 @@ class WorldProgramBuilder {
     bool scaled;             // made in the stage that finishes the reduction
   };
   static void add(const ftk::WorldEntry& e, WorldProgram* out) {
-    if (e.nsteps > out->widest) out->widest = e.nsteps;
     out->entries.push_back(e);
   }
   uint64_t everyone() const { return world_ >= 64 ? ~0ull : (1ull << world_) - 1; }
@@ -268,6 +325,7 @@ class WorldProgramCache {
       for (int b = 0; b < (form == WorldForm::rotated ? world : 1); ++b) builder.flat(b, b, &e.program);
     }
     if (!e.program.ok) return nullptr;
+    compact_world_program(world, &e.program);
     entries_.push_back(std::move(e));
     return &entries_.back();
   }

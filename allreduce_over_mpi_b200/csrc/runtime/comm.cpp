@@ -45,7 +45,9 @@ cudaError_t launch_hybrid(int pol, const CommDev& c, const NvlsArgs& a, int lane
 cudaError_t launch_ll_tree(int pol, const CommDev& c, const LLTreeArgs& a, cudaStream_t st);
 cudaError_t launch_nvls_oneshot(int pol, const CommDev& c, const OneShotArgs& a, uint64_t slot_bytes, int lanes, int threads, cudaStream_t st);
 template <int RANKS>
-cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, int depth, int steps, bool wide, cudaStream_t st);
+cudaError_t launch_world(int pol, const WorldArgs<RANKS>& a, int entries, bool wide, cudaStream_t st);
+cudaError_t launch_world_tree(int pol, const WorldTreeArgs& a, int tree, int entries, bool wide, cudaStream_t st);
+cudaError_t launch_world_copy(const WorldTreeArgs& a, int entries, bool wide, cudaStream_t st);
 cudaError_t launch_wait_probe(const CommDev& c, int peer, unsigned long long timeout_ns, cudaStream_t st);
 }  // namespace ftk
 
@@ -462,20 +464,44 @@ int launch_ll_call(ft_comm* c, const Prepared& pr, const void* sendbuf, void* re
   return FT_OK;
 }
 
+// 32 bytes per thread where every copy and block starts on such a boundary and that leaves every SM a few CTAs; below,
+// twice the threads hide more of the latency.
+bool world_wide(int world, const void* const* in, void* const* out, uint64_t bytes, uint64_t block_bytes) {
+  uintptr_t all = block_bytes;
+  for (int r = 0; r < world; ++r) all |= (uintptr_t)in[r] | (uintptr_t)out[r];
+  return all % 32 == 0 && bytes >= (2u << 20);
+}
+
 template <int RANKS>
 cudaError_t world_launch(const ft::WorldProgram& wp, int pol, int world, const void* const* in, void* const* out, uint64_t bytes,
                                 uint64_t block_bytes, uint32_t es, float scale, cudaStream_t st) {
   ftk::WorldArgs<RANKS> a;
-  uintptr_t all = block_bytes;
-  for (int r = 0; r < world; ++r) all |= (uintptr_t)in[r] | (uintptr_t)out[r];
   if (!ft::fill_world_args(wp, world, in, out, &a)) return cudaErrorInvalidValue;   // (asked by the caller)
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
   a.es = es;
   a.scale = scale;
-  // 32 bytes per thread once that leaves every SM a few CTAs; below, twice the threads hide more of the latency
-  const bool wide = all % 32 == 0 && bytes >= (2u << 20);
-  return ftk::launch_world<RANKS>(pol, a, (int)wp.entries.size(), wp.depth, wp.widest, wide, st);
+  const bool wide = world_wide(world, in, out, bytes, block_bytes);
+  return ftk::launch_world<RANKS>(pol, a, (int)wp.entries.size(), wide, st);
+}
+
+bool is_floating(int pol) { return pol == ftk::POL_F32 || pol == ftk::POL_F64 || pol == ftk::POL_BF16 || pol == ftk::POL_F16; }
+// The compiled form of a program, or -1.  An integer sum is the same whatever the plan's order: where only whole sums are
+// stored, integers take the flat form.
+int compiled_tree(const ft::WorldProgram& wp, int world, int pol) {
+  return wp.tree < 0 || is_floating(pol) ? wp.tree : wp.partial ? -1 : world - 2;
+}
+cudaError_t tree_launch(const ft::WorldProgram& wp, int pol, int world, const void* const* in, void* const* out, uint64_t bytes,
+                        uint64_t block_bytes, uint32_t es, float scale, cudaStream_t st) {
+  ftk::WorldTreeArgs a;
+  ft::fill_tree_args(wp, world, in, out, &a);
+  a.total_bytes = bytes;
+  a.block_bytes = block_bytes;
+  a.es = es;
+  a.scale = scale;
+  const bool wide = world_wide(world, in, out, bytes, block_bytes);
+  return wp.copies ? ftk::launch_world_copy(a, (int)wp.words.size(), wide, st)
+                   : ftk::launch_world_tree(pol, a, compiled_tree(wp, world, pol), (int)wp.words.size(), wide, st);
 }
 
 }  // namespace
@@ -1188,13 +1214,16 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
   if (!we) return FT_ERR_NOT_AVAILABLE;
   const ft::WorldProgram* wp = &we->program;
   if (algo == FT_ALGO_LL && nw > 0 && !ll_tree_fits(c, Prepared{pol, es, bytes, resident != 0}, count, we->nslots)) return FT_ERR_NOT_AVAILABLE;
-  const int cap = n <= 8 ? 8 : ftk::kWorldRanks;
-  if (wp->depth > (n <= 8 ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap) return FT_ERR_NOT_AVAILABLE;
+  // the kernels with programs compiled in where there is one; of the rest, small worlds' integers by the smaller parameters
+  const bool compiled = wp->copies || compiled_tree(*wp, n, pol) >= 0, small = n <= 8 && !is_floating(pol);
+  const int cap = small ? 8 : ftk::kWorldRanks;
+  if (!compiled && (wp->depth > (small ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap)) return FT_ERR_NOT_AVAILABLE;
   if (wp->entries.empty()) return FT_OK;
   const uint64_t block_bytes = blocks ? pick_block_elems(count, n, es) * es : (bytes + 15) / 16 * 16;
   // copies move raw words: 16-bit floats do not pass through fp32
   const int kernel_pol = phase == 2 ? (int)ftk::POL_OR : pol;
-  const cudaError_t e = n <= 8 ? world_launch<8>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
+  const cudaError_t e = compiled ? tree_launch(*wp, pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
+                        : small ? world_launch<8>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
                                : world_launch<16>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream);
   return e == cudaSuccess ? FT_OK : fail(c, FT_ERR_CUDA, std::string("world launch: ") + cudaGetErrorString(e));
 }

@@ -484,11 +484,50 @@ static void run_world_args(const ftk::WorldArgs<RANKS>& a, int entries, int dept
       if (en.mask >> r & 1) at(a.ptr[a.kSteps + r], en.block) = ft::float_to_bf16(acc).bits;
   }
 }
+// The same for the programs that are compiled in: world_tree_kernel's and world_copy_kernel's reading of their parameters.
+static void run_tree_args(const ftk::WorldTreeArgs& a, int entries, int tree, uint16_t (*copy)[ftk::kWorldRanks]) {
+  const auto at = [&](const void* rank, int block) -> uint16_t& { return copy[(const char*)rank - rank_copy][block]; };
+  for (int e = 0; e < entries; ++e) {
+    const uint64_t word = a.entry[e];
+    const int block = (int)(word >> ftk::kTreeBlock) & 7, n = tree < 0 ? 1 : ftk::kWorldTrees[tree].ranks;
+    const uint32_t code = tree < 0 ? 1 : ftk::kWorldTrees[tree].code[word >> ftk::kTreeWhich & 1];
+    float v[ftk::kTreeRanks], acc = 0;
+    for (int k = 0; k < n; ++k) v[k] = ft::bf16_to_float({at(a.in[word >> (3 * k) & 7], block)});
+    std::vector<float> aside;
+    for (int k = 0, t = 0; k < n; ++k) {
+      if (code >> (4 * k) & 1) {
+        if (k) aside.push_back(acc);
+        acc = v[k];
+      } else {
+        acc += v[k];
+      }
+      EXPECT(aside.size() <= 2);
+      const int rounds = (int)(code >> (4 * k) & 15) >> 2;
+      for (int r = 0; r < rounds; ++r) {
+        const ft::bf16_t w = ft::float_to_bf16(acc);
+        EXPECT(t < ftk::kTreeRounds);
+        const int to = (int)(word >> (ftk::kTreeStore + 4 * t++)) & 15;
+        if (to != 15) at(a.out[to], block) = w.bits;
+        acc = ft::bf16_to_float(w);
+        if (r + 1 < rounds || (code >> (4 * k) & 2)) {
+          acc = aside.back() + acc;
+          aside.pop_back();
+        }
+      }
+    }
+    EXPECT(aside.empty());
+    for (int r = 0; r < ftk::kTreeRanks; ++r)
+      if (word >> (ftk::kTreeMask + r) & 1) at(a.out[r], block) = ft::float_to_bf16(acc).bits;
+  }
+}
+static int compiled_programs[ftk::kWorldTreeCount], uncompiled_programs;
+
 template <int RANKS>
 static bool world_program_as_plan(int n, const ft::Plan& p, ft::WorldPhase phase) {
-  const ft::WorldProgram wp = ft::WorldProgramBuilder(n).run(p, phase);
+  ft::WorldProgram wp = ft::WorldProgramBuilder(n).run(p, phase);
+  ft::compact_world_program(n, &wp);
   if (!wp.ok || wp.depth > (RANKS == 8 ? 2 : 3)) return false;
-  void* in[RANKS];
+  void* in[ftk::kWorldRanks];
   ftk::WorldArgs<RANKS> a;
   std::memset((void*)&a, 0xab, sizeof a);
   for (int r = 0; r < RANKS; ++r) in[r] = rank_copy + r;
@@ -507,6 +546,18 @@ static bool world_program_as_plan(int n, const ft::Plan& p, ft::WorldPhase phase
   const int half = p.num_stages / 2;
   EXPECT(ft::run_plan_snapshot(p, FT_SUM, FT_BF16, bufs, n, 1, phase == ft::WorldPhase::all_gather ? half : 0,
                                phase == ft::WorldPhase::reduce_scatter ? half : -1) == FT_OK);
+  if (wp.tree >= 0 || wp.copies) {
+    uint16_t compact[ftk::kWorldRanks][ftk::kWorldRanks];
+    std::memcpy(compact, got, sizeof got);
+    ftk::WorldTreeArgs t;
+    ft::fill_tree_args(wp, n, in, in, &t);
+    EXPECT(wp.copies == (phase == ft::WorldPhase::all_gather) && wp.words.size() == wp.entries.size());
+    run_tree_args(t, (int)wp.words.size(), wp.copies ? -1 : wp.tree, compact);
+    EXPECT(!std::memcmp(compact, want, sizeof compact));
+    if (!wp.copies) ++compiled_programs[wp.tree];
+  } else if (n <= ftk::kTreeRanks) {
+    ++uncompiled_programs;
+  }
   run_world_args(a, (int)wp.entries.size(), wp.depth, got);
   EXPECT(!std::memcmp(got, want, sizeof got));
   return true;
@@ -518,10 +569,12 @@ static void world_programs() {
       const ft::Plan p = ft::build_plan(n, s);
       for (ft::WorldPhase phase : {ft::WorldPhase::all, ft::WorldPhase::reduce_scatter, ft::WorldPhase::all_gather}) {
         ++shapes;
-        taken += n <= 8 ? world_program_as_plan<8>(n, p, phase) : world_program_as_plan<16>(n, p, phase);
+        taken += world_program_as_plan<16>(n, p, phase) && (n > 8 || world_program_as_plan<8>(n, p, phase));
       }
     }
   EXPECT(shapes > 250 && taken == shapes);
+  for (int c : compiled_programs) EXPECT(c >= 2);   // every compiled program is some shape's, as a whole and as a reduce-scatter
+  EXPECT(uncompiled_programs == 0);
 }
 
 // Threads that ask one world for programs at the same time get the same ones; shapes that are none leave nothing behind.
