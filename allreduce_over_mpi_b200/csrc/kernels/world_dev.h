@@ -88,7 +88,7 @@ constexpr int kWorldTreeCount = sizeof kWorldTrees / sizeof kWorldTrees[0];
 // there, or 15.
 constexpr int kTreeMask = 24, kTreeBlock = 32, kTreeWhich = 35, kTreeStore = 36;
 
-// 216 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
+// 224 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
 // cache after the other.
 struct WorldTreeArgs {
   uint64_t entry[kTreeRanks];
@@ -97,6 +97,7 @@ struct WorldTreeArgs {
   uint64_t total_bytes, block_bytes;
   uint32_t es;
   float scale;
+  uint32_t streams;   // what is read, and copies that are written, leave L2 before other data
 };
 
 }  // namespace ftk

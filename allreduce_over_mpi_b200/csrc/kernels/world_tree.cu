@@ -24,14 +24,21 @@ namespace ftk {
 constexpr int kTreeThreads = 128;
 constexpr bool floating(int pol) { return pol == POL_F32 || pol == POL_F64 || pol == POL_BF16 || pol == POL_F16; }
 
+// L2's choice of what leaves first, for accesses of 32 bytes (narrower ones have none): before the rest, or as usual.
+__device__ __forceinline__ uint64_t l2_policy(bool first) {
+  uint64_t normal, early;
+  asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(early));
+  return first ? early : normal;
+}
 // Predicated accesses (no branch, so that all of them are issued back to back): V 16-byte vectors at p.
 template <int V>
-__device__ __forceinline__ void tree_load(const unsigned char* p, bool ok, uint4 (&v)[V]) {
+__device__ __forceinline__ void tree_load(const unsigned char* p, bool ok, uint4 (&v)[V], uint64_t policy) {
   if constexpr (V == 2)
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %9, 0;\n\t"
-                 "@q ld.global.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t}"
+                 "@q ld.global.L1::no_allocate.L2::cache_hint.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %10;\n\t}"
                  : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w)
-                 : "l"(p), "r"((uint32_t)ok) : "memory");
+                 : "l"(p), "r"((uint32_t)ok), "l"(policy) : "memory");
   else
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
                  "@q ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
@@ -46,6 +53,16 @@ __device__ __forceinline__ void tree_store(unsigned char* p, bool ok, const uint
   else
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q st.global.v4.u32 [%0], {%1,%2,%3,%4};\n\t}"
                  ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"((uint32_t)ok) : "memory");
+}
+template <int V>
+__device__ __forceinline__ void tree_store(unsigned char* p, bool ok, const uint4 (&v)[V], uint64_t policy) {
+  if constexpr (V == 2)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %9, 0;\n\t"
+                 "@q st.global.L2::cache_hint.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8}, %10;\n\t}"
+                 ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
+                   "r"((uint32_t)ok), "l"(policy) : "memory");
+  else
+    tree_store<V>(p, ok, v);
 }
 
 // Where a thread works: whole vectors of V x 16 bytes first, then the elements behind the last one, a thread each.
@@ -134,8 +151,9 @@ __global__ void __launch_bounds__(kTreeThreads, 4) world_tree_kernel(const __gri
   pdl_begin();
   if (!at.any) return;
   uint4 v[N][V];
+  const uint64_t policy = l2_policy(a.streams);
 #pragma unroll
-  for (int k = 0; k < N; ++k) tree_load<V>(src[k], at.full, v[k]);
+  for (int k = 0; k < N; ++k) tree_load<V>(src[k], at.full, v[k], policy);
   if (!at.full) {
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k][0] = ld_element(src[k], ES);
@@ -173,11 +191,12 @@ __global__ void __launch_bounds__(kTreeThreads) world_copy_kernel(const __grid_c
   pdl_begin();
   if (!at.any) return;
   uint4 v[V];
-  tree_load<V>(src, at.full, v);
+  const uint64_t policy = l2_policy(a.streams);
+  tree_load<V>(src, at.full, v, policy);
   if (!at.full) v[0] = ld_element(src, a.es);
   const uint32_t mask = lo >> kTreeMask;
 #pragma unroll
-  for (int r = 0; r < kTreeRanks; ++r) tree_store<V>((unsigned char*)a.out[r] + at.off, at.full && (mask >> r & 1), v);
+  for (int r = 0; r < kTreeRanks; ++r) tree_store<V>((unsigned char*)a.out[r] + at.off, at.full && (mask >> r & 1), v, policy);
   if (!at.full)
     for (int r = 0; r < kTreeRanks; ++r)
       if (mask >> r & 1) st_element((unsigned char*)a.out[r] + at.off, v[0], a.es);

@@ -492,9 +492,15 @@ int compiled_tree(const ft::WorldProgram& wp, int world, int pol) {
   return wp.tree < 0 || is_floating(pol) ? wp.tree : wp.partial ? -1 : world - 2;
 }
 cudaError_t tree_launch(const ft::WorldProgram& wp, int pol, int world, const void* const* in, void* const* out, uint64_t bytes,
-                        uint64_t block_bytes, uint32_t es, float scale, cudaStream_t st) {
+                        uint64_t block_bytes, uint32_t es, float scale, int phase, cudaStream_t st) {
   ftk::WorldTreeArgs a;
   ft::fill_tree_args(wp, world, in, out, &a);
+  // The halves of an all-reduce: what the reduce-scatter leaves is what the all-gather reads, everything else either of them
+  // touches has served.  Both calls, fp32 25 MB a rank, us, three sets of tensors in turn (twelve, so that nothing is left
+  // from the time before): flat of eight 71.7 (71.7) -> 65.2 (66.2), 2*4 80.7 (80.7) -> 75.3 (75.3), flat of four 35.6 (35.6)
+  // -> 32.8 (34.5), of two 18.9 (19.0) -> 17.0 (19.2).  Worth saying only where a world's copies take a good part of L2 (126
+  // MB): four of 6 MB, three sets of which stay there, took 7.6 instead of 7.0.  An all-reduce has nothing to keep: 63.2 -> 63.6.
+  a.streams = phase != 0 && bytes * world >= (32u << 20);
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
   a.es = es;
@@ -1222,7 +1228,7 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
   const uint64_t block_bytes = blocks ? pick_block_elems(count, n, es) * es : (bytes + 15) / 16 * 16;
   // copies move raw words: 16-bit floats do not pass through fp32
   const int kernel_pol = phase == 2 ? (int)ftk::POL_OR : pol;
-  const cudaError_t e = compiled ? tree_launch(*wp, pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
+  const cudaError_t e = compiled ? tree_launch(*wp, pol, n, in, out, bytes, block_bytes, es, scale, phase, (cudaStream_t)stream)
                         : small ? world_launch<8>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream)
                                : world_launch<16>(*wp, kernel_pol, n, in, out, bytes, block_bytes, es, scale, (cudaStream_t)stream);
   return e == cudaSuccess ? FT_OK : fail(c, FT_ERR_CUDA, std::string("world launch: ") + cudaGetErrorString(e));

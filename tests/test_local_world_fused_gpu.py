@@ -80,10 +80,11 @@ def test_every_shape_same_bits(text, dtype):
 @pytest.mark.parametrize("text", ["2", "3", "5", "7", "2*2", "3*2", "4*2", "2*2*2", "ring3", "ring6", "2*2+1", "3*2+1", "2*3+2"])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float64, torch.int64, torch.uint8])
 def test_compiled_programs_same_bits(text, dtype):
-    """Types with a dispatch of their own, around an empty block, a lone element and the step to 32 bytes a thread."""
+    """Types with a dispatch of their own, around an empty block, a lone element, the step to 32 bytes a thread and, for
+    eight ranks, the one from which the halves say what leaves L2 first."""
     n = Shape.parse(text).world
     op = "avg" if dtype.is_floating_point else "sum"
-    for count in (1, 8 * n + 1, (2 << 20) // dtype.itemsize - 1, (2 << 20) // dtype.itemsize + 17):
+    for count in (1, 8 * n + 1, (2 << 20) // dtype.itemsize - 1, (2 << 20) // dtype.itemsize + 17, (4 << 20) // dtype.itemsize):
         make = tensors(n, count, dtype, True)
         assert both(n, make, lambda w, ts: w.all_reduce(ts, op=op, shape=text)) == 1
         assert both(n, make, lambda w, ts: (w.reduce_scatter(ts, op=op, shape=text), ts)[1]) == 1
