@@ -12,7 +12,6 @@ struct HostPrefixArgs {
   void* out[FT_MAX_FANIN];          // ordered by fan-in
   uint8_t first[FT_MAX_FANIN + 1];  // results first[k] .. first[k + 1] - 1 end with input k
   uint64_t bytes;                   // of each vector
-  uint32_t es;
   int n_in;
 };
 

@@ -102,7 +102,6 @@ int run_direct(int op, int dtype, const void* const* src, const int* fanin, void
   }
   a.first[a.n_in] = (uint8_t)filled;
   a.bytes = bytes;
-  a.es = (uint32_t)es;
   *err = ftk::launch_host_prefix(pol, a, st);
   return *err == cudaSuccess ? FT_OK : FT_ERR_CUDA;
 }

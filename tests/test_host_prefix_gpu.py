@@ -55,3 +55,26 @@ def test_results_over_later_inputs_and_over_one_another():
     torch.cuda.synchronize()
     assert torch.equal(hin[10], want[0]) and torch.equal(both, want[2])
     pipe.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.uint8])
+@pytest.mark.parametrize("n", [2, 3, 8])
+def test_cuts_of_the_pcie_kernel(dtype, n):
+    """Around a CTA's vectors, a warp of vectors with elements behind it, and the step to two vectors a thread: a last turn
+    that is full, nearly empty, or elements only."""
+    es = dtype.itemsize
+    pipe = HostReducePipeline(device=DEV, max_inputs=n, max_outputs=2)
+    for nvec in (0, 1, 31, 32, 1023, 1024, 6144, 6145, 18_432, 18_433, 24_577):
+        for tail in (0, 1, 16 // es - 1):
+            length = nvec * (16 // es) + tail
+            if not length:
+                continue
+            g = torch.Generator().manual_seed(length)
+            vecs = [torch.randint(0, 100, (length,), generator=g).to(dtype).pin_memory() for _ in range(n)]
+            flat = [torch.zeros(length + 32, dtype=dtype, pin_memory=True) for _ in range(2)]
+            pipe.run(vecs, [1, n], [f[:length] for f in flat])
+            torch.cuda.synchronize()
+            assert torch.equal(flat[0][:length], vecs[0])
+            assert torch.equal(flat[1][:length], reduce_nway([v.to(DEV) for v in vecs]).cpu()), (nvec, tail)
+            assert not any(f[length:].any() for f in flat)
+    pipe.close()
