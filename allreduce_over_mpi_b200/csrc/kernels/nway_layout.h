@@ -21,10 +21,13 @@ struct NwayArgs {
   int n;
   uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
   uint8_t shift[FT_MAX_FANIN];  // shifted kernels: bytes by which source k's body lies behind a 16-byte (realign: 32-byte) boundary
+  uint32_t ahead;             // CTAs that fetch their sources ahead of the kernel before (set at the launch)
 };
 
 // CTAs of a launch that covers the body once, `per_cta` vectors each, and the one for the edges.
 inline unsigned long long nway_grid(const NwayArgs& a, unsigned per_cta) { return (a.nvec + per_cta - 1) / per_cta + (a.edge != 0); }
+// CTAs of a call that moves `moved` bytes which fetch their sources ahead, `per_cta` bytes each: see pdl.cuh.
+inline uint32_t ahead_ctas(unsigned long long moved, unsigned per_cta) { return moved < (50u << 20) ? 0 : (12u << 20) / per_cta; }
 constexpr unsigned kWideThreads = 128;                  // wide and scaled kernels: a vector each
 constexpr unsigned kRealignThreads = 128, kRealignPerCta = kRealignThreads / 32 * 31;   // a warp stores 31 of the 32 it sums
 inline bool shift_long(const NwayArgs& a) { return a.nvec >= (3u << 20) / 16; }   // shifted kernel: 64 threads, two vectors each; else 128, one

@@ -6,9 +6,18 @@
 // stream order holds as before.  Every kernel launched this way calls pdl_begin().
 // fp32 x2 of 64 Ki elements, launches back to back: 4.1 -> 2.0 us each; bf16 x8 of 4 Mi: 14.4 -> 11.7.
 //
-// No kernel here asks for its successor earlier (griddepcontrol.launch_dependents): waiting CTAs then hold registers
-// and slots that the running kernel's own next CTAs want.  fp32 x4 of 1 M: 4.0 us with the request at the start, 2.6
-// with it behind the loads, 2.3 without.
+// Where data comes from HBM, some 1.7 us of the memory's time were still lost between two calls: the last CTAs of one drain,
+// the first of the next wait for their data.  So a call that moves 50 MB or more
+//   * lets its successor be set up once all its CTAs have issued their loads (pdl_next()), and
+//   * has its first CTAs fetch their sources into L2 while they wait in pdl_begin() (l2_ahead()): 12 MB, what HBM delivers in
+//     that time.  More, or all CTAs, cost L2 what they give HBM.
+// us a call, calls in a row on fresh tensors, without and with both: fp32 x2 of 5 M 10.0 -> 9.3, x5 (views) of 4 M 15.8 ->
+// 14.7, x8 of 2.5 M 14.3 -> 13.7, of 6.5 M 34.1 -> 33.7; bf16 x8 of 4 M 11.9 -> 11.0, its views 11.8 -> 10.4, averaged 12.0
+// -> 10.6; eight ranks' all-reduce of 6 MB 16.3 -> 15.4, of 25 MB 63.3 -> 62.1.  The request alone gives nothing.
+// Smaller calls neither ask nor fetch: in L2 the waiting CTAs hold slots that the running kernel's own next CTAs want, and the
+// fetches are in the way (fp32 x3 of 1 M in L2 2.2 us, 2.7 with both; x4 of 1 M with the request at the start 4.0 instead of
+// 2.3).  Above 50 MB that is so only for calls in a row on the same tensors, 100 MB at most (x3 of 5 M 6.1 -> 6.4, x4 7.2 ->
+// 9.0, x8 of 2.5 M 6.3 -> 6.4).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -28,6 +37,14 @@ inline cudaError_t launched(cudaError_t e) {
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+
+// The successor may be set up from here on; it still waits in its pdl_begin().
+__device__ __forceinline__ void pdl_next(uint32_t early) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q griddepcontrol.launch_dependents;\n\t}" ::"r"(early) : "memory");
+}
+// Fetch the line at p into L2.  In front of pdl_begin() too: L2 is where all SMs meet, so a line that the kernel before
+// this one still writes is the written one afterwards.
+__device__ __forceinline__ void l2_ahead(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 
 template <class... Params, class... Args>
 cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Args&... args) {

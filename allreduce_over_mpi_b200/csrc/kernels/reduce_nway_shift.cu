@@ -34,8 +34,13 @@ __device__ __forceinline__ uint4 join(uint4 lo, uint4 hi, uint32_t shift) {
 template <int POL, int UNROLL, int GROUP, int THREADS>
 __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
-  pdl_begin();
   const unsigned long long base = (unsigned long long)blockIdx.x * THREADS * UNROLL + threadIdx.x;
+  if (blockIdx.x < a.ahead && !(threadIdx.x & 7))
+    for (int k = 0; k < a.n; ++k)
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u)
+        if (base + u * THREADS < a.nvec) l2_ahead((const unsigned char*)a.src[k] + (base + u * THREADS) * 16);
+  pdl_begin();
   const bool last_lane = (threadIdx.x & 31) == 31;
   typename P::Acc acc[UNROLL];
   for (int k0 = 0; k0 < a.n; k0 += GROUP) {
@@ -53,6 +58,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid
           ex[g][u] = shift && last_lane && i < a.nvec ? ld_stream(p + i + 1) : make_uint4(0, 0, 0, 0);
         }
       }
+    if (k0 + GROUP >= a.n) pdl_next(a.ahead);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < a.n) {
@@ -106,10 +112,12 @@ __device__ __forceinline__ void join32(const uint32_t (&lo)[8], const uint32_t (
 template <int POL, int GROUP>
 __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
-  pdl_begin();
   const uint32_t lane = threadIdx.x & 31, shift = a.shift[0];
   const unsigned long long i = (unsigned long long)blockIdx.x * kRealignPerCta + threadIdx.x / 32 * 31 + lane;
   const bool ok = i <= a.nvec;   // one unit more than the result has
+  if (blockIdx.x < a.ahead && ok && !(lane & 3))
+    for (int k = 0; k < a.n; ++k) l2_ahead((const unsigned char*)a.src[k] - shift + i * 32);
+  pdl_begin();
   typename P::Acc al, ah;
   for (int k0 = 0; k0 < a.n; k0 += GROUP) {
     uint4 lo[GROUP], hi[GROUP];
@@ -121,6 +129,7 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
                      : "=r"(lo[g].x), "=r"(lo[g].y), "=r"(lo[g].z), "=r"(lo[g].w), "=r"(hi[g].x), "=r"(hi[g].y), "=r"(hi[g].z), "=r"(hi[g].w)
                      : "l"(p) : "memory");
       }
+    if (k0 + GROUP >= a.n) pdl_next(a.ahead);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < a.n) {
@@ -144,7 +153,9 @@ template <int POL, int UNROLL, int GROUP, int THREADS>
 static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
   const unsigned long long grid = nway_grid(a, THREADS * UNROLL);
   if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-  return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, a);
+  NwayArgs b = a;
+  b.ahead = ahead_ctas((a.n + 1) * a.nvec * 16, a.n * THREADS * UNROLL * 16);
+  return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, b);
 }
 // Long vectors want many small CTAs with few registers, two vectors of two sources at a time: with 256 threads and two
 // vectors of four sources 100 MB of fp32 x4 took 117 us, so they take 77 (6.5 TB/s).  Below 3 MB the chip is not full and
@@ -155,8 +166,10 @@ static cudaError_t launch_t(const NwayArgs& a, bool realign, cudaStream_t st) {
   if (realign) {
     const unsigned long long grid = nway_grid(a, kRealignPerCta);
     if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-    return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, kRealignThreads, 0, st, a)
-                    : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, kRealignThreads, 0, st, a);
+    NwayArgs b = a;
+    b.ahead = ahead_ctas((a.n + 1) * a.nvec * 32, a.n * kRealignPerCta * 32);
+    return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, kRealignThreads, 0, st, b)
+                    : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, kRealignThreads, 0, st, b);
   }
   return shift_long(a) ? launch_t<POL, 2, 2, 64>(a, st) : launch_t<POL, 1, 4, 128>(a, st);
 }

@@ -59,9 +59,16 @@ __device__ __forceinline__ void st32(void* p, const uint4& a, const uint4& b) {
 template <int POL, int NSRC, int THREADS, int GROUP>
 __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
-  pdl_begin();
   const unsigned long long i = (unsigned long long)blockIdx.x * THREADS + threadIdx.x;
   const bool ok = i < a.nvec;
+  if (blockIdx.x < a.ahead && ok && !(threadIdx.x & 3)) {
+#pragma unroll
+    for (int k = 0; k < (NSRC > 0 ? NSRC : FT_MAX_FANIN); ++k) {
+      if (NSRC == 0 && k >= a.n) break;
+      l2_ahead((const unsigned char*)a.src[k] + i * 32);
+    }
+  }
+  pdl_begin();
   constexpr int G = (NSRC > 0 && NSRC < GROUP) ? NSRC : GROUP;
   typename P::Acc al, ah;
 #pragma unroll
@@ -71,6 +78,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
 #pragma unroll
     for (int g = 0; g < G; ++g)
       if (ok && g0 + g < (NSRC > 0 ? NSRC : a.n)) ld32<0>((const unsigned char*)a.src[g0 + g] + i * 32, lo[g], hi[g]);
+    if (g0 + G >= (NSRC > 0 ? NSRC : a.n)) pdl_next(a.ahead);
 #pragma unroll
     for (int g = 0; g < G; ++g)
       if (g0 + g < (NSRC > 0 ? NSRC : a.n)) {
@@ -159,7 +167,9 @@ static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t
   if (code == 0) {
     const unsigned long long grid = nway_grid(a, kWideThreads);
     if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4>, (unsigned)grid, kWideThreads, 0, st, a);
+    NwayArgs b = a;
+    b.ahead = ahead_ctas((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32);
+    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4>, (unsigned)grid, kWideThreads, 0, st, b);
   }
   if constexpr (TUNING) {
     switch (code / 10) {

@@ -46,6 +46,7 @@ struct WorldArgs {
 // ---- programs the tree kernel is compiled for -----------------------------------------------------------------------
 // A program's steps as one word: start | pop << 1 | rounds << 2 of step k in bits 4k .. 4k + 3.  As text: S starts, a
 // adds, r is a round, p a pop.
+constexpr int kTreeThreads = 128;
 constexpr int kTreeRanks = 8, kTreeRounds = 6;   // ranks, and rounds of one entry, of a program in this form
 constexpr uint32_t tree_code(const char* s) {
   uint32_t code = 0;
@@ -88,7 +89,7 @@ constexpr int kWorldTreeCount = sizeof kWorldTrees / sizeof kWorldTrees[0];
 // there, or 15.
 constexpr int kTreeMask = 24, kTreeBlock = 32, kTreeWhich = 35, kTreeStore = 36;
 
-// 224 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
+// 240 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
 // cache after the other.
 struct WorldTreeArgs {
   uint64_t entry[kTreeRanks];
@@ -98,6 +99,7 @@ struct WorldTreeArgs {
   uint32_t es;
   float scale;
   uint32_t streams;   // what is read, and copies that are written, leave L2 before other data
+  uint32_t early, ahead;   // the next kernel may be set up early; CTAs that fetch their sources ahead (pdl.cuh)
 };
 
 }  // namespace ftk

@@ -1,0 +1,89 @@
+"""Large calls let the next one be set up before they end, and it fetches its sources ahead: whatever the calls in a row
+read of one another's results, and write over one another's sources, comes out as in stream order."""
+import pytest
+import torch
+
+from allreduce_over_mpi_b200.ops import reduce_nway, reduce_nway_scaled
+from allreduce_over_mpi_b200.parallel.comm import LocalWorld
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+N = 5_000_011   # three int32 vectors in, one out: 80 MB
+
+
+def vectors(n, offsets, dtype=torch.int32, seed=1):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return [torch.randint(-1000, 1000, (N + o,), generator=g, device=DEV).to(dtype)[o:] for _, o in zip(range(n), offsets)]
+
+
+@pytest.mark.parametrize("offsets", [(0, 0, 0, 0), (1, 1, 1, 0), (0, 1, 2, 3)], ids=["wide", "realign", "shift"])
+@pytest.mark.parametrize("between", ["nothing", "small", "torch"])
+def test_chain_of_sums(offsets, between):
+    ring, want = vectors(4, offsets), vectors(4, offsets)
+    tiny = [torch.ones(64, dtype=torch.int32, device=DEV) for _ in range(2)]
+    for step in range(16):   # each result is a source of the next call, over the oldest source of this one
+        k = [(step + j) % 4 for j in range(4)]
+        reduce_nway([ring[k[0]], ring[k[1]], ring[k[2]]], out=ring[k[3]])
+        if between == "small":
+            reduce_nway(tiny, out=tiny[step % 2])
+        elif between == "torch":
+            ring[k[3]].add_(step)
+    torch.cuda.synchronize()
+    for step in range(16):
+        k = [(step + j) % 4 for j in range(4)]
+        want[k[3]].copy_(want[k[0]] + want[k[1]] + want[k[2]] + (step if between == "torch" else 0))
+        torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(ring, want))
+
+
+def test_chain_of_averages():
+    ring = vectors(4, (0, 0, 0, 0), torch.float32)
+    want = [v.clone() for v in ring]
+    for step in range(12):
+        k = [(step + j) % 4 for j in range(4)]
+        reduce_nway_scaled([ring[k[0]], ring[k[1]], ring[k[2]]], scale=0.5, out=ring[k[3]])
+    torch.cuda.synchronize()
+    for step in range(12):
+        k = [(step + j) % 4 for j in range(4)]
+        want[k[3]].copy_((want[k[0]] + want[k[1]] + want[k[2]]) * 0.5)   # the kernel's additions, in its order
+    assert all(torch.equal(a, b) for a, b in zip(ring, want))
+
+
+@pytest.mark.parametrize("shape", ["2", "4", "2*4"])
+def test_chain_of_collectives(shape):
+    world = {"2": 2, "4": 4, "2*4": 8}[shape]
+    count = (64 << 20) // 4 // world + 5
+    w = LocalWorld(world, heap_bytes=(count * 4 + (1 << 20)), staging_bytes=1 << 20)
+    ts = [c.alloc(count, torch.int32) for c in w.ranks]
+    g = torch.Generator(device=DEV).manual_seed(3)
+    host = [torch.randint(-1000, 1000, (count,), generator=g, device=DEV).to(torch.int32) for _ in ts]
+    for t, h in zip(ts, host):
+        t.copy_(h)
+    want = torch.stack(host).sum(0, dtype=torch.int32)
+    for step in range(6):   # every rank's copy is the sum of all, so each call multiplies by the world
+        w.all_reduce(ts, shape=shape)
+        w.reduce_scatter(ts, shape=shape)
+        w.all_gather(ts, shape=shape)
+    torch.cuda.synchronize()
+    want = want * (world ** 11 % (1 << 32) if world ** 11 % (1 << 32) < 1 << 31 else world ** 11 % (1 << 32) - (1 << 32))
+    assert all(torch.equal(t, want) for t in ts)
+    w.close()
+
+
+def test_two_streams():
+    """Each stream's chain for itself, both at once."""
+    a, b = vectors(4, (0, 0, 0, 0), seed=5), vectors(4, (0, 0, 0, 0), seed=6)
+    want = [[v.clone() for v in a], [v.clone() for v in b]]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for step in range(16):
+        k = [(step + j) % 4 for j in range(4)]
+        for ring, st in ((a, streams[0]), (b, streams[1])):
+            with torch.cuda.stream(st):
+                reduce_nway([ring[k[0]], ring[k[1]], ring[k[2]]], out=ring[k[3]])
+    torch.cuda.synchronize()
+    for ring in want:
+        for step in range(16):
+            k = [(step + j) % 4 for j in range(4)]
+            ring[k[3]].copy_(ring[k[0]] + ring[k[1]] + ring[k[2]])
+    assert all(torch.equal(x, y) for x, y in zip(a + b, want[0] + want[1]))
