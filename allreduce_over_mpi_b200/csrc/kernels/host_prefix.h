@@ -13,6 +13,7 @@ struct HostPrefixArgs {
   uint8_t first[FT_MAX_FANIN + 1];  // results first[k] .. first[k + 1] - 1 end with input k
   uint64_t bytes;                   // of each vector
   int n_in;
+  uint64_t fill[4];                 // to a size that is cheap to launch with (pdl.cuh)
 };
 
 cudaError_t launch_host_prefix(int pol, const HostPrefixArgs& a, cudaStream_t st);

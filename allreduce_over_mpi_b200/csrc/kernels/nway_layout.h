@@ -22,6 +22,8 @@ struct NwayArgs {
   uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
   uint8_t shift[FT_MAX_FANIN];  // shifted kernels: bytes by which source k's body lies behind a 16-byte (realign: 32-byte) boundary
   uint32_t ahead;             // CTAs that fetch their sources ahead of the kernel before (set at the launch)
+  float scale;                // scaled kernels
+  uint64_t fill[2];           // to a size that is cheap to launch with (pdl.cuh)
 };
 
 // CTAs of a launch that covers the body once, `per_cta` vectors each, and the one for the edges.

@@ -464,7 +464,8 @@ int ft_reduce_nway_scaled(int in_dtype, int out_dtype, const void* const* src, v
   }
   a.dst = dst;
   a.n = n;
-  const cudaError_t e = launch_scaled(in_dtype == FT_BF16, out_dtype == FT_BF16, a, len, scale, dev_info().sms, (cudaStream_t)stream);
+  a.scale = scale;
+  const cudaError_t e = launch_scaled(in_dtype == FT_BF16, out_dtype == FT_BF16, a, len, dev_info().sms, (cudaStream_t)stream);
   return e == cudaSuccess ? FT_OK : cuda_fail(e, "reduce_nway_scaled launch");
 }
 

@@ -14,8 +14,8 @@ namespace ftk {
 cudaError_t launch_wide(int pol, const NwayArgs& a, int code, int sms, cudaStream_t st);
 // Kernels for pointers that do not agree modulo 32 (reduce_nway_shift.cu); `realign`: the sources do, the result does not.
 cudaError_t launch_shift(int pol, const NwayArgs& a, bool realign, cudaStream_t st);
-// out = scale * sum over `len` elements of whole vectors in `a` (reduce_nway_scaled.cu).
-cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st);
+// out = a.scale * sum over `len` elements of whole vectors in `a` (reduce_nway_scaled.cu).
+cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, int sms, cudaStream_t st);
 
 #ifdef __CUDACC__
 // The edges of the vector, by the CTA the launch adds for them (less than 160 bytes: one or two units a thread).

@@ -51,7 +51,7 @@ __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, f
 // WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
 // 32); not WIDE: 128-bit ones.
 template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP>
-__global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a, float scale) {
+__global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a) {
   constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
   const unsigned long long i = (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
   if (blockIdx.x < a.ahead && i < a.nvec && !(threadIdx.x & 3))
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   if (i >= a.nvec) {   // (with a predicate on each load instead, fp32 x2 -> bf16 of 8 M took 14.8 us, not 12.9)
     if (a.edge && blockIdx.x == gridDim.x - 1)
       for (int e = threadIdx.x; e < (int)a.edge; e += kThreads)
-        scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), scale);
+        scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), a.scale);
     return;
   }
   float acc[E];
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   constexpr int W = OUT_BF16 ? E / 2 : E;   // output words
   uint32_t o[W];
 #pragma unroll
-  for (int j = 0; j < W; ++j) o[j] = OUT_BF16 ? pack_bf16x2(acc[(2 * j) % E] * scale, acc[(2 * j + 1) % E] * scale) : __float_as_uint(acc[j] * scale);
+  for (int j = 0; j < W; ++j) o[j] = OUT_BF16 ? pack_bf16x2(acc[(2 * j) % E] * a.scale, acc[(2 * j + 1) % E] * a.scale) : __float_as_uint(acc[j] * a.scale);
   unsigned char* d = (unsigned char*)a.dst + i * (W * 4);
   if constexpr (W == 4) {
     st_vec_cs(d, make_uint4(o[0], o[1], o[2], o[3]));
@@ -102,10 +102,10 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
 // Eight sources of 6.5 M, one element off: fp32 36.6 us (34.6 with a common vector), fp32 -> bf16 34.9 (33.1); bf16, with two
 // bytes an access, 27.4 us (15.4), 4.3 TB/s.
 template <bool IN_BF16, bool OUT_BF16>
-__global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __grid_constant__ NwayArgs a, unsigned long long len, float scale) {
+__global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __grid_constant__ NwayArgs a) {
   pdl_begin();
-  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (unsigned long long)gridDim.x * blockDim.x)
-    scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, scale);
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.nbody; i += (unsigned long long)gridDim.x * blockDim.x)
+    scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, a.scale);
 }
 
 // Two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up the loop is as good or
@@ -113,34 +113,36 @@ __global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __
 // sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with four, 24.7
 // with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four).
 template <bool IN_BF16, bool OUT_BF16, bool WIDE>
-static cudaError_t launch_n(const NwayArgs& a, unsigned grid, float scale, cudaStream_t st) {
+static cudaError_t launch_n(const NwayArgs& a, unsigned grid, cudaStream_t st) {
   switch (a.n) {
-    case 2: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 2, 2>, grid, kThreads, 0, st, a, scale);
-    case 3: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 3, 3>, grid, kThreads, 0, st, a, scale);
+    case 2: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 2, 2>, grid, kThreads, 0, st, a);
+    case 3: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 3, 3>, grid, kThreads, 0, st, a);
     default: break;
   }
-  return a.n <= 8 ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 4>, grid, kThreads, 0, st, a, scale)
-                  : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 8>, grid, kThreads, 0, st, a, scale);
+  return a.n <= 8 ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 4>, grid, kThreads, 0, st, a)
+                  : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 8>, grid, kThreads, 0, st, a);
 }
 
 template <bool IN_BF16, bool OUT_BF16>
-static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, float scale, int sms, cudaStream_t st) {
+static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, int sms, cudaStream_t st) {
   NwayArgs a;
   bool wide;
   if (!layout_scaled(in, len, IN_BF16, OUT_BF16, &a, &wide)) {
     const unsigned long long want = (len + 255) / 256, cap = (unsigned long long)sms * 8;
-    return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, in, len, scale);
+    a = in;
+    a.nbody = len;
+    return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, a);
   }
   const unsigned long long grid = nway_grid(a, kThreads);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
   constexpr unsigned out_bytes = (IN_BF16 ? 16 : 8) * (OUT_BF16 ? 2 : 4);
   a.ahead = ahead_ctas((a.n * 32 + out_bytes) * a.nvec, a.n * kThreads * 32);
-  return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, scale, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, scale, st);
+  return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, st);
 }
 
-cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, float scale, int sms, cudaStream_t st) {
-  if (in_bf16) return out_bf16 ? launch_t<true, true>(a, len, scale, sms, st) : launch_t<true, false>(a, len, scale, sms, st);
-  return out_bf16 ? launch_t<false, true>(a, len, scale, sms, st) : launch_t<false, false>(a, len, scale, sms, st);
+cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, int sms, cudaStream_t st) {
+  if (in_bf16) return out_bf16 ? launch_t<true, true>(a, len, sms, st) : launch_t<true, false>(a, len, sms, st);
+  return out_bf16 ? launch_t<false, true>(a, len, sms, st) : launch_t<false, false>(a, len, sms, st);
 }
 
 }  // namespace ftk

@@ -29,7 +29,7 @@ struct WorldEntry {
 // What is left of a step in the kernel's parameters besides the pointer: start | pop << 1 | rounds << 2.
 // One table of pointers: of step k the copy it takes, and from kSteps on the ranks' results.  The kernel looks the sources
 // up in groups, past an entry's last step, without reading them: behind the last step of all lies rank 0's input or
-// these.  (56 bytes more for that cost every call 0.24 us: 1048 bytes of parameters 2.58 us, 1104 bytes 2.82.)
+// these.
 template <int RANKS>
 struct WorldArgs {
   static constexpr int kSteps = RANKS * RANKS;
@@ -89,17 +89,18 @@ constexpr int kWorldTreeCount = sizeof kWorldTrees / sizeof kWorldTrees[0];
 // there, or 15.
 constexpr int kTreeMask = 24, kTreeBlock = 32, kTreeWhich = 35, kTreeStore = 36;
 
-// 240 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
+// 224 bytes, looked up by few and short chains: the interpreter's 1 KB of tables costs each launch one miss of the constant
 // cache after the other.
 struct WorldTreeArgs {
   uint64_t entry[kTreeRanks];
   const void* in[kTreeRanks];
   void* out[kTreeRanks];
   uint64_t total_bytes, block_bytes;
-  uint32_t es;
   float scale;
-  uint32_t streams;   // what is read, and copies that are written, leave L2 before other data
-  uint32_t early, ahead;   // the next kernel may be set up early; CTAs that fetch their sources ahead (pdl.cuh)
+  uint32_t ahead;   // CTAs that fetch their sources ahead (pdl.cuh)
+  uint8_t es;
+  uint8_t early;    // the next kernel may be set up early
+  uint8_t streams;  // what is read, and copies that are written, leave L2 before other data
 };
 
 }  // namespace ftk

@@ -504,7 +504,7 @@ cudaError_t tree_launch(const ft::WorldProgram& wp, int pol, int world, const vo
   a.streams = phase != 0 && bytes * world >= (32u << 20);
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
-  a.es = es;
+  a.es = (uint8_t)es;
   a.scale = scale;
   const bool wide = world_wide(world, in, out, bytes, block_bytes);
   // Fetching ahead and an early successor (pdl.cuh) as in the n-way sums.  A gather finds its sources in L2.  One of two ranks
