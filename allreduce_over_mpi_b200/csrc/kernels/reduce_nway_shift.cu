@@ -5,7 +5,8 @@
 // bytes behind a boundary there is read with aligned 16-byte loads, and each lane puts its vector together from
 // its own load and its right neighbour's (a warp shuffle; lane 31 loads the one vector more).  Memory bounds the
 // kernel: every byte is still read once, where the one-element loads this replaces moved 4 bytes an instruction.
-// The host keeps all loads inside the vectors (layout_shift in nway_layout.h).
+// The host keeps all loads inside the vectors (layout_shift in nway_layout.h).  Fetching ahead (pdl.cuh) gives it nothing:
+// fp32 x5 of 4 M 18.4 us without, 18.5 with, bf16 x8 of 4 M 14.7 and 15.0.
 //
 // Where all sources lie at one phase and only the result at another (views summed into a new tensor), the second
 // kernel keeps 256-bit loads on the sources' boundaries and moves the RESULT across: one shuffle step per 32 bytes of
@@ -35,11 +36,6 @@ template <int POL, int UNROLL, int GROUP, int THREADS>
 __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   const unsigned long long base = (unsigned long long)blockIdx.x * THREADS * UNROLL + threadIdx.x;
-  if (blockIdx.x < a.ahead && !(threadIdx.x & 7))
-    for (int k = 0; k < a.n; ++k)
-#pragma unroll
-      for (int u = 0; u < UNROLL; ++u)
-        if (base + u * THREADS < a.nvec) l2_ahead((const unsigned char*)a.src[k] + (base + u * THREADS) * 16);
   pdl_begin();
   const bool last_lane = (threadIdx.x & 31) == 31;
   typename P::Acc acc[UNROLL];
@@ -58,7 +54,6 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_shift_kernel(const __grid
           ex[g][u] = shift && last_lane && i < a.nvec ? ld_stream(p + i + 1) : make_uint4(0, 0, 0, 0);
         }
       }
-    if (k0 + GROUP >= a.n) pdl_next(a.ahead);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < a.n) {
@@ -108,7 +103,8 @@ __device__ __forceinline__ void join32(const uint32_t (&lo)[8], const uint32_t (
 
 // A warp sums 32 units of 32 bytes on the sources' boundaries and stores the 31 units of the result between them; the
 // next warp sums the last one again (a hit in L2).  a.nvec: units of the result; shift[0]: bytes by which it lies behind
-// the sources' boundaries.  bf16 x8 of 4 M, sources one element off: 14.3 us by the kernel above, 12.0 here.
+// the sources' boundaries.  bf16 x8 of 4 M, sources one element off: 14.3 us by the kernel above, 11.2 here, 10.1 in a row
+// with fetching ahead (pdl.cuh); the edges are the first CTA's then, which is not the last to end.
 template <int POL, int GROUP>
 __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
@@ -146,16 +142,14 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
   if (lane < 31 && i < a.nvec)
     asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                  ::"l"((unsigned char*)a.dst + i * 32), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-  if (a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
+  if (a.edge && blockIdx.x == (a.ahead ? 0 : gridDim.x - 1)) reduce_edges<POL, ScalarOp>(a);
 }
 
 template <int POL, int UNROLL, int GROUP, int THREADS>
 static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
   const unsigned long long grid = nway_grid(a, THREADS * UNROLL);
   if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
-  NwayArgs b = a;
-  b.ahead = ahead_ctas((a.n + 1) * a.nvec * 16, a.n * THREADS * UNROLL * 16);
-  return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, b);
+  return launch_pdl(reduce_nway_shift_kernel<POL, UNROLL, GROUP, THREADS>, (unsigned)grid, THREADS, 0, st, a);
 }
 // Long vectors want many small CTAs with few registers, two vectors of two sources at a time: with 256 threads and two
 // vectors of four sources 100 MB of fp32 x4 took 117 us, so they take 77 (6.5 TB/s).  Below 3 MB the chip is not full and

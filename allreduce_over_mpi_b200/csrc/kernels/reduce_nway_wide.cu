@@ -46,22 +46,32 @@ __device__ __forceinline__ void st32(void* p, const uint4& a, const uint4& b) {
 
 // The default: one 32-byte unit per thread, 128 threads, the grid covers the vector once, evict-first stores.  NSRC > 0:
 // the fan-in is known at compile time; NSRC == 0: it is a.n (any value up to FT_MAX_FANIN).  Sources are taken GROUP at
-// a time (four, or eight from nine sources up): all loads of a group are issued before its first add.  How a thread
+// a time: all loads of a group are issued before its first add.  How a thread
 // behind the end is kept from loading decides how many the compiler leaves in flight: a predicate on each load keeps a
 // group and more (72 registers, bf16 x8 of 4 M 11.7 us), leaving early 50 registers and 12.2 us, loading zeros instead
-// 40 registers and 14.1 us.  The edges, the job of the last CTA, come behind for the same reason: a branch in front of
-// the loads cost 3 to 5 %.
+// 40 registers and 14.1 us.
 //
-// What bounds it is HBM, or L2 below about 100 MB.  Over 2, 4, 8 and 16 sources of 16 KB to 256 MB in fp32, bf16 and fp16
-// it is 0.8 % from the best of 12 configurations on average and 8 % at most (128-512 threads, groups of 4 and 8, three
-// places for the dependent launch); 256 threads lose up to 26 % where the grid fills the chip only once or twice.
-// fp32 x8 of 1 M: 4.0 us; of 10 M: 51.9 us (6.9 TB/s); of 64 Mi: 334 us (7.2 TB/s).
-template <int POL, int NSRC, int THREADS, int GROUP>
+// What bounds it is HBM, or L2 below about 100 MB.
+// Calls below 50 MB: groups of four (eight from nine sources up).  Over 2, 4, 8 and 16 sources of 16 KB to 256 MB in fp32,
+// bf16 and fp16 that is 0.8 % from the best of 12 configurations on average and 8 % at most (128-512 threads, groups of 4
+// and 8, three places for the dependent launch); 256 threads lose up to 26 % where the grid fills the chip only once or
+// twice.  The edges are the job of a CTA of their own, the last one, behind the body: a branch in front of the loads cost 3
+// to 5 %.  fp32 x8 of 1 M: 4.8 us.
+// Larger ones (EARLY) fetch ahead and ask for their successor (pdl.cuh).  Where they ask decides what it is worth: behind
+// the first load of the last group, with the edges between the loads and the additions, it works; with code behind the
+// store it worked no better than asking at the very end.  All of up to eight sources in flight together pay then, and the
+// edges are the first CTA's: the last one starts when the call is nearly over (fp32 x3 views of 5 M 12.2 us with the last
+// one, 11.4 with the first).  us, calls in a row on fresh tensors, neither / this: fp32 x2 of 5 M 10.1 / 8.8, x3 views 12.9
+// / 11.4, x4 of 2.7 M 9.2 / 7.9, x8 of 1.5 M 9.4 / 8.0, of 2.5 M 14.5 / 12.9, of 6.5 M 34.3 / 33.2 (7.1 TB/s), of 64 Mi
+// 335.1 / 334.2 (7.2); bf16 x8 of 4 M 12.0 / 10.6; int32 masks x6 of 3 M 13.6 / 12.1; fp64 x2 of 4 M 15.4 / 14.1.  From nine
+// sources up they ask behind the fourth load of the last group (fp32 x16 of 1.2 M 13.2 / 12.1), in 16-bit floats behind all of
+// them (x16 of 8 M 40.2, 39.1 so, 39.8 behind the fourth).  In a captured graph less of it is left: x8 of 2.5 M 14.3 / 14.0.
+template <int POL, int NSRC, int THREADS, int GROUP, bool EARLY>
 __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
   const unsigned long long i = (unsigned long long)blockIdx.x * THREADS + threadIdx.x;
   const bool ok = i < a.nvec;
-  if (blockIdx.x < a.ahead && ok && !(threadIdx.x & 3)) {
+  if (EARLY && blockIdx.x < a.ahead && ok && !(threadIdx.x & 3)) {
 #pragma unroll
     for (int k = 0; k < (NSRC > 0 ? NSRC : FT_MAX_FANIN); ++k) {
       if (NSRC == 0 && k >= a.n) break;
@@ -70,15 +80,21 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
   }
   pdl_begin();
   constexpr int G = (NSRC > 0 && NSRC < GROUP) ? NSRC : GROUP;
+  constexpr bool between = EARLY && NSRC > 0 && sizeof(typename ScalarOp<POL>::elem) < 8;   // (8-byte edges there take up to 166 registers)
+  // the load of the last group behind which the successor is asked for
+  constexpr int ASK = between ? 0 : NSRC > 0 ? (G - 1) / 2 : POL == POL_BF16 || POL == POL_F16 ? G - 1 : 3;
   typename P::Acc al, ah;
 #pragma unroll
   for (int g0 = 0; g0 < (NSRC > 0 ? NSRC : FT_MAX_FANIN); g0 += G) {
     if (NSRC == 0 && g0 >= a.n) break;
+    const bool last = g0 + G >= (NSRC > 0 ? NSRC : a.n);
     uint4 lo[G], hi[G];
 #pragma unroll
-    for (int g = 0; g < G; ++g)
+    for (int g = 0; g < G; ++g) {
       if (ok && g0 + g < (NSRC > 0 ? NSRC : a.n)) ld32<0>((const unsigned char*)a.src[g0 + g] + i * 32, lo[g], hi[g]);
-    if (g0 + G >= (NSRC > 0 ? NSRC : a.n)) pdl_next(a.ahead);
+      if (EARLY && g == ASK && last) pdl_next(1);
+    }
+    if (between && last && a.edge && blockIdx.x == 0) reduce_edges<POL, ScalarOp>(a);
 #pragma unroll
     for (int g = 0; g < G; ++g)
       if (g0 + g < (NSRC > 0 ? NSRC : a.n)) {
@@ -87,7 +103,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
       }
   }
   if (ok) st32<1>((unsigned char*)a.dst + i * 32, P::fin(al), P::fin(ah));
-  if (!ok && a.edge && blockIdx.x == gridDim.x - 1) reduce_edges<POL, ScalarOp>(a);
+  if (!between && (EARLY || !ok) && a.edge && blockIdx.x == (EARLY ? 0 : gridDim.x - 1)) reduce_edges<POL, ScalarOp>(a);
 }
 
 // The configurations that are asked for by number: one thread handles UNROLL 32-byte units per step, THREADS apart (every warp access is one
@@ -169,7 +185,8 @@ static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t
     if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
     NwayArgs b = a;
     b.ahead = ahead_ctas((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32);
-    return launch_pdl(reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4>, (unsigned)grid, kWideThreads, 0, st, b);
+    return launch_pdl(b.ahead ? reduce_nway_wide_kernel<POL, NSRC, kWideThreads, 8, true>
+                              : reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4, false>, (unsigned)grid, kWideThreads, 0, st, b);
   }
   if constexpr (TUNING) {
     switch (code / 10) {

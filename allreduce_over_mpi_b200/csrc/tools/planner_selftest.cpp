@@ -628,8 +628,9 @@ struct NwayReplay {
       write(dst(i * (long long)os), os, os);
     }
   }
-  // wide and scaled kernels: 32 bytes of every source a thread, `out` bytes of the result
-  void wide(size_t load, size_t out, size_t store) {
+  // wide and scaled kernels: 32 bytes of every source a thread, `out` bytes of the result.  `first`: the edges are the
+  // first CTA's, as in calls that fetch ahead, else the last one's
+  void wide(size_t load, size_t out, size_t store, bool first = false) {
     const unsigned long long grid = ftk::nway_grid(a, ftk::kWideThreads);
     need(grid > 0);
     for (unsigned long long cta = 0; cta < grid; ++cta)
@@ -638,12 +639,13 @@ struct NwayReplay {
         if (i < a.nvec) {
           for (int k = 0; k < a.n; ++k) read(k, src(k, i * 32), 32, load);
           write(dst(i * out), out, store);
-        } else if (cta == grid - 1) {
+        } else if (!first && cta == grid - 1) {
           edges(t, ftk::kWideThreads);
         }
+        if (first && cta == 0) edges(t, ftk::kWideThreads);
       }
   }
-  void realign() {
+  void realign(bool first = false) {
     const unsigned long long grid = ftk::nway_grid(a, ftk::kRealignPerCta);
     need(grid > 0 && a.shift[0] > 0 && a.shift[0] < 32);
     for (unsigned long long cta = 0; cta < grid; ++cta)
@@ -653,7 +655,7 @@ struct NwayReplay {
         if (i <= a.nvec)
           for (int k = 0; k < a.n; ++k) read(k, src(k, (long long)(i * 32) - a.shift[0]), 32, 32);
         if (lane < 31 && i < a.nvec) write(dst(i * 32), 32, 32);   // from this unit's sum and the next lane's: i + 1 <= nvec
-        if (a.edge && cta == grid - 1) edges(t, ftk::kRealignThreads);
+        if (a.edge && cta == (first ? 0 : grid - 1)) edges(t, ftk::kRealignThreads);
       }
   }
   void shift() {
@@ -682,11 +684,11 @@ struct NwayReplay {
   }
 };
 static int nway_kernel_seen[5];   // wide, realign, shift, scaled wide, scaled narrow
-static bool replay_nway(const ftk::NwayArgs& in, size_t unit, size_t len) {
+static bool replay_nway(const ftk::NwayArgs& in, size_t unit, size_t len, bool first = false) {
   NwayReplay r{in, in, unit, unit, len, std::vector<uint8_t>(len * unit)};
   // the order of run_policy() in reduce_nway.cu
-  if (ftk::layout_wide(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[0]; r.wide(32, 32, 32); }
-  else if (ftk::layout_realign(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[1]; r.realign(); }
+  if (ftk::layout_wide(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[0]; r.wide(32, 32, 32, first); }
+  else if (ftk::layout_realign(in, len * unit, unit, &r.a)) { ++nway_kernel_seen[1]; r.realign(first); }
   else { ++nway_kernel_seen[2]; ftk::layout_shift(in, len * unit, unit, &r.a); r.shift(); }
   return r.done();
 }
@@ -713,7 +715,7 @@ static void nway_layouts() {
           ftk::NwayArgs in{};
           in.n = 2;
           in.dst = at(0, d); in.src[0] = at(1, s0); in.src[1] = at(2, s1);
-          for (size_t len : lens) EXPECT(replay_nway(in, unit, len));
+          for (size_t len : lens) EXPECT(replay_nway(in, unit, len) && replay_nway(in, unit, len, true));
           if (unit != 2 && unit != 4) continue;
           for (bool out_bf16 : {false, true})
             if (d % (out_bf16 ? 2 : 4) == 0)

@@ -87,3 +87,22 @@ def test_two_streams():
             k = [(step + j) % 4 for j in range(4)]
             ring[k[3]].copy_(ring[k[0]] + ring[k[1]] + ring[k[2]])
     assert all(torch.equal(x, y) for x, y in zip(a + b, want[0] + want[1]))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float64, torch.uint8, torch.int64])
+@pytest.mark.parametrize("n", [1, 2, 5, 8, 11, 16])
+def test_large_calls_of_every_fan_in(n, dtype):
+    """Just below and above the size from which calls fetch ahead, ragged at both ends: every element once, none beside."""
+    es = dtype.itemsize
+    for moved in ((50 << 20) - 4096, (50 << 20) + 8192):
+        for head, tail in ((0, 0), (1, 3)):
+            length = moved // ((n + 1) * es) // 32 * 32 + (32 - head if head else 0) + tail
+            g = torch.Generator(device=DEV).manual_seed(length)
+            ts = [torch.randint(0, 20, (length + head,), generator=g, device=DEV).to(dtype)[head:] for _ in range(n)]
+            flat = torch.full((length + head + 64,), 99, dtype=dtype, device=DEV)
+            out = reduce_nway(ts, out=flat[head:length + head])
+            want = ts[0].clone()
+            for t in ts[1:]:   # small whole numbers: exact in every type, in any order
+                want += t
+            assert torch.equal(out, want)
+            assert bool((flat[:head] == 99).all()) and bool((flat[length + head:] == 99).all())
