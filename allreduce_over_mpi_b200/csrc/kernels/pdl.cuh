@@ -11,13 +11,13 @@
 //   * lets its successor be set up once all its CTAs have issued their loads (pdl_next()), and
 //   * has its first CTAs fetch their sources into L2 while they wait in pdl_begin() (l2_ahead()): 12 MB, what HBM delivers in
 //     that time.  More, or all CTAs, cost L2 what they give HBM.
-// us a call, calls in a row on fresh tensors, without and with both: fp32 x2 of 5 M 10.0 -> 9.3, x5 (views) of 4 M 15.8 ->
-// 14.7, x8 of 2.5 M 14.3 -> 13.7, of 6.5 M 34.1 -> 33.7; bf16 x8 of 4 M 11.9 -> 11.0, its views 11.8 -> 10.4, averaged 12.0
-// -> 10.6; eight ranks' all-reduce of 6 MB 16.3 -> 15.4, of 25 MB 63.3 -> 62.1.  The request alone gives nothing.
+// us a call, calls in a row on fresh tensors, without and with both: fp32 x2 of 5 M 10.1 -> 8.8, x3 views 12.9 -> 11.4, x8 of 2.5 M
+// 14.5 -> 12.9, of 6.5 M 34.3 -> 33.2; bf16 x8 of 4 M 12.0 -> 10.6, its views 11.2 -> 10.1, averaged 12.0 -> 10.6; eight ranks'
+// all-reduce of 6 MB 16.6 -> 15.3, of 25 MB 63.5 -> 62.2.  The request alone gives nothing.
 // Smaller calls neither ask nor fetch: in L2 the waiting CTAs hold slots that the running kernel's own next CTAs want, and the
 // fetches are in the way (fp32 x3 of 1 M in L2 2.2 us, 2.7 with both; x4 of 1 M with the request at the start 4.0 instead of
-// 2.3).  Above 50 MB that is so only for calls in a row on the same tensors, 100 MB at most (x3 of 5 M 6.1 -> 6.4, x4 7.2 ->
-// 9.0, x8 of 2.5 M 6.3 -> 6.4).
+// 2.3).  Above 50 MB that is so only for calls in a row on one set of tensors that L2 holds whole, up to 100 MB (x2 of 5 M 5.0 ->
+// 6.0, x3 5.9 -> 6.4, x8 of 2.5 M 6.2 -> 7.0); with two sets in turn x2 has 7.1 -> 7.4, x3 12.7 -> 11.4, x8 14.5 -> 13.0.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
