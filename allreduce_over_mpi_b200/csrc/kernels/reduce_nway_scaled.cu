@@ -2,10 +2,10 @@
 // fused into the store).
 //
 // HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, four
-// sources in flight, the grid covers the vector once, edges in a CTA of their own, dependent launch.  The unit
+// or more sources in flight, the grid covers the vector once, dependent launch.  The unit
 // is 8 fp32 or 16 bf16 elements, whatever the output type, so that the source side (n streams to one) stays on 256-bit
 // loads.  fp32 -> bf16, 8 sources of 6.5 M: 38.9 us (5.7 TB/s, a strided loop with 16-byte loads of one source at a
-// time) -> 33.0 us (6.8 TB/s).
+// time) -> 31.6 us (7.0 TB/s).
 #include "../api/flextree.h"
 #include "pdl.cuh"
 #include "reduce_nway.cuh"
@@ -49,18 +49,25 @@ __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, f
 }
 
 // WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
-// 32); not WIDE: 128-bit ones.
-template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP>
+// 32); not WIDE: 128-bit ones.  ASK: kPlain, or (calls that fetch ahead, pdl.cuh) the load of the last group behind which
+// the successor is asked for, kAskLast behind all of them; the edges are the first CTA's then.  LEAVE: a thread behind the
+// end leaves; else a predicate keeps it from each load.
+constexpr int kPlain = -2, kAskLast = -1;
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK, bool LEAVE>
 __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a) {
   constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
+  constexpr bool early = ASK != kPlain;
   const unsigned long long i = (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
-  if (blockIdx.x < a.ahead && i < a.nvec && !(threadIdx.x & 3))
+  const bool ok = i < a.nvec;
+  if (early && blockIdx.x < a.ahead && ok && !(threadIdx.x & 3))
     for (int k = 0; k < (NSRC > 0 ? NSRC : a.n); ++k) l2_ahead((const unsigned char*)a.src[k] + i * 32);
   pdl_begin();
-  if (i >= a.nvec) {   // (with a predicate on each load instead, fp32 x2 -> bf16 of 8 M took 14.8 us, not 12.9)
-    if (a.edge && blockIdx.x == gridDim.x - 1)
-      for (int e = threadIdx.x; e < (int)a.edge; e += kThreads)
-        scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), a.scale);
+  const auto edges = [&] {
+    for (int e = threadIdx.x; e < (int)a.edge; e += kThreads)
+      scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), a.scale);
+  };
+  if (LEAVE && !ok) {
+    if (!early && a.edge && blockIdx.x == gridDim.x - 1) edges();
     return;
   }
   float acc[E];
@@ -68,11 +75,15 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   for (int j = 0; j < E; ++j) acc[j] = 0.f;
   const int n = NSRC > 0 ? NSRC : a.n;
   for (int k0 = 0; k0 < n; k0 += GROUP) {
+    const bool last = k0 + GROUP >= n;
     uint4 lo[GROUP], hi[GROUP];
 #pragma unroll
-    for (int g = 0; g < GROUP; ++g)
-      if (k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
-    if (k0 + GROUP >= n) pdl_next(a.ahead);
+    for (int g = 0; g < GROUP; ++g) {
+      if ((LEAVE || ok) && k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
+      if (ASK == g && last) pdl_next(1);
+    }
+    if (early && last && a.edge && blockIdx.x == 0) edges();
+    if (ASK == kAskLast && last) pdl_next(1);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < n) {
@@ -84,6 +95,7 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
         }
       }
   }
+  if (!LEAVE && !ok) return;
   constexpr int W = OUT_BF16 ? E / 2 : E;   // output words
   uint32_t o[W];
 #pragma unroll
@@ -108,19 +120,48 @@ __global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __
     scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, a.scale);
 }
 
-// Two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up the loop is as good or
-// better (with the fan-in known the compiler keeps fewer loads in flight: bf16 x8 of 4 M 14.3 us, not 12.0).  Eight
-// sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with four, 24.7
-// with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four).
+// Calls that do not fetch ahead: two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up
+// the loop is as good or better (with the fan-in known the compiler keeps fewer loads in flight: bf16 x8 of 4 M 14.3 us, not
+// 12.0).  Eight sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with
+// four, 24.7 with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four).  Threads behind the end leave: with a
+// predicate on each load fp32 x2 -> bf16 of 8 M took 14.8 us, not 12.9.
+// Calls that do, us on fresh tensors, not / asking behind all loads with the plain form / so: fp32 x2 of 6 M 11.9 / 11.1 / 10.9,
+// -> bf16 10.0 / 9.5 / 8.8; x3 -> bf16 of 5 M 11.4 / 11.0 / 10.9, bf16 x3 of 9 M 11.8 / 11.2 / 10.3; fp32 x4 -> bf16 of 5 M
+// 14.4 / 14.2 / 13.1 (four in flight; 14.0 with eight); fp32 x7 -> bf16 of 3 M 14.5 / 14.2 / 13.4, x8 -> bf16 of 6.5 M 33.0 / 32.4 /
+// 31.6 (7.0 TB/s), x8 of 2.5 M 14.8 / 13.7 / 13.1; bf16 x4 of 8 M 13.1 / 12.7 / 11.5, x7 of 8 M 20.0 / 19.6 / 18.3, x8 of 4 M 12.1 /
+// 11.1 / 10.7 (bf16 with the fan-in known; 11.8, 19.4 and 11.7 without); bf16 x16 of 5 M 26.1 / 25.4 / 25.1.
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK, bool LEAVE>
+static cudaError_t launch_k(const NwayArgs& a, unsigned grid, cudaStream_t st) {
+  return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, NSRC, GROUP, ASK, LEAVE>, grid, kThreads, 0, st, a);
+}
 template <bool IN_BF16, bool OUT_BF16, bool WIDE>
 static cudaError_t launch_n(const NwayArgs& a, unsigned grid, cudaStream_t st) {
-  switch (a.n) {
-    case 2: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 2, 2>, grid, kThreads, 0, st, a);
-    case 3: return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 3, 3>, grid, kThreads, 0, st, a);
-    default: break;
+  if (!a.ahead) {
+    switch (a.n) {
+      case 2: return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, kPlain, true>(a, grid, st);
+      case 3: return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, kPlain, true>(a, grid, st);
+      default: break;
+    }
+    return a.n <= 8 ? launch_k<IN_BF16, OUT_BF16, WIDE, 0, 4, kPlain, true>(a, grid, st)
+                    : launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kPlain, true>(a, grid, st);
   }
-  return a.n <= 8 ? launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 4>, grid, kThreads, 0, st, a)
-                  : launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, 0, 8>, grid, kThreads, 0, st, a);
+  constexpr bool some_bf16 = IN_BF16 || OUT_BF16;   // (fp32 to fp32 the leaving form spills: 12.8)
+  if (a.n == 2) return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, some_bf16 ? 0 : 1, some_bf16>(a, grid, st);
+  if (a.n == 3) return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, 0, false>(a, grid, st);
+  if constexpr (IN_BF16) {
+    switch (a.n) {
+      case 4: return launch_k<true, OUT_BF16, WIDE, 4, 4, 0, false>(a, grid, st);
+      case 5: return launch_k<true, OUT_BF16, WIDE, 5, 5, 0, false>(a, grid, st);
+      case 6: return launch_k<true, OUT_BF16, WIDE, 6, 6, 0, false>(a, grid, st);
+      case 7: return launch_k<true, OUT_BF16, WIDE, 7, 7, 0, false>(a, grid, st);
+      case 8: return launch_k<true, OUT_BF16, WIDE, 8, 8, 0, false>(a, grid, st);
+      default: break;
+    }
+  } else {
+    if (a.n == 4) return launch_k<false, OUT_BF16, WIDE, 0, 4, 3, false>(a, grid, st);
+    if (a.n > 4 && a.n <= 8) return launch_k<false, OUT_BF16, WIDE, 0, 8, 0, false>(a, grid, st);
+  }
+  return launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kAskLast, true>(a, grid, st);
 }
 
 template <bool IN_BF16, bool OUT_BF16>
@@ -136,7 +177,7 @@ static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, int sms,
   const unsigned long long grid = nway_grid(a, kThreads);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
   constexpr unsigned out_bytes = (IN_BF16 ? 16 : 8) * (OUT_BF16 ? 2 : 4);
-  a.ahead = ahead_ctas((a.n * 32 + out_bytes) * a.nvec, a.n * kThreads * 32);
+  a.ahead = a.n > 1 ? ahead_ctas((a.n * 32 + out_bytes) * a.nvec, a.n * kThreads * 32) : 0;
   return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, st);
 }
 

@@ -106,3 +106,21 @@ def test_large_calls_of_every_fan_in(n, dtype):
                 want += t
             assert torch.equal(out, want)
             assert bool((flat[:head] == 99).all()) and bool((flat[length + head:] == 99).all())
+
+
+@pytest.mark.parametrize("src", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("to", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 8, 9, 16])
+def test_large_averages_of_every_fan_in(n, src, to):
+    for moved in ((50 << 20) - 8192, (50 << 20) + 16384):
+        for head, tail, offset in ((0, 0, 0), (1, 3, 0), (0, 5, 4)):   # offset: results off a 32-byte boundary where that is 16 bytes
+            length = moved // (n * src.itemsize + to.itemsize) // 64 * 64 + (32 - head if head else 0) + tail
+            g = torch.Generator(device=DEV).manual_seed(length)
+            ts = [torch.randint(0, 20, (length + head,), generator=g, device=DEV).to(src)[head:] for _ in range(n)]
+            flat = torch.full((length + head + offset + 64,), 99.0, dtype=to, device=DEV)
+            out = reduce_nway_scaled(ts, scale=0.5, out=flat[head + offset:length + head + offset])
+            want = ts[0].float()
+            for t in ts[1:]:   # small whole numbers: the sum is exact, one rounding of the result
+                want += t.float()
+            assert torch.equal(out, (want * 0.5).to(to))
+            assert bool((flat[:head + offset] == 99).all()) and bool((flat[length + head + offset:] == 99).all())
