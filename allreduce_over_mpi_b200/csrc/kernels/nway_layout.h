@@ -10,6 +10,19 @@
 
 namespace ftk {
 
+// What a call does about its neighbours on the stream: its first `ahead` CTAs fetch their sources before the kernel in front
+// has ended, and those from `ask` on ask for the one behind.  Why, and why these sizes: pdl.cuh.  `moved`: the call's bytes;
+// `fetched`: bytes of sources per CTA; `ctas`: of 128 threads each.
+struct Seam {
+  uint32_t ahead, ask;
+};
+constexpr uint32_t kNoCta = ~0u;
+inline Seam seam_of(unsigned long long moved, unsigned fetched, unsigned long long ctas) {
+  if (moved < (50u << 20)) return {0, kNoCta};
+  const unsigned asking = moved < (100u << 20) ? 148 * 16 : 148 * 20;
+  return {(12u << 20) / fetched, ctas > asking ? (uint32_t)(ctas - asking) : 0};
+}
+
 // One launch covers a whole vector: the body in 32- or 16-byte vectors, and the elements in front of and behind it
 // (the edges) one by one in a CTA of their own (the last one), so that neither a ragged length nor a slice that starts
 // off a vector boundary costs a second launch or takes the rest of the vector off the vector loads.
@@ -21,15 +34,13 @@ struct NwayArgs {
   int n;
   uint16_t head, edge;        // scalar units in front of the body; in front of and behind it together
   uint8_t shift[FT_MAX_FANIN];  // shifted kernels: bytes by which source k's body lies behind a 16-byte (realign: 32-byte) boundary
-  uint32_t ahead;             // CTAs that fetch their sources ahead of the kernel before (set at the launch)
+  Seam seam;                  // set at the launch
   float scale;                // scaled kernels
-  uint64_t fill[2];           // to a size that is cheap to launch with (pdl.cuh)
+  uint32_t fill[3];           // to a size that is cheap to launch with (pdl.cuh)
 };
 
 // CTAs of a launch that covers the body once, `per_cta` vectors each, and the one for the edges.
 inline unsigned long long nway_grid(const NwayArgs& a, unsigned per_cta) { return (a.nvec + per_cta - 1) / per_cta + (a.edge != 0); }
-// CTAs of a call that moves `moved` bytes which fetch their sources ahead, `per_cta` bytes each: see pdl.cuh.
-inline uint32_t ahead_ctas(unsigned long long moved, unsigned per_cta) { return moved < (50u << 20) ? 0 : (12u << 20) / per_cta; }
 constexpr unsigned kWideThreads = 128;                  // wide and scaled kernels: a vector each
 constexpr unsigned kRealignThreads = 128, kRealignPerCta = kRealignThreads / 32 * 31;   // a warp stores 31 of the 32 it sums
 inline bool shift_long(const NwayArgs& a) { return a.nvec >= (3u << 20) / 16; }   // shifted kernel: 64 threads, two vectors each; else 128, one

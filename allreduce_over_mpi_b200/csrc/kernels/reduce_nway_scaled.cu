@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   constexpr bool early = ASK != kPlain;
   const unsigned long long i = (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
   const bool ok = i < a.nvec;
-  if (early && blockIdx.x < a.ahead && ok && !(threadIdx.x & 3))
+  if (early && blockIdx.x < a.seam.ahead && ok && !(threadIdx.x & 3))
     for (int k = 0; k < (NSRC > 0 ? NSRC : a.n); ++k) l2_ahead((const unsigned char*)a.src[k] + i * 32);
   pdl_begin();
   const auto edges = [&] {
@@ -80,10 +80,10 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
 #pragma unroll
     for (int g = 0; g < GROUP; ++g) {
       if ((LEAVE || ok) && k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
-      if (ASK == g && last) pdl_next(1);
+      if (ASK == g && last) pdl_next(blockIdx.x >= a.seam.ask);
     }
     if (early && last && a.edge && blockIdx.x == 0) edges();
-    if (ASK == kAskLast && last) pdl_next(1);
+    if (ASK == kAskLast && last) pdl_next(blockIdx.x >= a.seam.ask);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < n) {
@@ -136,7 +136,7 @@ static cudaError_t launch_k(const NwayArgs& a, unsigned grid, cudaStream_t st) {
 }
 template <bool IN_BF16, bool OUT_BF16, bool WIDE>
 static cudaError_t launch_n(const NwayArgs& a, unsigned grid, cudaStream_t st) {
-  if (!a.ahead) {
+  if (!a.seam.ahead) {
     switch (a.n) {
       case 2: return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, kPlain, true>(a, grid, st);
       case 3: return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, kPlain, true>(a, grid, st);
@@ -177,7 +177,7 @@ static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, int sms,
   const unsigned long long grid = nway_grid(a, kThreads);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
   constexpr unsigned out_bytes = (IN_BF16 ? 16 : 8) * (OUT_BF16 ? 2 : 4);
-  a.ahead = a.n > 1 ? ahead_ctas((a.n * 32 + out_bytes) * a.nvec, a.n * kThreads * 32) : 0;
+  a.seam = seam_of(a.n > 1 ? (a.n * 32 + out_bytes) * a.nvec : 0, a.n * kThreads * 32, grid);
   return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, st);
 }
 

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
   const uint32_t lane = threadIdx.x & 31, shift = a.shift[0];
   const unsigned long long i = (unsigned long long)blockIdx.x * kRealignPerCta + threadIdx.x / 32 * 31 + lane;
   const bool ok = i <= a.nvec;   // one unit more than the result has
-  if (blockIdx.x < a.ahead && ok && !(lane & 3))
+  if (blockIdx.x < a.seam.ahead && ok && !(lane & 3))
     for (int k = 0; k < a.n; ++k) l2_ahead((const unsigned char*)a.src[k] - shift + i * 32);
   pdl_begin();
   typename P::Acc al, ah;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
                      : "=r"(lo[g].x), "=r"(lo[g].y), "=r"(lo[g].z), "=r"(lo[g].w), "=r"(hi[g].x), "=r"(hi[g].y), "=r"(hi[g].z), "=r"(hi[g].w)
                      : "l"(p) : "memory");
       }
-    if (k0 + GROUP >= a.n) pdl_next(a.ahead);
+    if (k0 + GROUP >= a.n) pdl_next(a.seam.ahead);   // (all CTAs: asking is not what bounds these, fp32 x3 of 5 M 10.35 us, 10.45 from a.seam.ask on)
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < a.n) {
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
   if (lane < 31 && i < a.nvec)
     asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                  ::"l"((unsigned char*)a.dst + i * 32), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-  if (a.edge && blockIdx.x == (a.ahead ? 0 : gridDim.x - 1)) reduce_edges<POL, ScalarOp>(a);
+  if (a.edge && blockIdx.x == (a.seam.ahead ? 0 : gridDim.x - 1)) reduce_edges<POL, ScalarOp>(a);
 }
 
 template <int POL, int UNROLL, int GROUP, int THREADS>
@@ -161,7 +161,7 @@ static cudaError_t launch_t(const NwayArgs& a, bool realign, cudaStream_t st) {
     const unsigned long long grid = nway_grid(a, kRealignPerCta);
     if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
     NwayArgs b = a;
-    b.ahead = ahead_ctas((a.n + 1) * a.nvec * 32, a.n * kRealignPerCta * 32);
+    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kRealignPerCta * 32, grid);
     return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, kRealignThreads, 0, st, b)
                     : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, kRealignThreads, 0, st, b);
   }

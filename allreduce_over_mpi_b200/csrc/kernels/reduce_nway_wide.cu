@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
   using P = typename PolById<POL>::type;
   const unsigned long long i = (unsigned long long)blockIdx.x * THREADS + threadIdx.x;
   const bool ok = i < a.nvec;
-  if (EARLY && blockIdx.x < a.ahead && ok && !(threadIdx.x & 3)) {
+  if (EARLY && blockIdx.x < a.seam.ahead && ok && !(threadIdx.x & 3)) {
 #pragma unroll
     for (int k = 0; k < (NSRC > 0 ? NSRC : FT_MAX_FANIN); ++k) {
       if (NSRC == 0 && k >= a.n) break;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if (ok && g0 + g < (NSRC > 0 ? NSRC : a.n)) ld32<0>((const unsigned char*)a.src[g0 + g] + i * 32, lo[g], hi[g]);
-      if (EARLY && g == ASK && last) pdl_next(1);
+      if (EARLY && g == ASK && last) pdl_next(blockIdx.x >= a.seam.ask);
     }
     if (between && last && a.edge && blockIdx.x == 0) reduce_edges<POL, ScalarOp>(a);
 #pragma unroll
@@ -184,8 +184,8 @@ static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t
     const unsigned long long grid = nway_grid(a, kWideThreads);
     if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
     NwayArgs b = a;
-    b.ahead = ahead_ctas((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32);
-    return launch_pdl(b.ahead ? reduce_nway_wide_kernel<POL, NSRC, kWideThreads, 8, true>
+    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32, grid);
+    return launch_pdl(b.seam.ahead ? reduce_nway_wide_kernel<POL, NSRC, kWideThreads, 8, true>
                               : reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4, false>, (unsigned)grid, kWideThreads, 0, st, b);
   }
   if constexpr (TUNING) {

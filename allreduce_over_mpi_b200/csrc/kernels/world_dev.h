@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "nway_layout.h"
+
 namespace ftk {
 
 constexpr int kWorldRanks = 16;      // ranks, and entries of a program, that fit the kernel's parameters
@@ -97,9 +99,8 @@ struct WorldTreeArgs {
   void* out[kTreeRanks];
   uint64_t total_bytes, block_bytes;
   float scale;
-  uint32_t ahead;   // CTAs that fetch their sources ahead (pdl.cuh)
+  Seam seam;        // (nway_layout.h); CTAs counted along the blocks first
   uint8_t es;
-  uint8_t early;    // the next kernel may be set up early
   uint8_t streams;  // what is read, and copies that are written, leave L2 before other data
 };
 

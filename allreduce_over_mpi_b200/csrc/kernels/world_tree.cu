@@ -80,7 +80,7 @@ __device__ __forceinline__ TreePlace tree_place(const WorldTreeArgs& a, uint32_t
   return {off, full, off < end};
 }
 
-__device__ __forceinline__ bool tree_ahead(const WorldTreeArgs& a) { return blockIdx.y * gridDim.x + blockIdx.x < a.ahead; }
+__device__ __forceinline__ uint32_t tree_cta() { return blockIdx.y * gridDim.x + blockIdx.x; }
 
 // A step's code and a round's place are constants here: with all loops unrolled nothing is left of them but the additions,
 // the roundings and, of the values put aside, their registers.  A value that was just rounded is put aside in the element
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kTreeThreads, 4) world_tree_kernel(const __gri
   const unsigned char* src[N];
 #pragma unroll
   for (int k = 0; k < N; ++k) src[k] = (const unsigned char*)a.in[lo >> (3 * k) & 7] + at.off;
-  if (tree_ahead(a) && at.full && !(threadIdx.x & 3)) {
+  if (tree_cta() < a.seam.ahead && at.full && !(threadIdx.x & 3)) {
 #pragma unroll
     for (int k = 0; k < N; ++k) l2_ahead(src[k]);
   }
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kTreeThreads, 4) world_tree_kernel(const __gri
   const uint64_t policy = l2_policy(a.streams);
 #pragma unroll
   for (int k = 0; k < N; ++k) tree_load<V>(src[k], at.full, v[k], policy);
-  pdl_next(a.early);
+  pdl_next(tree_cta() >= a.seam.ask);
   if (!at.full) {
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k][0] = ld_element(src[k], ES);
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kTreeThreads) world_copy_kernel(const __grid_c
   uint4 v[V];
   const uint64_t policy = l2_policy(a.streams);
   tree_load<V>(src, at.full, v, policy);
-  pdl_next(a.early);
+  pdl_next(tree_cta() >= a.seam.ask);
   if (!at.full) v[0] = ld_element(src, a.es);
   const uint32_t mask = lo >> kTreeMask;
 #pragma unroll

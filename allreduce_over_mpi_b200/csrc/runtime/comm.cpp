@@ -512,9 +512,9 @@ cudaError_t tree_launch(const ft::WorldProgram& wp, int pol, int world, const vo
   // does not ask for its successor: both halves of two times 25 MB took 19.1 us (20.8 with fresh tensors) that way, 17.2
   // (19.0) without; of four 31.8 (33.3) and 32.7 (34.2).
   const uint64_t moved = bytes * (wp.copies ? world : phase ? world + 1 : 2 * world);
-  const uint32_t ahead = wide ? ftk::ahead_ctas(moved, world * ftk::kTreeThreads * 32) : 0;
-  a.early = ahead && !(wp.copies && world == 2);
-  a.ahead = wp.copies ? 0 : ahead;
+  const uint64_t ctas = wp.words.size() * ((block_bytes / 32 + ftk::kTreeThreads - 1) / ftk::kTreeThreads);
+  a.seam = ftk::seam_of(wide ? moved : 0, world * ftk::kTreeThreads * 32, ctas);
+  if (wp.copies) a.seam = {0, world == 2 ? ftk::kNoCta : a.seam.ask};
   return wp.copies ? ftk::launch_world_copy(a, (int)wp.words.size(), wide, st)
                    : ftk::launch_world_tree(pol, a, compiled_tree(wp, world, pol), (int)wp.words.size(), wide, st);
 }
