@@ -1,11 +1,13 @@
 // out = scale * sum_k src[k] on one GPU, fp32 accumulation, fp32 or bf16 in and out (gradient averaging with the cast
 // fused into the store).
 //
-// HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, four
-// or more sources in flight, the grid covers the vector once, dependent launch.  The unit
+// HBM bounds it, as it does reduce_nway_wide.cu, whose layout it shares: 32 bytes of every source per thread, several
+// sources in flight, the grid covers the vector once, dependent launch.  The unit
 // is 8 fp32 or 16 bf16 elements, whatever the output type, so that the source side (n streams to one) stays on 256-bit
 // loads.  fp32 -> bf16, 8 sources of 6.5 M: 38.9 us (5.7 TB/s, a strided loop with 16-byte loads of one source at a
 // time) -> 31.6 us (7.0 TB/s).
+#include <type_traits>
+
 #include "../api/flextree.h"
 #include "pdl.cuh"
 #include "reduce_nway.cuh"
@@ -36,13 +38,31 @@ __device__ __forceinline__ void store32(unsigned char* p, const uint4& a, const 
   }
 }
 
-// Element i (of a body that starts at element 0) of the result.
-template <bool IN_BF16, bool OUT_BF16>
+// Element i (of a body that starts at element 0) of the result, G sources in flight at a time; G == 1: as many as eight, the
+// rest one by one (in the kernel for nine sources and more any other form takes registers from the body).  The few edges of a
+// vector are on a call's critical path: with all but the whole eights one by one fp32 x7 of 1 M took 7.2 us, now 6.3.
+template <bool IN_BF16, bool OUT_BF16, int NSRC, int G>
 __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, float scale) {
+  using T = std::conditional_t<IN_BF16, __nv_bfloat16, float>;
+  const int n = NSRC > 0 ? NSRC : a.n;
   float acc = 0.f;
-#pragma unroll 8
-  for (int k = 0; k < a.n; ++k)
-    acc += IN_BF16 ? __bfloat162float(((const __nv_bfloat16*)a.src[k])[i]) : ((const float*)a.src[k])[i];
+#pragma unroll(G == 1 ? 8 : 1)
+  for (int k0 = 0; k0 < n; k0 += G) {
+    T v[G];
+    if (k0 + G <= n) {   // (a predicate on each load costs bf16 x8 of 6.5 M, one element off, 4 us of 29)
+#pragma unroll
+      for (int g = 0; g < G; ++g) v[g] = ((const T*)a.src[k0 + g])[i];
+#pragma unroll
+      for (int g = 0; g < G; ++g) acc += (float)v[g];
+    } else {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (k0 + g < n) v[g] = ((const T*)a.src[k0 + g])[i];
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (k0 + g < n) acc += (float)v[g];
+    }
+  }
   acc *= scale;
   if (OUT_BF16) ((__nv_bfloat16*)a.dst)[i] = __float2bfloat16_rn(acc);
   else ((float*)a.dst)[i] = acc;
@@ -50,11 +70,11 @@ __device__ __forceinline__ void scaled_element(const NwayArgs& a, long long i, f
 
 // WIDE: 256-bit accesses (every source on a 32-byte boundary, the output on one of 16 bytes for fp32 -> bf16, else
 // 32); not WIDE: 128-bit ones.  ASK: kPlain, or (calls that fetch ahead, pdl.cuh) the load of the last group behind which
-// the successor is asked for, kAskLast behind all of them; the edges are the first CTA's then.  LEAVE: a thread behind the
-// end leaves; else a predicate keeps it from each load.
+// the successor is asked for, kAskLast behind all of them; the edges are the first CTA's then.  Registers: left alone the
+// compiler takes 32 for two fp32 sources, and spills, and 72 for seven, and loads the edges one after the other.
 constexpr int kPlain = -2, kAskLast = -1;
-template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK, bool LEAVE>
-__global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a) {
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK>
+__global__ void __launch_bounds__(kThreads, ASK == kPlain ? 0 : NSRC == 2 ? 12 : NSRC == 7 ? 6 : 0) reduce_nway_scaled_kernel(const __grid_constant__ NwayArgs a) {
   constexpr int E = IN_BF16 ? 16 : 8;   // elements per thread: 32 bytes of every source
   constexpr bool early = ASK != kPlain;
   const unsigned long long i = (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
@@ -64,9 +84,9 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
   pdl_begin();
   const auto edges = [&] {
     for (int e = threadIdx.x; e < (int)a.edge; e += kThreads)
-      scaled_element<IN_BF16, OUT_BF16>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), a.scale);
+      scaled_element<IN_BF16, OUT_BF16, NSRC, (NSRC > 0 ? NSRC : early ? 1 : 8)>(a, e < a.head ? (long long)e - a.head : (long long)(a.nbody + (e - a.head)), a.scale);
   };
-  if (LEAVE && !ok) {
+  if (!ok) {
     if (!early && a.edge && blockIdx.x == gridDim.x - 1) edges();
     return;
   }
@@ -79,7 +99,7 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
     uint4 lo[GROUP], hi[GROUP];
 #pragma unroll
     for (int g = 0; g < GROUP; ++g) {
-      if ((LEAVE || ok) && k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
+      if (k0 + g < n) load32<WIDE>((const unsigned char*)a.src[k0 + g] + i * 32, lo[g], hi[g]);
       if (ASK == g && last) pdl_next(blockIdx.x >= a.seam.ask);
     }
     if (early && last && a.edge && blockIdx.x == 0) edges();
@@ -95,7 +115,6 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
         }
       }
   }
-  if (!LEAVE && !ok) return;
   constexpr int W = OUT_BF16 ? E / 2 : E;   // output words
   uint32_t o[W];
 #pragma unroll
@@ -111,13 +130,14 @@ __global__ void __launch_bounds__(kThreads) reduce_nway_scaled_kernel(const __gr
 }
 
 // Pointers no common vector fits, views summed into a result at another offset for instance: one element at a time.
-// Eight sources of 6.5 M, one element off: fp32 36.6 us (34.6 with a common vector), fp32 -> bf16 34.9 (33.1); bf16, with two
-// bytes an access, 27.4 us (15.4), 4.3 TB/s.
+// Eight sources of 6.5 M, one element off: fp32 36.3 us (33.2 with a common vector), fp32 -> bf16 34.6 (31.6); bf16, with two
+// bytes an access, 28.8 us (15.8), 4.1 TB/s.  Five sources 26.8, 25.4 and 30.8 us (62.6, 61.2 and 59.6 while only whole eights of
+// them were in flight together).
 template <bool IN_BF16, bool OUT_BF16>
 __global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __grid_constant__ NwayArgs a) {
   pdl_begin();
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.nbody; i += (unsigned long long)gridDim.x * blockDim.x)
-    scaled_element<IN_BF16, OUT_BF16>(a, (long long)i, a.scale);
+    scaled_element<IN_BF16, OUT_BF16, 0, 8>(a, (long long)i, a.scale);
 }
 
 // Calls that do not fetch ahead: two and three sources have kernels of their own (bf16 x3 of 4 M 4.0 -> 3.1 us); from four up
@@ -125,43 +145,40 @@ __global__ void __launch_bounds__(256) reduce_nway_scaled_scalar_kernel(const __
 // 12.0).  Eight sources in flight pay from nine up only: they cost registers, and those CTAs (bf16 x4 of 13 M 20.4 us with
 // four, 24.7 with eight and 256 threads; x16 of 1 M 5.0 us with eight, 5.5 with four).  Threads behind the end leave: with a
 // predicate on each load fp32 x2 -> bf16 of 8 M took 14.8 us, not 12.9.
-// Calls that do, us on fresh tensors, not / asking behind all loads with the plain form / so: fp32 x2 of 6 M 11.9 / 11.1 / 10.9,
-// -> bf16 10.0 / 9.5 / 8.8; x3 -> bf16 of 5 M 11.4 / 11.0 / 10.9, bf16 x3 of 9 M 11.8 / 11.2 / 10.3; fp32 x4 -> bf16 of 5 M
-// 14.4 / 14.2 / 13.1 (four in flight; 14.0 with eight); fp32 x7 -> bf16 of 3 M 14.5 / 14.2 / 13.4, x8 -> bf16 of 6.5 M 33.0 / 32.4 /
-// 31.6 (7.0 TB/s), x8 of 2.5 M 14.8 / 13.7 / 13.1; bf16 x4 of 8 M 13.1 / 12.7 / 11.5, x7 of 8 M 20.0 / 19.6 / 18.3, x8 of 4 M 12.1 /
-// 11.1 / 10.7 (bf16 with the fan-in known; 11.8, 19.4 and 11.7 without); bf16 x16 of 5 M 26.1 / 25.4 / 25.1.
-template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK, bool LEAVE>
+// Calls that do, up to eight sources: the fan-in known, all sources in flight, the successor asked for behind the first load.
+// From nine up groups of eight, asked for behind the last load.  Of 13 forms (fan-in known, groups of four, of eight; asking
+// behind the first, the second, all; threads behind the end leave, or not) over 64, 90 and 200 MB, fresh or all in L2, that is
+// within 1 % of the best for every type and fan-in.  us for 90 MB of fresh tensors, plain form / this:
+//   sources         2            3            4            5            6            7            8            16
+//   fp32            14.5 / 12.7  14.2 / 12.8  14.3 / 12.9  14.7 / 12.9  14.7 / 12.9  14.8 / 13.0  14.7 / 13.0  15.0 / 13.9
+//   fp32 -> bf16    14.1 / 12.9  14.2 / 12.9  14.3 / 12.9  14.9 / 13.0  14.6 / 13.0  14.8 / 13.0  14.7 / 13.0  14.9 / 14.0
+//   bf16 -> fp32    14.5 / 13.2  14.5 / 13.3  14.4 / 13.2  14.8 / 13.1  14.8 / 13.2  14.8 / 13.1  14.4 / 12.9  14.9 / 14.2
+//   bf16            14.5 / 12.7  14.3 / 12.8  14.5 / 12.9  15.1 / 13.0  14.6 / 13.0  14.8 / 13.0  14.9 / 13.0  15.0 / 14.1
+// (12.9 is 7.0 TB/s.)
+template <bool IN_BF16, bool OUT_BF16, bool WIDE, int NSRC, int GROUP, int ASK>
 static cudaError_t launch_k(const NwayArgs& a, unsigned grid, cudaStream_t st) {
-  return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, NSRC, GROUP, ASK, LEAVE>, grid, kThreads, 0, st, a);
+  return launch_pdl(reduce_nway_scaled_kernel<IN_BF16, OUT_BF16, WIDE, NSRC, GROUP, ASK>, grid, kThreads, 0, st, a);
 }
 template <bool IN_BF16, bool OUT_BF16, bool WIDE>
 static cudaError_t launch_n(const NwayArgs& a, unsigned grid, cudaStream_t st) {
   if (!a.seam.ahead) {
     switch (a.n) {
-      case 2: return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, kPlain, true>(a, grid, st);
-      case 3: return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, kPlain, true>(a, grid, st);
+      case 2: return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, kPlain>(a, grid, st);
+      case 3: return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, kPlain>(a, grid, st);
       default: break;
     }
-    return a.n <= 8 ? launch_k<IN_BF16, OUT_BF16, WIDE, 0, 4, kPlain, true>(a, grid, st)
-                    : launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kPlain, true>(a, grid, st);
+    return a.n <= 8 ? launch_k<IN_BF16, OUT_BF16, WIDE, 0, 4, kPlain>(a, grid, st) : launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kPlain>(a, grid, st);
   }
-  constexpr bool some_bf16 = IN_BF16 || OUT_BF16;   // (fp32 to fp32 the leaving form spills: 12.8)
-  if (a.n == 2) return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, some_bf16 ? 0 : 1, some_bf16>(a, grid, st);
-  if (a.n == 3) return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, 0, false>(a, grid, st);
-  if constexpr (IN_BF16) {
-    switch (a.n) {
-      case 4: return launch_k<true, OUT_BF16, WIDE, 4, 4, 0, false>(a, grid, st);
-      case 5: return launch_k<true, OUT_BF16, WIDE, 5, 5, 0, false>(a, grid, st);
-      case 6: return launch_k<true, OUT_BF16, WIDE, 6, 6, 0, false>(a, grid, st);
-      case 7: return launch_k<true, OUT_BF16, WIDE, 7, 7, 0, false>(a, grid, st);
-      case 8: return launch_k<true, OUT_BF16, WIDE, 8, 8, 0, false>(a, grid, st);
-      default: break;
-    }
-  } else {
-    if (a.n == 4) return launch_k<false, OUT_BF16, WIDE, 0, 4, 3, false>(a, grid, st);
-    if (a.n > 4 && a.n <= 8) return launch_k<false, OUT_BF16, WIDE, 0, 8, 0, false>(a, grid, st);
+  switch (a.n) {
+    case 2: return launch_k<IN_BF16, OUT_BF16, WIDE, 2, 2, 0>(a, grid, st);
+    case 3: return launch_k<IN_BF16, OUT_BF16, WIDE, 3, 3, 0>(a, grid, st);
+    case 4: return launch_k<IN_BF16, OUT_BF16, WIDE, 4, 4, 0>(a, grid, st);
+    case 5: return launch_k<IN_BF16, OUT_BF16, WIDE, 5, 5, 0>(a, grid, st);
+    case 6: return launch_k<IN_BF16, OUT_BF16, WIDE, 6, 6, 0>(a, grid, st);
+    case 7: return launch_k<IN_BF16, OUT_BF16, WIDE, 7, 7, 0>(a, grid, st);
+    case 8: return launch_k<IN_BF16, OUT_BF16, WIDE, 8, 8, 0>(a, grid, st);
+    default: return launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kAskLast>(a, grid, st);
   }
-  return launch_k<IN_BF16, OUT_BF16, WIDE, 0, 8, kAskLast, true>(a, grid, st);
 }
 
 template <bool IN_BF16, bool OUT_BF16>

@@ -124,3 +124,21 @@ def test_large_averages_of_every_fan_in(n, src, to):
                 want += t.float()
             assert torch.equal(out, (want * 0.5).to(to))
             assert bool((flat[:head + offset] == 99).all()) and bool((flat[length + head + offset:] == 99).all())
+
+
+@pytest.mark.parametrize("src", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("to", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [2, 4, 6, 7, 8, 12])
+def test_averages_with_edges_of_every_length(n, src, to):
+    """The edges are summed by code of their own: from none to a line in front and behind, in calls of both kinds."""
+    unit = 32 // src.itemsize
+    for body in (3 * unit, (51 << 20) // (n * src.itemsize + to.itemsize)):
+        for head, tail in ((0, 1), (1, 0), (unit - 1, unit - 1), (unit // 2, 3), (5, 2 * unit + 1)):
+            length = body // unit * unit + head + tail
+            g = torch.Generator(device=DEV).manual_seed(length)
+            ts = [torch.randint(0, 20, (length + 7,), generator=g, device=DEV).to(src)[7:] for _ in range(n)]
+            flat = torch.full((length + 64,), 99.0, dtype=to, device=DEV)
+            out = reduce_nway_scaled(ts, scale=0.25, out=flat[7:length + 7])
+            want = torch.stack(ts).float().sum(0)   # small whole numbers: the sum is exact, one rounding of the result
+            assert torch.equal(out, (want * 0.25).to(to))
+            assert bool((flat[:7] == 99).all()) and bool((flat[length + 7:] == 99).all())
