@@ -101,7 +101,21 @@ struct WorldTreeArgs {
   float scale;
   Seam seam;        // (nway_layout.h); CTAs counted along the blocks first
   uint8_t es;
-  uint8_t streams;  // what is read, and copies that are written, leave L2 before other data
+  uint8_t streams;  // what is read, and by a gather written, leaves L2 before other data (halves_stream)
 };
+
+// Whether a half of an all-reduce tells L2 (126 MB) that what it reads, and as a gather what it writes, may leave first.
+// `copies`: bytes of all ranks' copies.
+// What the reduce-scatter leaves is what the gather reads; everything else it touches has served.  Worth saying only where the
+// copies take a good part of L2: both halves of four ranks of 6 MB took 7.0 us, 7.6 with it.
+// The gather's copies are read by whoever comes behind, and are found in L2 as long as that holds them all: with an update of
+// the owned blocks between the halves and a sum over every copy behind them, us with neither / the reduce-scatter / both saying it:
+//   copies   58 MB               84 MB               100 MB              112 MB              128 MB
+//   2 ranks  57.6 / 57.1 / 59.9  71.7 / 70.5 / 73.1  86.8 / 82.1 / 80.1  96.3 / 88.1 / 86.1  107.7/100.9/ 95.6
+//   4 ranks  74.0 / 73.7 / 80.6  90.8 / 88.8 / 93.1  103.2/ 98.1/100.1   112.9/108.1/104.7   123.7/116.1/112.3
+//   8 ranks  115.6/114.8/121.4   129.5/126.8/135.9   139.9/136.4/141.4   151.1/143.9/145.6   163.1/155.8/153.7
+// The halves alone, nobody between or behind them, 4 ranks: 19.7 / 19.7 / 18.4, 27.8 / 27.2 / 26.0, 32.9 / 32.8 / 30.6, 36.9 / 36.1 /
+// 34.4, 43.0 / 42.1 / 39.5.
+inline bool halves_stream(bool gather, uint64_t copies) { return copies >= (gather ? 100u << 20 : 32u << 20); }
 
 }  // namespace ftk

@@ -496,13 +496,8 @@ cudaError_t tree_launch(const ft::WorldProgram& wp, int pol, int world, const vo
                         uint64_t block_bytes, uint32_t es, float scale, int phase, cudaStream_t st) {
   ftk::WorldTreeArgs a;
   ft::fill_tree_args(wp, world, in, out, &a);
-  // The halves of an all-reduce: what the reduce-scatter leaves is what the all-gather reads, everything else either of them
-  // touches has served.  Both calls, fp32 25 MB a rank, us, three sets of tensors in turn (twelve, so that nothing is left
-  // from the time before): flat of eight 71.7 (71.7) -> 65.2 (66.2), 2*4 80.7 (80.7) -> 75.3 (75.3), flat of four 35.6 (35.6)
-  // -> 32.8 (34.5), of two 18.9 (19.0) -> 17.0 (19.2).  Worth saying only where a world's copies take a good part of L2 (126
-  // MB): four of 6 MB, three sets of which stay there, took 7.6 instead of 7.0.  An all-reduce has nothing to keep: 63.2 -> 63.6.
-  // (All before fetching ahead, with which these are: eight 64.4 (65.1), 2*4 73.4 (73.6), four 32.0 (33.5), two 17.2 (19.1).)
-  a.streams = phase != 0 && bytes * world >= (32u << 20);
+  // (an all-reduce has nothing to keep: eight ranks of 25 MB 63.2 us without, 63.6 with it)
+  a.streams = phase != 0 && ftk::halves_stream(wp.copies, bytes * world);
   a.total_bytes = bytes;
   a.block_bytes = block_bytes;
   a.es = (uint8_t)es;

@@ -745,9 +745,16 @@ static void seams() {
     }
 }
 
+// Gathered copies that L2 holds stay there for whoever reads them.
+static void halves_in_l2() {
+  for (uint64_t mb : {33, 58, 64, 84, 99}) EXPECT(!ftk::halves_stream(true, mb << 20) && ftk::halves_stream(false, mb << 20));
+  for (uint64_t mb : {1, 24, 31}) EXPECT(!ftk::halves_stream(true, mb << 20) && !ftk::halves_stream(false, mb << 20));
+  for (uint64_t mb : {126, 200, 4000}) EXPECT(ftk::halves_stream(true, mb << 20) && ftk::halves_stream(false, mb << 20));
+}
+
 int main(int argc, char** argv) {
   const bool threads = argc > 1 && !std::strcmp(argv[1], "threads");
-  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); nway_layouts(); seams(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
+  if (!threads) { proc_world_forked(); plans_and_snapshot(); device_tables(); world_programs(); nway_layouts(); seams(); halves_in_l2(); heap_offsets(); enumerators_and_models(); policy_and_json(); fd_passing(); }
   world_program_cache();
   thread_world(false);
   thread_world_phases();

@@ -70,6 +70,39 @@ def test_chain_of_collectives(shape):
     w.close()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", ["2", "4", "2*4", "2*2*2"])
+@pytest.mark.parametrize("copies", [64 << 20, 110 << 20], ids=["64MB", "110MB"])
+def test_chain_of_float_collectives(shape, dtype, copies):
+    """As above on the compiled programs, with the halves' choice of what leaves L2 for copies that it holds and that it does
+    not, and a reader behind the gather.  Small whole numbers times a power of two: exact, whatever the order."""
+    world = {"2": 2, "4": 4, "2*4": 8, "2*2*2": 8}[shape]
+    count = copies // dtype.itemsize // world + 5
+    w = LocalWorld(world, heap_bytes=count * dtype.itemsize + (1 << 20), staging_bytes=1 << 20)
+    ts = [c.alloc(count, dtype) for c in w.ranks]
+    g = torch.Generator(device=DEV).manual_seed(3)
+    want = torch.zeros(count, device=DEV)
+    for t in ts:
+        h = torch.randint(-8, 8, (count,), generator=g, device=DEV).to(dtype)
+        t.copy_(h)
+        want += h.float()
+    read = []
+    for step in range(4):   # every rank's copy is the sum of all, so each call multiplies by the world
+        w.all_reduce(ts, shape=shape)
+        owned = w.reduce_scatter(ts, shape=shape)
+        for blocks in owned:
+            for b in blocks if isinstance(blocks, (list, tuple)) else [blocks]:
+                b.mul_(0.5)
+        w.all_gather(ts, shape=shape)
+        read.append(reduce_nway(ts[:2]))
+    torch.cuda.synchronize()
+    for step in range(4):
+        want *= world * 0.5 * (world if step else 1)
+        assert torch.equal(read[step].float(), want * 2)
+    assert all(torch.equal(t.float(), want) for t in ts)
+    w.close()
+
+
 def test_two_streams():
     """Each stream's chain for itself, both at once."""
     a, b = vectors(4, (0, 0, 0, 0), seed=5), vectors(4, (0, 0, 0, 0), seed=6)
