@@ -11,6 +11,9 @@
 // them, with the same number of turns each.  Two inputs of 16 KB took 4.8 us with four CTAs of 256 threads and take 3.9 with
 // one; of 64 KB 8.8 -> 6.9, of 256 KB 16.9 -> 14.8 (16.1 with two vectors a thread); eight of 8 KB 5.8 -> 4.8, of 64 KB
 // 17.3 -> 15.2, of 1 MB 173.2 -> 171.0.
+// The second CTA costs 1.1 us, so up to 32 KB of two to four inputs one CTA takes two vectors a thread: two inputs of 20 KB 4.8
+// us (5.4 with two CTAs of 1024, 5.4 with five of 256), of 32 KB 5.2 (5.9 and 5.9), four of 24 KB 6.4 (6.9 and 7.0).  More inputs
+// would need twice the registers.
 // Where the host memory is near, 100 KB of loads in flight fill the link; from a farther socket 256 KB reach 41 GB/s only
 // (49 with 1 MB).  So from three turns up a thread takes two vectors at a time of two or three inputs: 384 KB in flight at
 // least.  Many CTAs make reads and writes collide (592 of 256 threads 771 us).
@@ -93,7 +96,9 @@ static cudaError_t launch_u(const HostPrefixArgs& a, cudaStream_t st) {
 }
 template <int POL>
 static cudaError_t launch_t(const HostPrefixArgs& a, cudaStream_t st) {
-  return a.n_in <= 3 && a.bytes > 3 * kHostCtas * kHostThreads * 16 ? launch_u<POL, 2>(a, st) : launch_u<POL, 1>(a, st);
+  constexpr uint64_t turn = kHostThreads * 16;   // bytes of a vector that a CTA takes at a time
+  const bool one_cta = a.n_in <= 4 && a.bytes > turn && a.bytes <= 2 * turn;   // instead of two
+  return one_cta || (a.n_in <= 3 && a.bytes > 3 * kHostCtas * turn) ? launch_u<POL, 2>(a, st) : launch_u<POL, 1>(a, st);
 }
 
 cudaError_t launch_host_prefix(int pol, const HostPrefixArgs& a, cudaStream_t st) {

@@ -78,3 +78,24 @@ def test_cuts_of_the_pcie_kernel(dtype, n):
             assert torch.equal(flat[1][:length], reduce_nway([v.to(DEV) for v in vecs]).cpu()), (nvec, tail)
             assert not any(f[length:].any() for f in flat)
     pipe.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.uint8])
+@pytest.mark.parametrize("n", [1, 2, 4, 5])
+def test_two_vectors_a_thread_in_one_cta(dtype, n):
+    """Between one and two vectors for each thread of a CTA: the second ones from none to all, with elements behind them, in
+    place too."""
+    per = 16 // dtype.itemsize
+    pipe = HostReducePipeline(device=DEV, max_inputs=n, max_outputs=2)
+    for nvec in (1024, 1025, 1055, 1056, 1057, 1536, 2015, 2016, 2017, 2047, 2048):
+        for tail in (0, 1, per - 1):
+            length = nvec * per + tail
+            g = torch.Generator().manual_seed(length)
+            vecs = [torch.randint(0, 25, (length,), generator=g).to(dtype).pin_memory() for _ in range(n)]
+            want = [reduce_nway([v.to(DEV) for v in vecs[:f]]).cpu() for f in (1, n)]
+            flat = torch.zeros(length + 32, dtype=dtype, pin_memory=True)
+            pipe.run(vecs, [1, n], [flat[:length], vecs[n - 1]])
+            torch.cuda.synchronize()
+            assert torch.equal(flat[:length], want[0]) and torch.equal(vecs[n - 1], want[1]), (nvec, tail)
+            assert not flat[length:].any()
+    pipe.close()
