@@ -1,6 +1,7 @@
 // What the host hands to the kernels that run one pass over the copies of all ranks of a world that lives on one device:
-// world_tree_kernel and world_copy_kernel (world_tree.cu) for floating sums and copies of up to eight ranks,
-// world_reduce_kernel (world_reduce.cu), which interprets its program, for the rest.  Programs are built by planner/world_program.hpp.
+// of up to eight ranks world_tree_kernel (world_tree.cu) for floating sums, and for integers wherever whole sums are stored (a
+// flat sum then, whatever the plan), and world_copy_kernel for copies; for the rest world_reduce_kernel (world_reduce.cu), which
+// interprets its program.  Programs are built by planner/world_program.hpp.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>

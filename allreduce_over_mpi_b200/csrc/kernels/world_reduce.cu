@@ -4,8 +4,9 @@
 // itself is 16 times a rank's bytes (every input read once, every result written once), and that is what this kernel
 // moves.  HBM bounds it from a few MB up, the launch below.  A thread takes 16 or 32 bytes of one block from every
 // rank, eight loads in flight, evaluates the block's program (planner/world_program.hpp: the plan's own order of
-// additions and roundings) in registers and stores the copies that change.  The program sits in the kernel's
-// parameters, so nothing has to be fetched before the first load; all its branches are uniform across the grid's CTA.
+// additions and roundings) in registers and stores the copies that change.  The program is looked up in the kernel's
+// parameters, in chains of a few constant-cache misses before the first load (which is why the programs of up to eight ranks
+// are compiled in, world_tree.cu); all its branches are uniform across a CTA.
 #include <algorithm>
 
 #include "../api/flextree.h"
@@ -40,8 +41,7 @@ __device__ __forceinline__ void world_store(unsigned char* p, bool ok, const uin
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q st.global.v4.u32 [%0], {%1,%2,%3,%4};\n\t}"
                  ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"((uint32_t)ok) : "memory");
 }
-// blockIdx.y: the program entry.  V: 16-byte vectors per thread and rank; DEPTH: accumulators the program puts aside
-// (0: one flat sum, no step but the first does more than add); G: steps whose loads are in flight together; RANKS: size
+// blockIdx.y: the program entry.  V: 16-byte vectors per thread and rank; DEPTH: accumulators the program may put aside; G: steps whose loads are in flight together; RANKS: size
 // of the parameters.  At most 128 registers, so that four CTAs of 128 threads fit an SM: with 144 and CTAs of 256 only
 // one did, and the 2*4 tree over eight bf16 buckets of 25 MB took 87 us instead of 66 (6.4 TB/s).
 template <int POL, int V, int DEPTH, int G, int RANKS>
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
   const bool full = i < whole;
   const uint64_t off = lo + (full ? i * (V * 16) : whole * (V * 16) + (i - whole) * a.es);
   if (off >= end) return;
-  typename P::Acc acc[V], aside[DEPTH > 0 ? DEPTH : 1][V];
+  typename P::Acc acc[V], aside[DEPTH][V];
   for (int k0 = 0; k0 < nsteps; k0 += G) {
     uint4 v[G][V];
 #pragma unroll
@@ -73,22 +73,19 @@ __global__ void __launch_bounds__(kWorldThreads, 4) world_reduce_kernel(const __
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if (k0 + g >= nsteps) break;
-      const uint32_t code = DEPTH > 0 ? a.code[first + k0 + g] : (k0 + g == 0);
+      const uint32_t code = a.code[first + k0 + g];
       if (code & 1) {
 #pragma unroll
         for (int h = 0; h < V; ++h) {
-          if (DEPTH > 0) {   // (the first step puts aside a value nothing takes back)
 #pragma unroll
-            for (int d = DEPTH - 1; d > 0; --d) aside[d][h] = aside[d - 1][h];
-            aside[0][h] = acc[h];
-          }
+          for (int d = DEPTH - 1; d > 0; --d) aside[d][h] = aside[d - 1][h];
+          aside[0][h] = acc[h];   // (the first step puts aside a value nothing takes back)
           P::init(acc[h], v[g][h]);
         }
       } else {
 #pragma unroll
         for (int h = 0; h < V; ++h) P::add(acc[h], v[g][h]);
       }
-      if (DEPTH == 0) continue;
       const int rounds = (int)(code >> 2);
       for (int r = 0; r < rounds; ++r) {
         uint4 w[V];
@@ -134,9 +131,8 @@ static cudaError_t launch_t(const WorldArgs<RANKS>& a, int entries, cudaStream_t
   return launch_pdl(world_reduce_kernel<POL, V, DEPTH, G, RANKS>, dim3((unsigned)per, (unsigned)entries), kWorldThreads, 0, st, a);
 }
 
-// Of integers of up to eight ranks only the reduce-scatters of trees come here (one word a value, so the deepest form costs
-// nothing: eight int32 buckets of 25 MB flat 63.8 us, 2*4 64.3).  From nine ranks up, and for a floating sum of fewer
-// whose program is not compiled in, every program runs the deepest form: sixteen fp32 buckets flat 130 us (6.5 TB/s), 4*4
+// Of up to eight ranks only the integers' reduce-scatters of trees come here (one word a value, so the deepest form costs
+// nothing: eight int32 buckets of 25 MB flat 63.8 us, 2*4 64.3).  From nine ranks up every program runs the deepest form: sixteen fp32 buckets flat 130 us (6.5 TB/s), 4*4
 // 132, 2*2*2*2 141 (6.0 TB/s), in bf16 139, 151 and 166 us.
 template <int POL, int RANKS>
 static cudaError_t launch_r(const WorldArgs<RANKS>& a, int entries, bool wide, cudaStream_t st) {

@@ -1224,10 +1224,12 @@ int ft_local_world_run(ft_comm* const* comms, int n, const void* const* in, void
   if (!we) return FT_ERR_NOT_AVAILABLE;
   const ft::WorldProgram* wp = &we->program;
   if (algo == FT_ALGO_LL && nw > 0 && !ll_tree_fits(c, Prepared{pol, es, bytes, resident != 0}, count, we->nslots)) return FT_ERR_NOT_AVAILABLE;
-  // the kernels with programs compiled in where there is one; of the rest, small worlds' integers by the smaller parameters
-  const bool compiled = wp->copies || compiled_tree(*wp, n, pol) >= 0, small = n <= 8 && !is_floating(pol);
+  // The kernels with programs compiled in where there is one, as for every floating sum of a small world; of the rest, small
+  // worlds by the smaller parameters.
+  const bool compiled = wp->copies || compiled_tree(*wp, n, pol) >= 0, small = n <= 8;
   const int cap = small ? 8 : ftk::kWorldRanks;
-  if (!compiled && (wp->depth > (small ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap)) return FT_ERR_NOT_AVAILABLE;
+  if (!compiled && ((small && is_floating(pol)) || wp->depth > (small ? 2 : 3) || (int)wp->entries.size() > cap || (int)wp->steps.size() > cap * cap))
+    return FT_ERR_NOT_AVAILABLE;
   if (wp->entries.empty()) return FT_OK;
   const uint64_t block_bytes = blocks ? pick_block_elems(count, n, es) * es : (bytes + 15) / 16 * 16;
   // copies move raw words: 16-bit floats do not pass through fp32
