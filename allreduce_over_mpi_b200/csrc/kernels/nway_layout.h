@@ -24,8 +24,9 @@ inline Seam seam_of(unsigned long long moved, unsigned fetched, unsigned long lo
 }
 
 // One launch covers a whole vector: the body in 32- or 16-byte vectors, and the elements in front of and behind it
-// (the edges) one by one in a CTA of their own (the last one), so that neither a ragged length nor a slice that starts
-// off a vector boundary costs a second launch or takes the rest of the vector off the vector loads.
+// (the edges) one by one in a CTA of their own (the last one; in calls that fetch ahead by the first CTA, beside its part of
+// the body), so that neither a ragged length nor a slice that starts off a vector boundary costs a second launch or takes
+// the rest of the vector off the vector loads.
 struct NwayArgs {
   const void* src[FT_MAX_FANIN];  // start of the body in every source
   void* dst;
@@ -39,8 +40,9 @@ struct NwayArgs {
   uint32_t fill[3];           // to a size that is cheap to launch with (pdl.cuh)
 };
 
-// CTAs of a launch that covers the body once, `per_cta` vectors each, and the one for the edges.
-inline unsigned long long nway_grid(const NwayArgs& a, unsigned per_cta) { return (a.nvec + per_cta - 1) / per_cta + (a.edge != 0); }
+// CTAs of a launch that covers the body once, `per_cta` vectors each; and with the one for the edges.
+inline unsigned long long body_ctas(const NwayArgs& a, unsigned per_cta) { return (a.nvec + per_cta - 1) / per_cta; }
+inline unsigned long long nway_grid(const NwayArgs& a, unsigned per_cta) { return body_ctas(a, per_cta) + (a.edge && !a.seam.ahead); }
 constexpr unsigned kWideThreads = 128;                  // wide and scaled kernels: a vector each
 constexpr unsigned kRealignThreads = 128, kRealignPerCta = kRealignThreads / 32 * 31;   // a warp stores 31 of the 32 it sums
 inline bool shift_long(const NwayArgs& a) { return a.nvec >= (3u << 20) / 16; }   // shifted kernel: 64 threads, two vectors each; else 128, one

@@ -18,7 +18,7 @@ cudaError_t launch_shift(int pol, const NwayArgs& a, bool realign, cudaStream_t 
 cudaError_t launch_scaled(bool in_bf16, bool out_bf16, const NwayArgs& a, unsigned long long len, int sms, cudaStream_t st);
 
 #ifdef __CUDACC__
-// The edges of the vector, by the CTA the launch adds for them (less than 160 bytes: one or two units a thread).
+// The edges of the vector, by the CTA the launch adds for them, or the first one (less than 160 bytes: one or two units a thread).
 template <int POL, template <int> class Scalar>
 __device__ __forceinline__ void reduce_edges(const NwayArgs& a) {
   using S = Scalar<POL>;

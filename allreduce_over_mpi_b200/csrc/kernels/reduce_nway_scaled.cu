@@ -191,10 +191,10 @@ static cudaError_t launch_t(const NwayArgs& in, unsigned long long len, int sms,
     a.nbody = len;
     return launch_pdl(reduce_nway_scaled_scalar_kernel<IN_BF16, OUT_BF16>, (unsigned)(want < cap ? want : cap), 256, 0, st, a);
   }
+  constexpr unsigned out_bytes = (IN_BF16 ? 16 : 8) * (OUT_BF16 ? 2 : 4);
+  a.seam = seam_of(a.n > 1 ? (a.n * 32 + out_bytes) * a.nvec : 0, a.n * kThreads * 32, body_ctas(a, kThreads));
   const unsigned long long grid = nway_grid(a, kThreads);
   if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-  constexpr unsigned out_bytes = (IN_BF16 ? 16 : 8) * (OUT_BF16 ? 2 : 4);
-  a.seam = seam_of(a.n > 1 ? (a.n * 32 + out_bytes) * a.nvec : 0, a.n * kThreads * 32, grid);
   return wide ? launch_n<IN_BF16, OUT_BF16, true>(a, (unsigned)grid, st) : launch_n<IN_BF16, OUT_BF16, false>(a, (unsigned)grid, st);
 }
 

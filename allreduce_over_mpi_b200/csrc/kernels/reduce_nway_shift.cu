@@ -158,10 +158,10 @@ static cudaError_t launch_t(const NwayArgs& a, cudaStream_t st) {
 template <int POL>
 static cudaError_t launch_t(const NwayArgs& a, bool realign, cudaStream_t st) {
   if (realign) {
-    const unsigned long long grid = nway_grid(a, kRealignPerCta);
-    if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
     NwayArgs b = a;
-    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kRealignPerCta * 32, grid);
+    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kRealignPerCta * 32, body_ctas(a, kRealignPerCta));
+    const unsigned long long grid = nway_grid(b, kRealignPerCta);
+    if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
     return a.n <= 8 ? launch_pdl(reduce_nway_realign_kernel<POL, 4>, (unsigned)grid, kRealignThreads, 0, st, b)
                     : launch_pdl(reduce_nway_realign_kernel<POL, 8>, (unsigned)grid, kRealignThreads, 0, st, b);
   }

@@ -181,10 +181,10 @@ static cudaError_t launch_cfg(const NwayArgs& a, int code, int sms, cudaStream_t
   const int t = code % 10;
   if (t != 0 && t != 1 && t != 3) return cudaErrorInvalidValue;
   if (code == 0) {
-    const unsigned long long grid = nway_grid(a, kWideThreads);
-    if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
     NwayArgs b = a;
-    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32, grid);
+    b.seam = seam_of((a.n + 1) * a.nvec * 32, a.n * kWideThreads * 32, body_ctas(a, kWideThreads));
+    const unsigned long long grid = nway_grid(b, kWideThreads);
+    if (grid > 0x7fffffffull || grid == 0) return cudaErrorInvalidValue;
     return launch_pdl(b.seam.ahead ? reduce_nway_wide_kernel<POL, NSRC, kWideThreads, 8, true>
                               : reduce_nway_wide_kernel<POL, NSRC, kWideThreads, NSRC == 0 ? 8 : 4, false>, (unsigned)grid, kWideThreads, 0, st, b);
   }

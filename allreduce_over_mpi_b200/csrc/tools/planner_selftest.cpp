@@ -631,6 +631,8 @@ struct NwayReplay {
   // wide and scaled kernels: 32 bytes of every source a thread, `out` bytes of the result.  `first`: the edges are the
   // first CTA's, as in calls that fetch ahead, else the last one's
   void wide(size_t load, size_t out, size_t store, bool first = false) {
+    first = first && a.nvec;   // (such calls are long)
+    a.seam.ahead = first;
     const unsigned long long grid = ftk::nway_grid(a, ftk::kWideThreads);
     need(grid > 0);
     for (unsigned long long cta = 0; cta < grid; ++cta)
@@ -646,6 +648,7 @@ struct NwayReplay {
       }
   }
   void realign(bool first = false) {
+    a.seam.ahead = first;
     const unsigned long long grid = ftk::nway_grid(a, ftk::kRealignPerCta);
     need(grid > 0 && a.shift[0] > 0 && a.shift[0] < 32);
     for (unsigned long long cta = 0; cta < grid; ++cta)
@@ -692,13 +695,13 @@ static bool replay_nway(const ftk::NwayArgs& in, size_t unit, size_t len, bool f
   else { ++nway_kernel_seen[2]; ftk::layout_shift(in, len * unit, unit, &r.a); r.shift(); }
   return r.done();
 }
-static bool replay_scaled(const ftk::NwayArgs& in, bool in_bf16, bool out_bf16, size_t len) {
+static bool replay_scaled(const ftk::NwayArgs& in, bool in_bf16, bool out_bf16, size_t len, bool first) {
   const size_t is = in_bf16 ? 2 : 4, os = out_bf16 ? 2 : 4;
   NwayReplay r{in, in, is, os, len, std::vector<uint8_t>(len * os)};
   bool wide = false;
   if (!ftk::layout_scaled(in, len, in_bf16, out_bf16, &r.a, &wide)) return true;   // an element at a time
   ++nway_kernel_seen[wide ? 3 : 4];
-  r.wide(wide ? 32 : 16, 32 / is * os, wide && 32 / is * os >= 32 ? 32 : 16);
+  r.wide(wide ? 32 : 16, 32 / is * os, wide && 32 / is * os >= 32 ? 32 : 16, first);
   return r.done();
 }
 static void nway_layouts() {
@@ -719,7 +722,7 @@ static void nway_layouts() {
           if (unit != 2 && unit != 4) continue;
           for (bool out_bf16 : {false, true})
             if (d % (out_bf16 ? 2 : 4) == 0)
-              for (size_t len : lens) EXPECT(replay_scaled(in, unit == 2, out_bf16, len));
+              for (size_t len : lens) EXPECT(replay_scaled(in, unit == 2, out_bf16, len, false) && replay_scaled(in, unit == 2, out_bf16, len, true));
         }
     for (size_t bytes : {(3u << 20) - 40, 3u << 20, (3u << 20) + 56}) {   // where the shifted kernel changes its CTAs
       ftk::NwayArgs in{};
