@@ -3,7 +3,7 @@ read of one another's results, and write over one another's sources, comes out a
 import pytest
 import torch
 
-from allreduce_over_mpi_b200.ops import reduce_nway, reduce_nway_scaled
+from allreduce_over_mpi_b200.ops import HostReducePipeline, reduce_nway, reduce_nway_scaled
 from allreduce_over_mpi_b200.parallel.comm import LocalWorld
 
 pytestmark = pytest.mark.gpu
@@ -175,3 +175,112 @@ def test_averages_with_edges_of_every_length(n, src, to):
             want = torch.stack(ts).float().sum(0)   # small whole numbers: the sum is exact, one rounding of the result
             assert torch.equal(out, (want * 0.25).to(to))
             assert bool((flat[:7] == 99).all()) and bool((flat[length + 7:] == 99).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float64, torch.uint8, torch.int64])
+@pytest.mark.parametrize("n", [1, 2, 5, 8, 9, 16])
+def test_large_realigned_sums(n, dtype):
+    """Sources at one offset, the result at another, ragged, just below and above the size from which calls fetch ahead."""
+    es = dtype.itemsize
+    for moved in ((50 << 20) - 8192, (50 << 20) + 8192, 58 << 20):
+        for src, dst, tail in ((1, 0, 0), (0, 1, 5), (16 // es + 1, 2, 1)):
+            length = moved // ((n + 1) * es) // 32 * 32 + tail
+            g = torch.Generator(device=DEV).manual_seed(length)
+            ts = [torch.randint(0, 15, (length + src,), generator=g, device=DEV).to(dtype)[src:] for _ in range(n)]
+            flat = torch.full((length + dst + 64,), 99, dtype=dtype, device=DEV)
+            out = reduce_nway(ts, out=flat[dst:length + dst])
+            want = ts[0].clone()
+            for t in ts[1:]:   # small whole numbers: exact in every type, in any order
+                want += t
+            assert torch.equal(out, want)
+            assert bool((flat[:dst] == 99).all()) and bool((flat[length + dst:] == 99).all())
+
+
+@pytest.mark.parametrize("offsets", [(0, 0, 0, 0), (1, 1, 1, 0)], ids=["wide", "realign"])
+def test_chain_in_a_graph(offsets):
+    """In a captured graph the request becomes a programmatic edge between the nodes."""
+    ring, want = vectors(4, offsets, seed=9), vectors(4, offsets, seed=9)
+    stream = torch.cuda.Stream()
+
+    def row(ts, total):
+        for step in range(12):
+            k = [(step + j) % 4 for j in range(4)]
+            total(ts[k[0]], ts[k[1]], ts[k[2]], ts[k[3]])
+
+    with torch.cuda.stream(stream):
+        row(vectors(4, offsets), lambda a, b, c, d: reduce_nway([a, b, c], out=d))   # what is made on first use is made
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            row(ring, lambda a, b, c, d: reduce_nway([a, b, c], out=d))
+        for _ in range(3):
+            graph.replay()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        row(want, lambda a, b, c, d: d.copy_(a + b + c))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(ring, want))
+
+
+@pytest.mark.parametrize("graph", [False, True], ids=["stream", "graph"])
+def test_kernels_that_ask_one_after_the_other(graph):
+    """Every kernel that asks early in front of and behind the others, the host's vectors among them: sums, sums off the
+    sources' boundary, averages, and the collectives' programs and copies, each reading what the one before it wrote."""
+    world = LocalWorld(4, heap_bytes=N * 4 + (1 << 20), staging_bytes=1 << 20)
+    ts = [c.alloc(N, torch.float32) for c in world.ranks]
+    host = [torch.randint(0, 9, (70_001,)).float().pin_memory() for _ in range(3)]
+    out = torch.empty(70_001).pin_memory()
+    pipe = HostReducePipeline(device=DEV, max_inputs=3, max_outputs=1)
+
+    def start():
+        g = torch.Generator(device=DEV).manual_seed(2)
+        return [torch.randint(-4, 5, (N,), generator=g, device=DEV).float() for _ in range(10)]
+
+    def row(v, total, average, collective, half, hosts):   # values stay below 2^22 of their smallest step: exact in any order
+        a, b, c, d, e, f = v[:6]
+        for _ in range(2):
+            total([a, b, c], d)
+            total([d[1:], b[1:]], e[:-1])
+            average([d, e, a], 0.5, f)
+            total([f, d], v[6])
+            collective(v[6:])
+            half(v[6:])
+            hosts()
+            total([v[6], v[9], f], a)
+            average([a, d], 0.25, b)
+
+    def ours(v):
+        row(v, lambda x, o: reduce_nway(x, out=o), lambda x, s, o: reduce_nway_scaled(x, scale=s, out=o),
+            lambda x: world.all_reduce(x, shape="2*2"), lambda x: (world.reduce_scatter(x, shape="4"), world.all_gather(x, shape="4")),
+            lambda: pipe.run(host, [3], [out]))
+
+    def summed(x):
+        s = x[0] + x[1] + x[2] + x[3]
+        for t in x:
+            t.copy_(s)
+
+    got, want = start(), start()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        mine = got[:6] + ts
+        if graph:
+            for t, h in zip(ts, got[6:]):
+                t.copy_(h)
+            ours([v.clone() for v in got[:6]] + ts)   # what is made on first use is made
+            stream.synchronize()
+            recorded = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(recorded, stream=stream):
+                ours(mine)
+        for t, h in zip(ts, got[6:]):
+            t.copy_(h)
+        if graph:
+            recorded.replay()
+        else:
+            ours(mine)
+    torch.cuda.synchronize()
+    row(want, lambda x, o: o.copy_(sum(x[1:], x[0])), lambda x, s, o: o.copy_(sum(x[1:], x[0]) * s), summed, summed, lambda: None)
+    assert all(torch.equal(x, y) for x, y in zip(mine, want))
+    assert torch.equal(out, host[0] + host[1] + host[2])
+    world.close()
+    pipe.close()
