@@ -104,7 +104,8 @@ __device__ __forceinline__ void join32(const uint32_t (&lo)[8], const uint32_t (
 // A warp sums 32 units of 32 bytes on the sources' boundaries and stores the 31 units of the result between them; the
 // next warp sums the last one again (a hit in L2).  a.nvec: units of the result; shift[0]: bytes by which it lies behind
 // the sources' boundaries.  bf16 x8 of 4 M, sources one element off: 14.3 us by the kernel above, 11.2 here, 10.1 in a row
-// with fetching ahead (pdl.cuh); the edges are the first CTA's then, which is not the last to end.
+// with fetching ahead (pdl.cuh); the edges are the first CTA's then, which is not the last to end.  All CTAs ask for the
+// successor: they do enough for that not to count (fp32 x3 of 5 M 10.35 us, 10.45 if only the last ones do).
 template <int POL, int GROUP>
 __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(kRealignThreads) reduce_nway_realign_kernel(co
                      : "=r"(lo[g].x), "=r"(lo[g].y), "=r"(lo[g].z), "=r"(lo[g].w), "=r"(hi[g].x), "=r"(hi[g].y), "=r"(hi[g].z), "=r"(hi[g].w)
                      : "l"(p) : "memory");
       }
-    if (k0 + GROUP >= a.n) pdl_next(a.seam.ahead);   // (all CTAs: asking is not what bounds these, fp32 x3 of 5 M 10.35 us, 10.45 from a.seam.ask on)
+    if (k0 + GROUP >= a.n) pdl_next(a.seam.ahead);
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (k0 + g < a.n) {

@@ -61,11 +61,11 @@ __device__ __forceinline__ void st32(void* p, const uint4& a, const uint4& b) {
 // the first load of the last group, with the edges between the loads and the additions, it works; with code behind the
 // store it worked no better than asking at the very end.  All of up to eight sources in flight together pay then, and the
 // edges are the first CTA's: the last one starts when the call is nearly over (fp32 x3 views of 5 M 12.2 us with the last
-// one, 11.4 with the first).  us, calls in a row on fresh tensors, neither / this: fp32 x2 of 5 M 10.1 / 8.8, x3 views 12.9
+// one, 11.4 with the first).  us, calls in a row on fresh tensors, neither / this: fp32 x2 of 5 M 10.1 / 8.7, x3 views 12.9
 // / 11.4, x4 of 2.7 M 9.2 / 7.9, x8 of 1.5 M 9.4 / 8.0, of 2.5 M 14.5 / 12.9, of 6.5 M 34.3 / 33.2 (7.1 TB/s), of 64 Mi
 // 335.1 / 334.2 (7.2); bf16 x8 of 4 M 12.0 / 10.6; int32 masks x6 of 3 M 13.6 / 12.1; fp64 x2 of 4 M 15.4 / 14.1.  From nine
 // sources up they ask behind the fourth load of the last group (fp32 x16 of 1.2 M 13.2 / 12.1), in 16-bit floats behind all of
-// them (x16 of 8 M 40.2, 39.1 so, 39.8 behind the fourth).  In a captured graph less of it is left: x8 of 2.5 M 14.3 / 14.0.
+// them (x16 of 8 M 40.2, 39.1 so, 39.8 behind the fourth).  In a captured graph x8 of 2.5 M 14.5 / 13.1.
 template <int POL, int NSRC, int THREADS, int GROUP, bool EARLY>
 __global__ void __launch_bounds__(THREADS) reduce_nway_wide_kernel(const __grid_constant__ NwayArgs a) {
   using P = typename PolById<POL>::type;
